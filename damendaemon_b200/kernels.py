@@ -62,6 +62,8 @@ _SIGNATURES = {
                          _c_float, _c_void, _c_int, _c_void, _c_int, _c_int, _c_int, _c_int, _c_void, _c_void, _c_int, _c_void],
         "dd_retention_finish": [_c_void, _c_void, _c_int, _c_void, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_void, _c_void],
         "dd_gemm_simt": [_c_void, _c_int, _c_void, _c_int, _c_void, _c_void, _c_int, _c_void, _c_int] + [_c_int] * 6 + [_c_void],
+        "dd_gemm_split_plan": [_c_int] * 4 + [_c_void],
+        "dd_gemm_split": [_c_void, _c_int, _c_void, _c_int, _c_void, _c_void, _c_int, _c_void, _c_int] + [_c_int] * 7 + [_c_void] * 3,
         "dd_kv_store": [_c_void, _c_void, _c_int, _c_void, _c_void, _c_void, _c_int, _c_void] + [_c_int] * 7 + [_c_void, _c_void],
         "dd_attention_rows": [_c_void, _c_int, _c_void, _c_void, _c_void, _c_void, _c_int, _c_void, _c_int, _c_void, _c_void]
                              + [_c_int] * 7 + [_c_float, _c_int, _c_int, _c_void, _c_void],
@@ -1142,6 +1144,47 @@ def gemm_simt(a, w, bias=None, residual=None, activation=None, out_dtype=None, o
           _ptr(bias, "bias", torch.float32), _ptr(residual, "residual", torch.float32),
           0 if residual is None else residual.stride(0), _ptr(out, "out", out_dtype), out.stride(0),
           M, N, K, ACTIVATIONS[activation], _dt(a.dtype), _dt(out_dtype), _stream())
+    return out
+
+
+def gemm_split_fits(a, w):
+    """Whether gemm_split takes these operands: float32, 16-byte aligned rows, a reduction width that is a multiple of 4."""
+    return a.dtype == torch.float32 and w.dtype == torch.float32 and not (a.shape[1] % 4 or a.stride(0) % 4 or w.stride(0) % 4) and \
+        not (a.data_ptr() | w.data_ptr()) & 15
+
+
+_split_plans = {}
+
+
+def gemm_split(a, w, bias=None, residual=None, activation=None, out=None, token_tile=None, splits=None):
+    """act(a @ w.T + bias) (+ residual), all float32, on the tensor cores: every operand as the sum of three bfloat16
+    numbers, six products of them, k blocks of 32 summed in float32 registers (csrc/gemm_split_tcgen05.cu). a [M,K],
+    w [N,K], 16-byte aligned, K and the row strides multiples of 4. token_tile (16, 32, 64, 128) and splits (blocks that
+    share a tile's K) override the kernel's own plan."""
+    _rows(a, "a"), _rows(w, "w")
+    M, K = a.shape
+    N = w.shape[0]
+    if a.dtype != torch.float32 or w.dtype != torch.float32 or w.shape[1] != K:
+        raise KernelError(f"gemm_split: needs float32 a [M,K] and w [N,K]; got {tuple(a.shape)} {a.dtype}, {tuple(w.shape)} {w.dtype}")
+    if out is None:
+        out = torch.empty((M, N), dtype=torch.float32, device=a.device)
+    _rows(out, "out")
+    if residual is not None:
+        _rows(residual, "residual")
+    lib, sms = library("core"), sm_count(a.device)
+    plan = _split_plans.get((M, N, K))
+    if plan is None:
+        tile = ctypes.c_int(0)
+        planned = lib.dd_gemm_split_plan(M, N, K, sms, ctypes.byref(tile))
+        plan = _split_plans[(M, N, K)] = (planned, tile.value)
+    token_tile = plan[1] if token_tile is None else token_tile
+    planes = None if token_tile < 64 else \
+        torch.empty((-(-M // token_tile) * token_tile * -(-K // 32) * 192,), dtype=torch.uint8, device=a.device)
+    _call(lib, "dd_gemm_split", _ptr(a, "a"), a.stride(0), _ptr(w, "w"), w.stride(0), _ptr(bias, "bias", torch.float32),
+          _ptr(residual, "residual", torch.float32), 0 if residual is None else residual.stride(0),
+          _ptr(out, "out", torch.float32), out.stride(0), M, N, K, ACTIVATIONS[activation],
+          token_tile, plan[0] if splits is None else splits, sms, _ptr(planes), _ptr(error_flag(a.device)), _stream(),
+          n_kernels=1 if planes is None else 2)
     return out
 
 

@@ -1,0 +1,92 @@
+"""The float32 engine's products on the tensor cores, with every operand split into three bfloat16 numbers, against
+64-bit results at the edges of their tiles."""
+import pytest
+import torch
+
+from test_gpu_kernels import DEV, K  # noqa: F401  (K is a fixture)
+
+pytestmark = pytest.mark.gpu
+
+
+def operands(M, N, Kd, seed=1, mean=0.0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    a = torch.randn(M, Kd, generator=g, device=DEV) + mean
+    w = torch.randn(N, Kd, generator=g, device=DEV) * 0.1 + mean
+    return a, w
+
+
+@pytest.mark.parametrize("M,N,Kd", [(1, 1, 4), (1, 130, 36), (16, 127, 32), (17, 129, 100), (32, 513, 1600), (33, 128, 64), (64, 300, 260),
+                                    (65, 1600, 1600), (128, 128, 6400), (129, 257, 96), (300, 1281, 1280), (7, 1600, 6400)])
+def test_split_product(K, M, N, Kd):
+    """Against 64 bits: within the bound of float32 summation of the terms' sizes (one rounding a k block of 32 and its
+    few cut-off additions), and over all outputs no further off than one chain of float32 multiply-adds an output."""
+    for mean in (0.0, 1.0):
+        a, w = operands(M, N, Kd, mean=mean)
+        want, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+        got = K.gemm_split(a, w)
+        # a k block: 12 additions into the accumulator, each cut off at 2^-23 of what has been added so far; the blocks'
+        # sums, and the blocks of a cluster, one rounding each; the three products left out, 3 x 2^-25 of their term
+        allowed = size * (14 * 2.0 ** -23 + (Kd / 32 + 9) * 2.0 ** -24)
+        assert ((got.double() - want).abs() <= allowed).all()
+        plain = K.gemm_simt(a, w)
+        # (with a handful of outputs either of the two may be the lucky one)
+        if M * N >= 1024:
+            assert (got.double() - want).norm() <= (plain.double() - want).norm()
+        assert torch.equal(got, K.gemm_split(a, w)), "two runs are bit-equal"
+    bias, stream = torch.randn(N, device=DEV), torch.randn(M, N, device=DEV)
+    u = want + bias.double()
+    full = K.gemm_split(a, w, bias, residual=stream.clone(), activation="gelu")
+    exact = 0.5 * u * (1 + torch.erf(u / 2 ** 0.5)) + stream.double()
+    assert ((full.double() - exact).abs() <= 2 * allowed + 1e-6 * (1 + u.abs())).all()
+    in_place = stream.clone()
+    assert K.gemm_split(a, w, bias, residual=in_place, out=in_place).data_ptr() == in_place.data_ptr()
+    assert ((in_place.double() - u - stream.double()).abs() <= allowed + 1e-6 * (1 + u.abs())).all()
+    assert K.read_error_flag(DEV) == 0
+
+
+@pytest.mark.parametrize("tile,M", [(16, 9), (32, 50), (64, 130), (128, 131)])
+def test_split_product_in_any_tile_and_cluster(K, tile, M):
+    N, Kd = 390, 416
+    a, w = operands(M, N, Kd, seed=3)
+    wide = torch.full((M, N + 8), 7.0, device=DEV)
+    want = a.double() @ w.double().t()
+    for splits in (1, 2, 3, 8):
+        got = K.gemm_split(a, w, out=wide[:, 4:4 + N], token_tile=tile, splits=splits)
+        assert (got.double() - want).abs().max() < 2e-5
+        assert bool((wide[:, :4] == 7).all()) and bool((wide[:, 4 + N:] == 7).all())
+    # operands inside wider rows
+    big_a, big_w = torch.randn(M, Kd + 12, device=DEV), torch.randn(N, Kd + 4, device=DEV)
+    got = K.gemm_split(big_a[:, 4:4 + Kd], big_w[:, 4:4 + Kd], token_tile=tile)
+    assert (got.double() - big_a[:, 4:4 + Kd].double() @ big_w[:, 4:4 + Kd].double().t()).abs().max() < 4e-4
+    assert K.read_error_flag(DEV) == 0
+
+
+@pytest.mark.parametrize("M", [5, 40, 70, 200])
+def test_split_product_of_values_that_have_no_three_parts(K, M):
+    """Infinities, NaN, numbers that bfloat16 rounds to infinity, sums that overflow: what the float32 kernel gives."""
+    a, w = operands(M, 200, 160, seed=5)
+    a[1, 7], a[2, 9], a[3, 30], a[4, 31] = float("inf"), float("nan"), 3.4e38, -float("inf")
+    w[5, 11], w[6, 12], w[130, 40] = float("inf"), -3.395e38, float("nan")
+    a[0, :40] = 1e30
+    w[8, :40] = 1e12
+    w[9, :40] = 1e-30
+    got, plain = K.gemm_split(a, w), K.gemm_simt(a, w)
+    finite = torch.isfinite(plain)
+    assert torch.equal(torch.isnan(plain), torch.isnan(got)) and torch.equal(finite, torch.isfinite(got))
+    odd = ~finite & ~torch.isnan(plain)
+    assert torch.equal(got[odd], plain[odd]) and bool(odd.any())
+    assert ((got - plain)[finite].abs() <= 1e-4 * (1 + plain[finite].abs())).all()
+    tiny = torch.full((M, 160), 1e-20, device=DEV)
+    assert torch.allclose(K.gemm_split(tiny, w[20:60]) * 1e20, w[20:60].sum(1).expand(M, -1), atol=2e-5)
+
+
+def test_which_float32_products_are_split(K):
+    from types import SimpleNamespace
+    from damendaemon_b200.parts.linear import linear, splits_float32
+    assert splits_float32(1, 1600, 1600) and splits_float32(65, 96, 96) and not splits_float32(300, 96, 64) and not splits_float32(64, 512, 512)
+    a, w = operands(8, 1600, 1600)
+    auto, plain = SimpleNamespace(gemm="auto"), SimpleNamespace(gemm="simt")
+    assert torch.equal(linear(auto, a, w), K.gemm_split(a, w)) and torch.equal(linear(plain, a, w), K.gemm_simt(a, w))
+    # rows that start off a 16-byte boundary stay on the CUDA cores
+    shifted = torch.randn(8, 1601, device=DEV)[:, 1:]
+    assert torch.equal(linear(auto, shifted, w), K.gemm_simt(shifted, w))
