@@ -1,7 +1,7 @@
 """Paged causal attention of a step's tokens: the cache write and the choice of kernel.
 
-Five kernels can serve (csrc/attention_*.cu): the general one (any sizes, both dtypes: the float32 path, the
-fallback and the reference of the others; the mma.sync prompt kernel takes the portions of other head sizes in padded
+Seven kernels can serve (csrc/attention_*.cu): the general one (any sizes, both dtypes: the fallback and the
+reference of the others; two float32 ones, for portions and for single tokens; the mma.sync prompt kernel takes the portions of other head sizes in padded
 tiles), two bfloat16 decode kernels (rows by cp.async; whole pages of a group of
 heads by TMA) and two bfloat16 prompt kernels (mma.sync; tcgen05). Which one a step takes depends on the step
 (decode only or not, how many (token, head) pairs), on what each kernel supports (head size, page size, groups) and
@@ -76,6 +76,8 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
     k_new, v_new = (k, v) if cache.writable else (None, None)
     fast = runtime.attention != "rows"
     masked = dict(chunk=chunk, gate=gate)      # every kernel takes the chunked mask and the gate on its output
+    if fast and not special and kernels.attention_f32_supported(q, kv, k_new, v_new):
+        return float32_attention(ctx, q, k_new, v_new, kv, table, n_heads, scale, window, **masked)
     tensor = fast and runtime.attention != "mma" and not special
     # a sink alone (no kept first keys, no cap, no weights in two terms) the tcgen05 prompt kernel takes as well
     sink_only = sink is not None and not (keep_first or softcap or exact_weights)
@@ -134,6 +136,39 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
                                          out=out, **masked, **exact)
     return general_attention(ctx, q, kv, table, n_heads, scale, window, kv_heads, head_dim, head_dim, exact_weights, chunk=chunk,
                              gate=gate, **(more if special else {}))
+
+
+def float32_attention(ctx, q, k_new, v_new, kv, table, n_heads, scale, window, chunk, gate):
+    """A float32 cache: single tokens (which lie first) go to the kernel that reads whole rows and writes their own key and
+    value, portions to the one that shares key blocks among 64 queries."""
+    n1 = ctx.n_entries if ctx.decode_only else ctx.n_single
+    if n1 == q.shape[0]:
+        return kernels.attention_f32_decode(q, kv, ctx.positions, table, n_heads, scale, window, n_splits=float32_splits(ctx, n1, n_heads),
+                                            k_new=k_new, v_new=v_new, chunk=chunk, gate=gate)
+    import torch
+    out = torch.empty_like(q, memory_format=torch.contiguous_format)
+    if k_new is not None:
+        kernels.kv_store(k_new[n1:], v_new[n1:], ctx.token_entry[n1:], ctx.positions[n1:], table, kv)
+    if n1:
+        kernels.attention_f32_decode(q[:n1], kv, ctx.positions[:n1], table, n_heads, scale, window, n_splits=float32_splits(ctx, n1, n_heads),
+                                     out=out[:n1], k_new=None if k_new is None else k_new[:n1], v_new=None if v_new is None else v_new[:n1],
+                                     chunk=chunk, gate=None if gate is None else gate[:n1])
+    # A tile's keys are shared among blocks while tiles x heads leave SMs without their three blocks: few in all, or long
+    # portions whose last tiles work longest (us in 1 / 2 / 4 pieces: 32 queries x 2 heads at 100 keys 25 / 19 / 13, 200 x 4
+    # 46 / 27 / 18; 1,000 x 20 135 / 111 / 135; but 2 x 1,024 x 25 255 / 266 / 322, and 8 prompts of 64 x 25, whose tiles have
+    # one block of keys, 14 / 25 / 43).
+    n, entries = q.shape[0] - n1, ctx.n_entries - n1
+    blocks = (-(-n // 64) + entries - 1) * n_heads
+    splits = 4 if 4 * blocks <= 3 * ctx.sm_count else (2 if 2 * blocks <= 5 * ctx.sm_count and n >= 128 * entries else 1)
+    return kernels.attention_f32_prompt(q, kv, ctx.entry_start[n1:], ctx.entry_pos0[n1:], table[n1:], n_heads, scale, window, out=out,
+                                        n_splits=min(splits, max(1, ctx.split_context // 128)), chunk=chunk, gate=gate)
+
+
+def float32_splits(ctx, n_tokens, n_heads, keys_per_block=128):
+    """Blocks that share a token's keys: as many as are resident at once (two an SM; a second wave costs more than longer
+    pieces: 200 (token, head) pairs of 70 keys in one and in two pieces), each with at least two rounds of its eight warps."""
+    want = 2 * ctx.sm_count // max(1, n_tokens * n_heads)
+    return max(1, min(want, -(-ctx.split_context // keys_per_block), 8))
 
 
 def general_attention(ctx, q, kv, table, n_heads, scale, window, kv_heads, head_dim, value_dim, exact_weights=False, gate=None, **mask):

@@ -1,9 +1,9 @@
-"""The float32 engine's products on the tensor cores, with every operand split into three bfloat16 numbers, against
-64-bit results at the edges of their tiles."""
+"""The float32 engine's own kernels: products on the tensor cores with every operand split into three bfloat16 numbers,
+and paged attention of prompt portions and of single tokens, each against 64-bit results at the edges of its tiles."""
 import pytest
 import torch
 
-from test_gpu_kernels import DEV, K  # noqa: F401  (K is a fixture)
+from test_gpu_kernels import DEV, K, paged_case  # noqa: F401  (K is a fixture)
 
 pytestmark = pytest.mark.gpu
 
@@ -90,3 +90,63 @@ def test_which_float32_products_are_split(K):
     # rows that start off a 16-byte boundary stay on the CUDA cores
     shifted = torch.randn(8, 1601, device=DEV)[:, 1:]
     assert torch.equal(linear(auto, shifted, w), K.gemm_simt(shifted, w))
+
+
+SIZES = [(3, 3, 16, 16), (4, 2, 48, 8), (5, 5, 64, 16), (6, 2, 32, 12), (2, 1, 128, 32), (2, 2, 20, 4), (3, 1, 100, 16)]
+
+
+@pytest.mark.parametrize("heads,kv_heads,d,page", SIZES)
+@pytest.mark.parametrize("window", [None, 70])
+def test_prompt_attention(K, heads, kv_heads, d, page, window):
+    lengths, new = [64, 1, 65, 200, 331], [64, 1, 1, 129, 64]
+    c = paged_case(K, torch.float32, heads, kv_heads, d, page, lengths, new, window, 1)
+    assert K.attention_f32_supported(c["q"], c["cache"])
+    start = torch.tensor([0] + torch.tensor(new).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    pos0 = torch.tensor([n - m for n, m in zip(lengths, new)], dtype=torch.int32, device=DEV)
+    for splits in (1, 2, 3, 4):
+        got = K.attention_f32_prompt(c["q"], c["cache"], start, pos0, c["table"], heads, c["scale"], window, n_splits=splits)
+        assert (got.cpu().double() - c["ref"]).abs().max() < 2e-5
+    # the chunked mask and the gate, as the general kernel has them
+    gate = torch.randn(sum(new), heads, device=DEV)
+    more = dict(chunk=40, gate=gate)
+    want = K.attention_rows(c["q"], c["cache"], c["ent"], c["pos"], c["table"], heads, c["scale"], window, **more)
+    got = K.attention_f32_prompt(c["q"], c["cache"], start, pos0, c["table"], heads, c["scale"], window, n_splits=2, **more)
+    assert (got - want).abs().max() < 2e-5 and K.read_error_flag(DEV) == 0
+
+
+@pytest.mark.parametrize("heads,kv_heads,d,page", SIZES)
+@pytest.mark.parametrize("splits", [1, 3, 8])
+def test_single_token_attention(K, heads, kv_heads, d, page, splits):
+    lengths = [1, 2, 63, 64, 65, 300, 517]
+    for window, chunk in ((None, None), (70, None), (None, 40)):
+        c = paged_case(K, torch.float32, heads, kv_heads, d, page, lengths, [1] * len(lengths), window, 1, store=False)
+        k = c["packed"][:, heads * d:(heads + kv_heads) * d]
+        v = c["packed"][:, (heads + kv_heads) * d:]
+        stored = c["cache"].clone()
+        K.kv_store(k, v, c["ent"], c["pos"], c["table"], stored)
+        gate = torch.randn(len(lengths), heads, device=DEV) if chunk else None
+        got = K.attention_f32_decode(c["q"], c["cache"], c["pos"], c["table"], heads, c["scale"], window, n_splits=splits, k_new=k, v_new=v,
+                                     chunk=chunk, gate=gate)
+        assert torch.equal(torch.nan_to_num(c["cache"], nan=5.0), torch.nan_to_num(stored, nan=5.0)), "the new keys and values are in the cache"
+        if chunk is None:
+            assert (got.cpu().double() - c["ref"]).abs().max() < 2e-5
+        want = K.attention_rows(c["q"], stored, c["ent"], c["pos"], c["table"], heads, c["scale"], window, chunk=chunk, gate=gate)
+        assert (got - want).abs().max() < 2e-5
+        again = K.attention_f32_decode(c["q"], stored, c["pos"], c["table"], heads, c["scale"], window, n_splits=splits, chunk=chunk, gate=gate)
+        assert torch.equal(got, again) and K.read_error_flag(DEV) == 0
+
+
+def test_a_missing_page_is_reported(K):
+    lengths = [40, 90]
+    c = paged_case(K, torch.float32, 2, 2, 64, 16, lengths, [1, 1], None, 1)
+    table = c["table"].clone()
+    table[1, 2] = -1
+    got = K.attention_f32_decode(c["q"], c["cache"], c["pos"], table, 2, c["scale"])
+    assert K.read_error_flag(DEV) == 4 and torch.isfinite(got).all()
+    start, pos0 = (torch.tensor(x, dtype=torch.int32, device=DEV) for x in ([0, 1, 2], [39, 89]))
+    got = K.attention_f32_prompt(c["q"], c["cache"], start, pos0, table, 2, c["scale"])
+    assert K.read_error_flag(DEV) == 4 and torch.isfinite(got).all()
+    table[0, 2] = 1000
+    packed = c["packed"]
+    K.attention_f32_decode(c["q"], c["cache"], c["pos"], table, 2, c["scale"], k_new=packed[:, 128:256], v_new=packed[:, 256:])
+    assert K.read_error_flag(DEV) & 2
