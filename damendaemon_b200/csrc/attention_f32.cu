@@ -7,7 +7,7 @@
 // 1,100 us for 1,000 tokens x 20 heads of 64, where the multiply-adds alone need 38. Here a block of a prompt owns 64
 // queries of a head and reads each block of 64 keys once for all of them into shared memory (cp.async, the next block's
 // keys under this block's softmax and values, its values under the next scores); a thread holds 4 x 8 scores and 4
-// queries' pieces of the output in registers: 111 us. What bounds it now are the reads of shared memory (12 of 16 bytes
+// queries' pieces of the output in registers: 106 us. What bounds it now are the reads of shared memory (12 of 16 bytes
 // for 128 multiply-adds a thread, 56 us) and the few warps that hide them (registers: three blocks an SM). A single
 // token's block reads whole rows by groups of lanes, eight key and eight value rows of a group in flight at once, every
 // group with a running maximum and sum of its own; a token's keys may be cut over the blocks of a cluster, whose results
@@ -92,7 +92,7 @@ constexpr int PROMPT_SPLITS = 4;                            // blocks that may s
 // block a tile left 1.6 of three possible blocks on an SM for 1,000 tokens x 20 heads and the SMs with the last tiles busy
 // twice as long as the others: 148 us.)
 template <int D>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, D <= 64 ? 3 : 1)
 attention_f32_prompt_kernel(const float* __restrict__ q, int q_stride, const float* __restrict__ cache, const int* __restrict__ entry_start,
                             const int* __restrict__ entry_pos0, int n_entries, float* __restrict__ out, int out_stride, int H, Pages pages,
                             Mask mask, float scale, const float* __restrict__ gate, int gate_stride, int* __restrict__ error_flag) {
@@ -172,35 +172,44 @@ attention_f32_prompt_kernel(const float* __restrict__ q, int q_stride, const flo
         look_up(b + S, turn + 1);
         cp_wait<1>();
         __syncthreads();                                    // this block's keys are there, the next one's rows looked up
-        pair_t part[4][8];                                  // a score's sums over even and odd elements
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) part[i][j] = 0;
-#pragma unroll 2
-        for (int c = 0; c < D; c += 4) {
-            Quad a[4], k[8];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = load_quad(sQ + (ty + 16 * i) * LD + c);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) k[j] = load_quad(sK + (tx + 8 * j) * LD + c);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    fma2(part[i][j], a[i].lo, k[j].lo);
-                    fma2(part[i][j], a[i].hi, k[j].hi);
-                }
-        }
+        // A score is the sum of pieces of 16 elements, each from its even and its odd ones: shorter chains of additions
+        // are less far from the exact sum (and from the sums that the single-token kernel makes in other orders).
         float s[4][8];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float even, odd;
-                unpair(part[i][j], even, odd);
-                s[i][j] = even + odd;
+            for (int j = 0; j < 8; ++j) s[i][j] = 0.f;
+#pragma unroll 1
+        for (int c0 = 0; c0 < D; c0 += 16) {
+            pair_t part[4][8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) part[i][j] = 0;
+#pragma unroll
+            for (int c = c0; c < c0 + 16; c += 4) {
+                Quad a[4], k[8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] = load_quad(sQ + (ty + 16 * i) * LD + c);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) k[j] = load_quad(sK + (tx + 8 * j) * LD + c);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        fma2(part[i][j], a[i].lo, k[j].lo);
+                        fma2(part[i][j], a[i].hi, k[j].hi);
+                    }
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    float even, odd;
+                    unpair(part[i][j], even, odd);
+                    s[i][j] += even + odd;
+                }
+        }
         __syncthreads();                                    // everybody is through with the keys
         load(b + S, turn + 1, sK, 0);
         bool live[8];
@@ -360,8 +369,7 @@ attention_f32_decode_kernel(const float* __restrict__ q, const float* __restrict
             *reinterpret_cast<float4*>(cache + at + value_plane + c) = *reinterpret_cast<const float4*>(own_v + c);
         }
     }
-    float4 qv = mine ? *reinterpret_cast<const float4*>(q + (size_t)t * q_stride + (size_t)h * d + c) : zero;
-    qv.x *= scale; qv.y *= scale; qv.z *= scale; qv.w *= scale;
+    const float4 qv = mine ? *reinterpret_cast<const float4*>(q + (size_t)t * q_stride + (size_t)h * d + c) : zero;
 
     const int lo = mask.first_seen(pos);
     // whole rounds of a warp's keys for every warp of every block: a piece starts on a multiple of a round
@@ -408,7 +416,7 @@ attention_f32_decode_kernel(const float* __restrict__ q, const float* __restrict
             s[u] = fmaf(qv.w, kv[u].w, fmaf(qv.z, kv[u].z, fmaf(qv.y, kv[u].y, qv.x * kv[u].x)));
 #pragma unroll
             for (int x = 1; x < LANES; x <<= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], x);
-            if (!live[u]) s[u] = -CUDART_INF_F;
+            s[u] = live[u] ? s[u] * scale : -CUDART_INF_F;
             top = fmaxf(top, s[u]);
         }
         if (top == -CUDART_INF_F) continue;                 // (no shuffles below: groups may part here until the next round)
