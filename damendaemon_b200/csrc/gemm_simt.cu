@@ -76,7 +76,8 @@ gemm_simt_kernel(const TI* __restrict__ A, int lda, const TI* __restrict__ W, in
     }
 }
 
-// ---- few rows (a decode step): float32 operands ----
+// ---- few rows (a decode step), or a small matrix: float32 operands ----
+// (blockIdx.y: which MR rows of A, where there are more than that)
 // A block owns RB_N (32, or 16 for a narrow product, so that a hundred blocks stream it) output features for all MR
 // rows of A and streams its rows of W once, in chunks of 32 k through
 // a ring of cp.async stages (16-byte copies; 128 bytes of a row per chunk), so that a step of a few tokens reads
@@ -101,7 +102,7 @@ gemm_simt_rows_kernel(const float* __restrict__ A, int lda, const float* __restr
     constexpr int RB_STAGES = MR <= 16 ? 6 : (MR <= 32 ? 4 : 3);   // at most 41 KB of static shared memory
     __shared__ __align__(16) float Ws[RB_STAGES][RB_N][RB_LD];
     __shared__ __align__(16) float As[RB_STAGES][MR][RB_LD];
-    const int n0 = blockIdx.x * RB_N;
+    const int n0 = blockIdx.x * RB_N, m0 = blockIdx.y * MR;
     const int nl = threadIdx.x % RB_N, mg = threadIdx.x / RB_N;
     const int chunks = (K + RB_K - 1) / RB_K;
     // a chunk of W: RB_N rows x 8 pieces of 16 bytes, one or two per thread; of A: MR rows x 8 pieces
@@ -118,8 +119,8 @@ gemm_simt_rows_kernel(const float* __restrict__ A, int lda, const float* __restr
         const int st = c % RB_STAGES, k0 = c * RB_K;
         for (int piece = threadIdx.x; piece < MR * 8; piece += RB_THREADS) {
             const int row = piece >> 3, kk = (piece & 7) * 4;
-            const bool live = row < M && k0 + kk < K;
-            cp_async16(&As[st][row][kk], A + (size_t)(live ? row : 0) * lda + (live ? k0 + kk : 0), live);
+            const bool live = m0 + row < M && k0 + kk < K;
+            cp_async16(&As[st][row][kk], A + (size_t)(live ? m0 + row : 0) * lda + (live ? k0 + kk : 0), live);
         }
     };
     // the weights do not depend on the kernel before this one: their first stages are requested before the wait
@@ -158,7 +159,7 @@ gemm_simt_rows_kernel(const float* __restrict__ A, int lda, const float* __restr
     const float b = bias ? bias[n] : 0.f;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
-        const int m = mg * PER + i;
+        const int m = m0 + mg * PER + i;
         if (m >= M) continue;
         float v = dd_activation(acc[i] + b, act);
         if (residual) v += residual[(size_t)m * ldr + n];
@@ -169,7 +170,7 @@ gemm_simt_rows_kernel(const float* __restrict__ A, int lda, const float* __restr
 template <int MR, int RB_N, typename TO>
 int launch_rows(const void* A, int lda, const void* W, int ldw, const float* bias, const float* residual, int ldr,
                 void* C, int ldc, int M, int N, int K, int act, cudaStream_t s) {
-    dd_launch(gemm_simt_rows_kernel<MR, RB_N, TO>, dim3(dd_ceil_div(N, RB_N)), dim3(RB_THREADS), 0, s, (const float*)A, lda,
+    dd_launch(gemm_simt_rows_kernel<MR, RB_N, TO>, dim3(dd_ceil_div(N, RB_N), dd_ceil_div(M, MR)), dim3(RB_THREADS), 0, s, (const float*)A, lda,
               (const float*)W, ldw, bias, residual, ldr, (TO*)C, ldc, M, N, K, act);
     return dd_check_launch("dd_gemm_simt");
 }
@@ -323,7 +324,7 @@ DD_API int dd_gemm_simt(const void* A, int lda, const void* W, int ldw, const fl
     if (K <= 0) return dd_fail("dd_gemm_simt: bad K=%d", K);
     cudaStream_t s = (cudaStream_t)stream;
     if (in_dtype == DD_F32 && out_dtype == DD_F32) {
-        // up to 64 rows with 16-byte aligned rows: the kernel that streams the weights once; more rows: tiles of 128 x 128
+        // up to 64 rows with 16-byte aligned rows: the kernel that streams the weights once
         const bool aligned = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && !(((uintptr_t)A | (uintptr_t)W) & 15);
         const bool narrow = N < 3200;                      // fewer than a hundred blocks of 32 features
         if (aligned && M <= 8) return narrow ? launch_rows<8, 16, float>(A, lda, W, ldw, bias, residual, ldr, C, ldc, M, N, K, act, s)
@@ -334,6 +335,12 @@ DD_API int dd_gemm_simt(const void* A, int lda, const void* W, int ldw, const fl
                                               : launch_rows<32, 32, float>(A, lda, W, ldw, bias, residual, ldr, C, ldc, M, N, K, act, s);
         if (aligned && M <= 64) return narrow ? launch_rows<64, 16, float>(A, lda, W, ldw, bias, residual, ldr, C, ldc, M, N, K, act, s)
                                               : launch_rows<64, 32, float>(A, lda, W, ldw, bias, residual, ldr, C, ldc, M, N, K, act, s);
+        // More rows: with fewer tiles of 128 x 128 than two thirds of the SMs their blocks are too few and each walks the
+        // whole K alone, so 64 rows at a time go through the kernel above (same bits): 512 x 512 at
+        // 100 and 2,000 rows 60 -> 12 and 62 -> 49 us, 288 x 96 at 200 rows 16.6 -> 4.0 us; 768 x 768 at 4,000 rows has 192 tiles.
+        if (aligned && (long long)dd_ceil_div(N, BG) * dd_ceil_div(M, BG) < 100 && dd_ceil_div(M, 64) <= 65535)
+            return narrow ? launch_rows<64, 16, float>(A, lda, W, ldw, bias, residual, ldr, C, ldc, M, N, K, act, s)
+                          : launch_rows<64, 32, float>(A, lda, W, ldw, bias, residual, ldr, C, ldc, M, N, K, act, s);
         if (aligned) return launch_big(A, lda, W, ldw, bias, residual, ldr, C, ldc, M, N, K, act, s);
         return launch<float, float>(A, lda, W, ldw, bias, residual, ldr, C, ldc, M, N, K, act, s);
     }

@@ -6,14 +6,14 @@ import torch
 from .. import kernels
 
 
-def splits_float32(rows, out, reduction):
-    """Whether a float32 product of these sizes goes to the tensor cores, every operand as three bfloat16 numbers (its
-    error against 64-bit sums is below that of float32 multiply-adds one after the other at every size tried, K = 4 to
-    6,400). What decides is time alone. Measured (split / CUDA cores, us): up to 64 rows the CUDA-core kernel streams
-    small matrices in fewer steps than the split one needs to start: 1024 x 256 at 8 rows 7.2 / 3.4, 512 x 512 at 8 and
-    64 rows 7.3 / 4.8 and 12.4 / 11.9; 1024 x 1024 7.5 / 8.1 and 11.3 / 21.8; 6400 -> 1600 15 / 41 and 21.5 / 125. Beyond
-    64 rows its tiles of 128 x 128 are few and long: 512 x 256 at 100 rows 15 / 33, 288 x 96 14 / 16, 192 x 64 13.5 / 12.2."""
-    return reduction >= 96 if rows > 64 else out * reduction >= 1 << 20
+def splits_float32(out, reduction):
+    """Whether a float32 product with a matrix of this size goes to the tensor cores, every operand as three bfloat16
+    numbers (its error against 64-bit sums is below that of float32 multiply-adds one after the other at every size tried,
+    K = 4 to 6,400). Smaller matrices stream through the CUDA-core kernel in fewer steps than the split one needs to
+    start (split / CUDA cores, us): 1024 x 256 at 8 rows 7.2 / 3.4, 512 x 512 at 8 and 64 rows 7.3 / 4.8 and 12.4 / 11.9;
+    1024 x 1024 7.5 / 8.1 and 11.3 / 21.8, 6400 -> 1600 15 / 41 and 21.5 / 125. The line goes by the matrix alone, so that
+    a row of a small model has the same bits whatever else is in the batch."""
+    return out * reduction >= 1 << 20
 
 
 def linear(runtime, a, w, bias=None, residual=None, activation=None, out_dtype=None, out=None):
@@ -22,7 +22,7 @@ def linear(runtime, a, w, bias=None, residual=None, activation=None, out_dtype=N
     bfloat16 engine: the tcgen05 tensor-core kernel, unless the runtime asks for 'simt' or the
     reduction width is no multiple of 8 (then the CUDA-core kernel with bfloat16 operands)."""
     if a.dtype == torch.float32 and runtime.gemm != "simt" and out_dtype in (None, torch.float32) and \
-            splits_float32(a.shape[0], w.shape[0], a.shape[1]) and kernels.gemm_split_fits(a, w):
+            splits_float32(w.shape[0], a.shape[1]) and kernels.gemm_split_fits(a, w):
         return kernels.gemm_split(a, w, bias, residual, activation, out)
     if a.dtype == torch.float32 or runtime.gemm == "simt":
         return kernels.gemm_simt(a, w, bias, residual, activation, out_dtype, out)
