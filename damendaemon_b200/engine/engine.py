@@ -111,8 +111,8 @@ class Engine:
         # portions (whose token counts seldom repeat exactly) at their fourth.
         self.capture_after = {True: 1, False: 3}        # decode only? -> appearances before the capturing one
         self.max_graphs = 48                            # replayable step shapes kept; the least recently used goes first
-        # programmatic dependent launch: a gain for the bfloat16 kernels, a loss for the float32 ones (kernels.pdl_scope)
-        self.early_launch = self.dtype == torch.bfloat16
+        # programmatic dependent launch: a gain but for the float32 products on the CUDA cores (kernels.pdl_scope)
+        self.early_launch = self.dtype == torch.bfloat16 or gemm != "simt"
         self.max_graph_tokens = 4096                    # larger steps run eagerly (a graph keeps its activations)
         kernels.error_flag(self.device)                 # allocated before any graph capture
         if self.dtype == torch.bfloat16 and gemm != "simt":
