@@ -14,36 +14,9 @@
 // meet in the shared memory of the first (no scratch, no second launch), and the step's own key and value are taken from
 // the projection and written to the cache here: 8 requests x 25 heads, 70 keys, in a graph 5.7 us against 34 for the
 // general kernel, its merge and the cache write; at 1,000 keys 31 us (3.3 TB/s).
-#include "common.cuh"
-#include <math_constants.h>
+#include "attention_cores.cuh"
 
 namespace {
-
-struct Pages {
-    const int* block_table;      // [entries, max_blocks]
-    int max_blocks, page_size, n_pages, kv_heads, d;
-    int page_shift;              // log2 of the page size where that is a power of two, else -1
-    // element offset of a key's row in the cache (its head kh), -1 without a page; the value row lies value_plane() further on
-    __device__ __forceinline__ long long key_row(int entry, int key, int kh) const {
-        const int blk = page_shift >= 0 ? key >> page_shift : key / page_size;
-        const int page = blk < max_blocks ? block_table[(size_t)entry * max_blocks + blk] : -1;
-        if (page < 0 || page >= n_pages) return -1;
-        return ((long long)page * 2 * kv_heads + kh) * page_size * d + (long long)(key - blk * page_size) * d;
-    }
-    __device__ __forceinline__ long long value_plane() const { return (long long)kv_heads * page_size * d; }
-};
-
-struct Mask {
-    int window, chunk;
-    // the first key that a query at pos sees
-    __device__ __forceinline__ int first_seen(int pos) const {
-        int lo = window > 0 ? max(0, pos - window + 1) : 0;
-        if (chunk > 0) lo = max(lo, pos - pos % chunk);
-        return lo;
-    }
-};
-
-__device__ __forceinline__ float logistic(float v) { return 1.0f / (1.0f + expf(-v)); }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool live) {
     const int bytes = live ? 16 : 0;                       // zeros where there is nothing to copy
@@ -52,10 +25,6 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool live
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ uint32_t cluster_size() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Four values to the same place in the shared memory of the cluster's first block.
 __device__ __forceinline__ void send4(const float* where, float4 v) {
     uint32_t remote;
@@ -93,9 +62,9 @@ constexpr int PROMPT_SPLITS = 4;                            // blocks that may s
 // twice as long as the others: 148 us.)
 template <int D>
 __global__ void __launch_bounds__(THREADS, D <= 64 ? 3 : 1)
-attention_f32_prompt_kernel(const float* __restrict__ q, int q_stride, const float* __restrict__ cache, const int* __restrict__ entry_start,
-                            const int* __restrict__ entry_pos0, int n_entries, float* __restrict__ out, int out_stride, int H, Pages pages,
-                            Mask mask, float scale, const float* __restrict__ gate, int gate_stride, int* __restrict__ error_flag) {
+attention_f32_prompt_kernel(const float* q, int q_stride, const float* cache, const int* entry_start, const int* entry_pos0, int n_entries,
+                            float* out, int out_stride, int H, Pages pages, Mask mask, float scale, const float* gate, int gate_stride,
+                            int* error_flag) {
     constexpr int LD = D + 4, LP = BKV + 4, NC = D / 4, OJ = D / 32;
     extern __shared__ __align__(16) float smem[];
     float* sQ = smem;
@@ -332,200 +301,6 @@ attention_f32_prompt_kernel(const float* __restrict__ q, int q_stride, const flo
     }
 }
 
-// ---- single tokens ----
-constexpr int DECODE_WARPS = 8, BATCH = 8;
-
-// D: 16, 32, 64 or 128; LANES lanes hold a row of D elements, 4 each. Blocks: tokens, their heads, the pieces of the keys.
-template <int D>
-__global__ void __launch_bounds__(32 * DECODE_WARPS)
-attention_f32_decode_kernel(const float* __restrict__ q, const float* __restrict__ k_new, const float* __restrict__ v_new, int q_stride,
-                            float* __restrict__ cache, const int* __restrict__ positions, float* __restrict__ out, int out_stride, int H,
-                            Pages pages, Mask mask, float scale, const float* __restrict__ gate, int gate_stride, int* __restrict__ error_flag) {
-    constexpr int LANES = D / 4, GROUPS = 32 / LANES;      // keys a warp reads at once
-    constexpr int MOST = 8;                                 // blocks of a cluster
-    __shared__ __align__(16) float part_o[DECODE_WARPS * GROUPS][D];
-    __shared__ float part_m[DECODE_WARPS * GROUPS], part_l[DECODE_WARPS * GROUPS];
-    __shared__ __align__(16) float all_o[MOST][D];
-    __shared__ float all_m[MOST], all_l[MOST];
-    dd_launch_dependents();
-    dd_grid_wait();
-    const int S = (int)cluster_size(), rank = (int)cluster_rank();
-    const int row = blockIdx.x / S, t = row / H, h = row % H;
-    if (S > 1) cluster_arrive();                            // "my shared memory exists"
-    const int ratio = H / pages.kv_heads, kh = h / ratio, d = pages.d;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = lane / LANES, c = lane % LANES * 4;
-    const bool mine = c < d;                                // this lane's four elements are inside the head
-    const int pos = positions[t];
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    const long long value_plane = pages.value_plane();
-    const float* own_k = k_new ? k_new + (size_t)t * q_stride + (size_t)kh * d : nullptr;
-    const float* own_v = v_new ? v_new + (size_t)t * q_stride + (size_t)kh * d : nullptr;
-    if (own_k && rank == S - 1 && h == kh * ratio && warp == DECODE_WARPS - 1 && lane < LANES && mine) {
-        const long long at = pos >= 0 ? pages.key_row(t, pos, kh) : -1;
-        if (at < 0) {
-            if (c == 0) atomicOr(error_flag, 2);
-        } else {
-            *reinterpret_cast<float4*>(cache + at + c) = *reinterpret_cast<const float4*>(own_k + c);
-            *reinterpret_cast<float4*>(cache + at + value_plane + c) = *reinterpret_cast<const float4*>(own_v + c);
-        }
-    }
-    const float4 qv = mine ? *reinterpret_cast<const float4*>(q + (size_t)t * q_stride + (size_t)h * d + c) : zero;
-
-    const int lo = mask.first_seen(pos);
-    // whole rounds of a warp's keys for every warp of every block: a piece starts on a multiple of a round
-    constexpr int ROUND = DECODE_WARPS * GROUPS * BATCH;
-    const int span = pos + 1 - lo;
-    int per = (span + S - 1) / S;
-    per = (per + GROUPS * BATCH - 1) / (GROUPS * BATCH) * (GROUPS * BATCH);
-    const int k_end = min(pos + 1, lo + (rank + 1) * per);
-    float m = -CUDART_INF_F, l = 0.f;
-    float4 o = zero;
-    for (int base = lo + rank * per + warp * GROUPS * BATCH + group; base - group < k_end; base += ROUND) {
-        float4 kv[BATCH], vv[BATCH];
-        bool live[BATCH];
-        const float* kp[BATCH];
-        const float* vp[BATCH];
-#pragma unroll
-        for (int u = 0; u < BATCH; ++u) {
-            const int key = base + u * GROUPS;
-            live[u] = key < k_end;
-            kp[u] = vp[u] = nullptr;
-            if (live[u]) {
-                if (own_k && key == pos) {
-                    kp[u] = own_k;
-                    vp[u] = own_v;
-                } else {
-                    const long long at = pages.key_row(t, key, kh);
-                    if (at < 0) {
-                        atomicOr(error_flag, 4);
-                        live[u] = false;
-                    } else {
-                        kp[u] = cache + at;
-                        vp[u] = cache + at + value_plane;
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < BATCH; ++u) kv[u] = live[u] && mine ? *reinterpret_cast<const float4*>(kp[u] + c) : zero;
-#pragma unroll
-        for (int u = 0; u < BATCH; ++u) vv[u] = live[u] && mine ? *reinterpret_cast<const float4*>(vp[u] + c) : zero;
-        float s[BATCH], top = m;
-#pragma unroll
-        for (int u = 0; u < BATCH; ++u) {
-            s[u] = fmaf(qv.w, kv[u].w, fmaf(qv.z, kv[u].z, fmaf(qv.y, kv[u].y, qv.x * kv[u].x)));
-#pragma unroll
-            for (int x = 1; x < LANES; x <<= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], x);
-            s[u] = live[u] ? s[u] * scale : -CUDART_INF_F;
-            top = fmaxf(top, s[u]);
-        }
-        if (top == -CUDART_INF_F) continue;                 // (no shuffles below: groups may part here until the next round)
-        const float corr = expf(m - top);
-        l *= corr;
-        o.x *= corr; o.y *= corr; o.z *= corr; o.w *= corr;
-#pragma unroll
-        for (int u = 0; u < BATCH; ++u) {
-            const float p = live[u] ? expf(s[u] - top) : 0.f;
-            l += p;
-            o.x = fmaf(p, vv[u].x, o.x);
-            o.y = fmaf(p, vv[u].y, o.y);
-            o.z = fmaf(p, vv[u].z, o.z);
-            o.w = fmaf(p, vv[u].w, o.w);
-        }
-        m = top;
-    }
-    __syncwarp();
-    const int slot = warp * GROUPS + group;
-    *reinterpret_cast<float4*>(&part_o[slot][c]) = o;
-    if (c == 0) {
-        part_m[slot] = m;
-        part_l[slot] = l;
-    }
-    __syncthreads();
-    // the block's result, then the cluster's: an element a thread
-    const int i = threadIdx.x;
-    float top = -CUDART_INF_F, sum = 0.f, acc = 0.f;
-    if (i < D) {
-#pragma unroll
-        for (int x = 0; x < DECODE_WARPS * GROUPS; ++x) top = fmaxf(top, part_m[x]);
-        for (int x = 0; x < DECODE_WARPS * GROUPS; ++x) {
-            if (part_m[x] == -CUDART_INF_F) continue;
-            const float w = expf(part_m[x] - top);
-            sum = fmaf(part_l[x], w, sum);
-            acc = fmaf(part_o[x][i], w, acc);
-        }
-    }
-    if (S > 1) {
-        __syncwarp();
-        cluster_wait();
-        if (i < D) {
-            auto send = [&](const float* where, float v) {
-                uint32_t remote;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"((unsigned)__cvta_generic_to_shared(where)));
-                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
-            };
-            send(&all_o[rank][i], acc);
-            if (i == 0) {
-                send(&all_m[rank], top);
-                send(&all_l[rank], sum);
-            }
-        }
-        __syncwarp();
-        cluster_arrive();
-        cluster_wait();
-        if (rank != 0) return;
-        if (i < D) {
-            top = -CUDART_INF_F;
-            for (int r = 0; r < S; ++r) top = fmaxf(top, all_m[r]);
-            sum = acc = 0.f;
-            for (int r = 0; r < S; ++r) {
-                if (all_m[r] == -CUDART_INF_F) continue;
-                const float w = expf(all_m[r] - top);
-                sum = fmaf(all_l[r], w, sum);
-                acc = fmaf(all_o[r][i], w, acc);
-            }
-        }
-    }
-    if (i < d) {
-        float inv = sum == 0.f ? 0.f : 1.0f / sum;
-        if (gate) inv *= logistic(gate[(size_t)t * gate_stride + h]);
-        out[(size_t)t * out_stride + (size_t)h * d + i] = acc * inv;
-    }
-}
-
-int shift_of(int page_size) { return page_size > 0 && !(page_size & (page_size - 1)) ? __builtin_ctz(page_size) : -1; }
-
-int check_sizes(const char* what, int n_heads, int kv_heads, int d, int page_size, const void* q, int q_stride, const void* cache, int window, int chunk) {
-    if (d <= 0 || d % 4 || d > 128) return dd_fail("%s: head size %d is not a multiple of 4 up to 128", what, d);
-    if (n_heads <= 0 || kv_heads <= 0 || n_heads % kv_heads || page_size <= 0)
-        return dd_fail("%s: %d heads, %d key/value heads, pages of %d tokens", what, n_heads, kv_heads, page_size);
-    if (q_stride % 4 || (((uintptr_t)q | (uintptr_t)cache) & 15)) return dd_fail("%s: rows must be 16-byte aligned", what);
-    if (window < 0 || chunk < 0) return dd_fail("%s: window %d and chunk %d must not be negative", what, window, chunk);
-    return 0;
-}
-
-template <typename... KArgs, typename... Args>
-int launch_clusters(const char* what, void (*kernel)(KArgs...), long long blocks, int splits, int threads, int smem, cudaStream_t s, Args... args) {
-    if (blocks * splits > 0x7fffffffLL) return dd_fail("%s: %lld x %d blocks are more than one launch takes", what, blocks, splits);
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3((unsigned)(blocks * splits));
-    config.blockDim = dim3(threads);
-    config.dynamicSmemBytes = smem;
-    config.stream = s;
-    cudaLaunchAttribute attrs[2];
-    attrs[0].id = cudaLaunchAttributeClusterDimension;
-    attrs[0].val.clusterDim.x = splits;
-    attrs[0].val.clusterDim.y = 1;
-    attrs[0].val.clusterDim.z = 1;
-    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attrs[1].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attrs;
-    config.numAttrs = dd_pdl_enabled ? 2 : 1;
-    const cudaError_t e = cudaLaunchKernelEx(&config, kernel, static_cast<KArgs>(args)...);
-    if (e != cudaSuccess) return dd_fail("%s (clusters of %d): %s", what, splits, cudaGetErrorString(e));
-    return dd_check_launch(what);
-}
-
 template <int D>
 int launch_prompt(const float* q, int q_stride, const float* cache, const int* entry_start, const int* entry_pos0, int n_entries, int n_tokens,
                   float* out, int out_stride, int H, int splits, const Pages& pages, const Mask& mask, float scale, const float* gate,
@@ -538,13 +313,6 @@ int launch_prompt(const float* q, int q_stride, const float* cache, const int* e
                            scale, gate, gate_stride, error_flag);
 }
 
-template <int D>
-int launch_decode(const float* q, const float* k_new, const float* v_new, int q_stride, float* cache, const int* positions, float* out,
-                  int out_stride, int n_tokens, int H, int splits, const Pages& pages, const Mask& mask, float scale, const float* gate,
-                  int gate_stride, int* error_flag, cudaStream_t s) {
-    return launch_clusters("dd_attention_f32_decode", attention_f32_decode_kernel<D>, (long long)n_tokens * H, splits, 32 * DECODE_WARPS, 0, s, q,
-                           k_new, v_new, q_stride, cache, positions, out, out_stride, H, pages, mask, scale, gate, gate_stride, error_flag);
-}
 }  // namespace
 
 // Runs of consecutive tokens: entry e's are rows entry_start[e] .. entry_start[e + 1] - 1 of q, at positions
@@ -556,7 +324,7 @@ DD_API int dd_attention_f32_prompt(const float* q, int q_stride, const float* ca
                                    int head_dim, int page_size, int n_pages, int window, int chunk, float scale, int splits, const float* gate,
                                    int gate_stride, int* error_flag, void* stream) {
     if (n_tokens <= 0 || n_entries <= 0) return 0;
-    if (int e = check_sizes("dd_attention_f32_prompt", n_heads, kv_heads, head_dim, page_size, q, q_stride, cache, window, chunk)) return e;
+    if (int e = check_sizes("dd_attention_f32_prompt", n_heads, kv_heads, head_dim, page_size, q, q_stride, 4, cache, window, chunk)) return e;
     if (splits < 1 || splits > PROMPT_SPLITS) return dd_fail("dd_attention_f32_prompt: %d splits", splits);
     if (out_stride % 4 || ((uintptr_t)out & 15)) return dd_fail("dd_attention_f32_prompt: rows of the result must be 16-byte aligned");
     const Pages pages = {block_table, max_blocks, page_size, n_pages, kv_heads, head_dim, shift_of(page_size)};
@@ -565,24 +333,4 @@ DD_API int dd_attention_f32_prompt(const float* q, int q_stride, const float* ca
     if (head_dim <= 32) return launch_prompt<32>(q, q_stride, cache, entry_start, entry_pos0, n_entries, n_tokens, out, out_stride, n_heads, splits, pages, mask, scale, gate, gate_stride, error_flag, s);
     if (head_dim <= 64) return launch_prompt<64>(q, q_stride, cache, entry_start, entry_pos0, n_entries, n_tokens, out, out_stride, n_heads, splits, pages, mask, scale, gate, gate_stride, error_flag, s);
     return launch_prompt<128>(q, q_stride, cache, entry_start, entry_pos0, n_entries, n_tokens, out, out_stride, n_heads, splits, pages, mask, scale, gate, gate_stride, error_flag, s);
-}
-
-// One query a token; token t is at positions[t] and belongs to row t of block_table. k_new, v_new: null (its key and value
-// are in the cache), or row views of q's stride with them, which are then written to the cache. splits: blocks (at most 8)
-// that share a token's keys.
-DD_API int dd_attention_f32_decode(const float* q, const float* k_new, const float* v_new, int q_stride, float* cache, const int* positions,
-                                   int n_tokens, const int* block_table, int max_blocks, float* out, int out_stride, int n_heads, int kv_heads,
-                                   int head_dim, int page_size, int n_pages, int window, int chunk, float scale, int splits, const float* gate,
-                                   int gate_stride, int* error_flag, void* stream) {
-    if (n_tokens <= 0) return 0;
-    if (int e = check_sizes("dd_attention_f32_decode", n_heads, kv_heads, head_dim, page_size, q, q_stride, cache, window, chunk)) return e;
-    if ((!k_new) != (!v_new) || (((uintptr_t)k_new | (uintptr_t)v_new) & 15)) return dd_fail("dd_attention_f32_decode: keys and values come together, 16-byte aligned");
-    if (splits < 1 || splits > 8) return dd_fail("dd_attention_f32_decode: %d splits", splits);
-    const Pages pages = {block_table, max_blocks, page_size, n_pages, kv_heads, head_dim, shift_of(page_size)};
-    const Mask mask = {window, chunk};
-    cudaStream_t s = (cudaStream_t)stream;
-    if (head_dim <= 16) return launch_decode<16>(q, k_new, v_new, q_stride, cache, positions, out, out_stride, n_tokens, n_heads, splits, pages, mask, scale, gate, gate_stride, error_flag, s);
-    if (head_dim <= 32) return launch_decode<32>(q, k_new, v_new, q_stride, cache, positions, out, out_stride, n_tokens, n_heads, splits, pages, mask, scale, gate, gate_stride, error_flag, s);
-    if (head_dim <= 64) return launch_decode<64>(q, k_new, v_new, q_stride, cache, positions, out, out_stride, n_tokens, n_heads, splits, pages, mask, scale, gate, gate_stride, error_flag, s);
-    return launch_decode<128>(q, k_new, v_new, q_stride, cache, positions, out, out_stride, n_tokens, n_heads, splits, pages, mask, scale, gate, gate_stride, error_flag, s);
 }

@@ -30,12 +30,12 @@ HERE = Path(__file__).resolve().parent
 
 LIBRARIES = {
     "core": ["errors.cu", "embed.cu", "layernorm.cu", "rmsnorm.cu", "rotary.cu", "head_norm.cu", "retention.cu", "gemm_simt.cu", "gemm_split_tcgen05.cu", "kv_store.cu",
-             "attention_rows.cu", "attention_f32.cu", "moe.cu", "sampling.cu", "depth_mix.cu", "delta_rule.cu", "latent.cu", "embed_pairs.cu", "stream_ops.cu",
+             "attention_rows.cu", "attention_f32.cu", "attention_tokens.cu", "moe.cu", "sampling.cu", "depth_mix.cu", "delta_rule.cu", "latent.cu", "embed_pairs.cu", "stream_ops.cu",
              "state_space.cu", "linear_recurrence.cu", "time_mix.cu", "matrix_memory.cu", "post_norm.cu"],
     "tensor": ["errors.cu", "gemm_tcgen05.cu", "gemm_grouped_tcgen05.cu", "attention_decode.cu", "attention_decode_pages.cu", "attention_prefill.cu", "attention_prefill_tcgen05.cu", "attention_latent.cu",
                "wait_probe.cu"],
 }
-HEADERS = ["common.cuh", "tcgen05.cuh", "no_alloc.h"]
+HEADERS = ["common.cuh", "attention_cores.cuh", "tcgen05.cuh", "no_alloc.h"]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
 

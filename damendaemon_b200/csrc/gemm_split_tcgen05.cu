@@ -422,7 +422,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 // ROWS rows of 64 bytes under the 64-byte swizzle; [token tiles][k blocks] of them, zeros behind K, rows past the last
 // token left as they are (nobody reads their columns of the product).
 template <int ROWS>
-__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ X, int ldx, uint8_t* __restrict__ planes, int M, int K, int kblocks) {
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* X, int ldx, uint8_t* planes, int M, int K, int kblocks) {
     dd_launch_dependents();
     dd_grid_wait();
     // neighbouring threads: the four pieces of eight k of a row's k block, then the next rows

@@ -74,8 +74,8 @@ _SIGNATURES = {
                                       _c_int, _c_float, _c_void, _c_int],
         "dd_attention_f32_prompt": [_c_void, _c_int, _c_void, _c_void, _c_void, _c_int, _c_int, _c_void, _c_int, _c_void, _c_int]
                                    + [_c_int] * 7 + [_c_float, _c_int, _c_void, _c_int, _c_void, _c_void],
-        "dd_attention_f32_decode": [_c_void, _c_void, _c_void, _c_int, _c_void, _c_void, _c_int, _c_void, _c_int, _c_void, _c_int]
-                                   + [_c_int] * 7 + [_c_float, _c_int, _c_void, _c_int, _c_void, _c_void],
+        "dd_attention_tokens": [_c_void, _c_void, _c_void, _c_int, _c_void, _c_void, _c_int, _c_void, _c_int, _c_void, _c_int]
+                               + [_c_int] * 7 + [_c_float, _c_int, _c_void, _c_int, _c_int, _c_void, _c_void],
         "dd_embed_pairs": [_c_void] * 9 + [_c_int] * 4 + [ctypes.c_longlong, ctypes.c_longlong, _c_int, _c_void, _c_void],
         "dd_tanh_norm": [_c_void] * 6 + [_c_int, _c_int, _c_int, _c_void],
         "dd_add_rows": [_c_void, _c_void, _c_void, _c_int, _c_int, _c_void],
@@ -1261,19 +1261,21 @@ def attention_rows(q, cache, token_entry, positions, block_table, n_heads, scale
     return out
 
 
-def attention_f32_supported(q, cache, k_new=None, v_new=None):
-    """Whether the float32 attention kernels take these: one size of key and value heads, a multiple of 4 up to 128, and
-    rows that are 16-byte aligned."""
-    if q.dtype != torch.float32 or cache.dtype != torch.float32 or cache.dim() != 5 or not cache.is_contiguous():
+def attention_cores_supported(q, cache, k_new=None, v_new=None):
+    """Whether the attention kernels on the CUDA cores that read whole rows take these: one size of key and value heads of up
+    to 128 elements, every row whole 16-byte pieces that are 16-byte aligned. (attention_tokens both dtypes,
+    attention_f32_prompt float32.)"""
+    if q.dtype != cache.dtype or q.dtype not in (torch.float32, torch.bfloat16) or cache.dim() != 5 or not cache.is_contiguous():
         return False
-    if cache.shape[4] % 4 or cache.shape[4] > 128 or q.stride(0) % 4:
+    element = 4 if q.dtype == torch.float32 else 2
+    if cache.shape[4] * element % 16 or cache.shape[4] > 128 or q.stride(0) * element % 16:
         return False
     return not any(t is not None and t.data_ptr() & 15 for t in (q, cache, k_new, v_new))
 
 
-def _attention_f32_operands(q, cache, n_heads, out, more=()):
+def _attention_cores_operands(q, cache, n_heads, out, more=()):
     n_pages, _, kv_heads, page_size, head_dim = cache.shape
-    if q.shape[1] != n_heads * head_dim or q.stride(1) != 1 or q.dtype != torch.float32 or cache.dtype != torch.float32 or not cache.is_contiguous():
+    if q.shape[1] != n_heads * head_dim or q.stride(1) != 1 or q.dtype != cache.dtype or not cache.is_contiguous():
         raise KernelError("attention: q does not fit the cache")
     for t in more:
         if t is not None and (t.stride(0) != q.stride(0) or t.stride(1) != 1 or t.dtype != q.dtype or t.shape != (q.shape[0], kv_heads * head_dim)):
@@ -1287,11 +1289,13 @@ def attention_f32_prompt(q, cache, entry_start, entry_pos0, block_table, n_heads
                          gate=None):
     """Attention of runs of consecutive tokens over a float32 cache that holds their keys and values already; arguments as
     attention_prefill and attention_rows. n_splits: blocks (at most 4) that share the keys of a tile of 64 queries."""
-    out, sizes = _attention_f32_operands(q, cache, n_heads, out)
+    out, sizes = _attention_cores_operands(q, cache, n_heads, out)
+    if q.dtype != torch.float32:
+        raise KernelError("attention_f32_prompt: q and the cache must be float32")
     n_entries = entry_pos0.numel()
     if entry_start.numel() != n_entries + 1:
         raise KernelError("attention: the entry arrays do not fit each other")
-    gate, gate_stride, chunk = _f32_gate(gate, q, n_heads, chunk)
+    gate, gate_stride, chunk = _cores_gate(gate, q, n_heads, chunk)
     _call(library("core"), "dd_attention_f32_prompt", _ptr(q, "q"), q.stride(0), _ptr(cache, "cache"),
           _ptr(entry_start, "entry_start", torch.int32), _ptr(entry_pos0, "entry_pos0", torch.int32), n_entries, q.shape[0],
           _ptr(block_table, "block_table", torch.int32), block_table.shape[1], _ptr(out, "out", torch.float32), out.stride(0), *sizes,
@@ -1300,22 +1304,23 @@ def attention_f32_prompt(q, cache, entry_start, entry_pos0, block_table, n_heads
     return out
 
 
-def attention_f32_decode(q, cache, positions, block_table, n_heads, scale, window=None, n_splits=1, out=None, k_new=None, v_new=None,
-                         chunk=None, gate=None):
-    """Attention of single tokens over a float32 cache, token t being entry t. With k_new/v_new (row views like q) their keys
-    and values are taken from there and written to the cache. n_splits: blocks (at most 8) that share a token's keys."""
+def attention_tokens(q, cache, positions, block_table, n_heads, scale, window=None, n_splits=1, out=None, k_new=None, v_new=None,
+                     chunk=None, gate=None):
+    """Attention of single tokens over a float32 or bfloat16 cache, token t being entry t. With k_new/v_new (row views like q)
+    their keys and values are taken from there and written to the cache. n_splits: blocks (at most 8) that share a token's
+    keys."""
     if (k_new is None) != (v_new is None):
         raise KernelError("attention: k_new and v_new come together")
-    out, sizes = _attention_f32_operands(q, cache, n_heads, out, (k_new, v_new))
-    gate, gate_stride, chunk = _f32_gate(gate, q, n_heads, chunk)
-    _call(library("core"), "dd_attention_f32_decode", _ptr(q, "q"), _ptr(k_new), _ptr(v_new), q.stride(0), _ptr(cache, "cache"),
+    out, sizes = _attention_cores_operands(q, cache, n_heads, out, (k_new, v_new))
+    gate, gate_stride, chunk = _cores_gate(gate, q, n_heads, chunk)
+    _call(library("core"), "dd_attention_tokens", _ptr(q, "q"), _ptr(k_new), _ptr(v_new), q.stride(0), _ptr(cache, "cache"),
           _ptr(positions, "positions", torch.int32), q.shape[0], _ptr(block_table, "block_table", torch.int32), block_table.shape[1],
-          _ptr(out, "out", torch.float32), out.stride(0), *sizes, 0 if window is None else int(window), chunk, float(scale), int(n_splits),
-          gate, gate_stride, _ptr(error_flag(q.device)), _stream())
+          _ptr(out, "out", q.dtype), out.stride(0), *sizes, 0 if window is None else int(window), chunk, float(scale), int(n_splits),
+          gate, gate_stride, _dt(q.dtype), _ptr(error_flag(q.device)), _stream())
     return out
 
 
-def _f32_gate(gate, q, n_heads, chunk):
+def _cores_gate(gate, q, n_heads, chunk):
     if gate is not None and (gate.shape != (q.shape[0], n_heads) or gate.stride(1) != 1 or gate.dtype != q.dtype):
         raise KernelError("attention: the gate must be a [tokens, heads] row view in q's dtype")
     return _ptr(gate, "gate"), 0 if gate is None else gate.stride(0), 0 if chunk is None else int(chunk)

@@ -1,8 +1,8 @@
 """Paged causal attention of a step's tokens: the cache write and the choice of kernel.
 
 Seven kernels can serve (csrc/attention_*.cu): the general one (any sizes, both dtypes: the fallback and the
-reference of the others; two float32 ones, for portions and for single tokens; the mma.sync prompt kernel takes the portions of other head sizes in padded
-tiles), two bfloat16 decode kernels (rows by cp.async; whole pages of a group of
+reference of the others; the mma.sync prompt kernel takes the portions of other head sizes in padded
+tiles), one for single tokens of either dtype (whole rows on the CUDA cores), a float32 prompt kernel, two bfloat16 decode kernels (rows by cp.async; whole pages of a group of
 heads by TMA) and two bfloat16 prompt kernels (mma.sync; tcgen05). Which one a step takes depends on the step
 (decode only or not, how many (token, head) pairs), on what each kernel supports (head size, page size, groups) and
 on thresholds that were measured, which are data: ``AttentionTuning``, a field of the runtime, not constants of a
@@ -11,6 +11,8 @@ model. A mixer calls ``paged_attention`` through ``ctx.attend``.
 from __future__ import annotations
 
 from dataclasses import dataclass
+
+import torch
 
 from .. import kernels
 
@@ -26,6 +28,11 @@ class AttentionTuning:
     pages_per_block: int = 128            # a block of the page-streaming kernel holds the ids of this many pages
     row_keys_per_block: int = 128         # key split of the row decode kernel: keys per block ...
     row_blocks_per_sm: int = 2            # ... and blocks wanted per SM
+    tokens_to_pairs: int = 50             # bfloat16 steps of at most this many (token, head) pairs: whole rows on the CUDA cores, four
+                                          # blocks a pair, all requested before the projection is done (25 pairs, us beside the product
+                                          # before it, against rows: 100 keys 3.4 / 5.5, 544 keys 3.5 / 6.2, 1,000 keys 4.0 / 6.5; 50
+                                          # pairs at 544 keys 7.0 / 7.6; 100 pairs 13.1 / 10.7, pages 9.6) ...
+    tokens_to_pair_keys: int = 60_000     # ... and at most this many pairs x keys of context (measured up to 25 x 1,000)
 
 
 def prompt_key_block(n_heads, kv_heads, head_dim, page_size, dtype):
@@ -51,7 +58,6 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
             (gate is not None and (gate.stride(0) != q.stride(0) or gate.stride(1) != 1)):
         # the kernels read q, k and v as row views of one buffer (what a fused projection leaves); a part that made
         # new tensors of some of them (a position encoding that does not rotate in place) gets them packed again
-        import torch
         parts = [q, k, v] + ([gate] if gate is not None else [])
         packed = torch.cat(parts, dim=1).split([p.shape[1] for p in parts], dim=1)
         q, k, v = packed[:3]
@@ -76,7 +82,9 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
     k_new, v_new = (k, v) if cache.writable else (None, None)
     fast = runtime.attention != "rows"
     masked = dict(chunk=chunk, gate=gate)      # every kernel takes the chunked mask and the gate on its output
-    if fast and not special and kernels.attention_f32_supported(q, kv, k_new, v_new):
+    # the kernels that read whole rows on the CUDA cores (CUDA tensors only: they ask for the rows' alignment)
+    cores = q.is_cuda and fast and not special and kernels.attention_cores_supported(q, kv, k_new, v_new)
+    if cores and q.dtype == torch.float32:
         return float32_attention(ctx, q, k_new, v_new, kv, table, n_heads, scale, window, **masked)
     tensor = fast and runtime.attention != "mma" and not special
     # a sink alone (no kept first keys, no cap, no weights in two terms) the tcgen05 prompt kernel takes as well
@@ -84,6 +92,16 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
     def wants_pages(n_tokens):
         pairs = n_tokens * n_heads
         return pairs >= tune.pages_from_pairs or pairs * ctx.split_context >= tune.pages_from_pair_keys
+    def wants_tokens(n_tokens):
+        # few pairs; or heads and sizes that the other decode kernels do not take: key/value groups (8 requests x 25 heads on 5,
+        # 400 keys: 9 us, 32 through the general kernel and the cache write; 32 x 16 on 4, 600 keys: 37 / 69; 8 x 32 heads of 128
+        # on 8: 32 / 41) and small heads
+        pairs = n_tokens * n_heads
+        few = pairs <= tune.tokens_to_pairs and pairs * ctx.split_context <= tune.tokens_to_pair_keys
+        return cores and tensor and (few or not kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype))
+    if ctx.decode_only and wants_tokens(ctx.n_tokens):
+        return kernels.attention_tokens(q, kv, ctx.positions, table, n_heads, scale, window, n_splits=token_splits(ctx, ctx.n_tokens, n_heads),
+                                        k_new=k_new, v_new=v_new, **masked)
     if ctx.decode_only and tensor and wants_pages(ctx.n_tokens) and \
             kernels.attention_decode_pages_supported(n_heads, kv_heads, head_dim, page_size, q.dtype):
         # whole pages of a group of heads by TMA; it takes the new keys and values from the projection and writes them
@@ -104,12 +122,12 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
     # kernel, the portions to a prompt kernel. A prompt kernel spends a tile of 64 or 128 query rows and a walk over all
     # key blocks on a single token (measured with 56 decoding requests beside 8 portions of 249 tokens, 36 layers:
     # 8.3 ms a step through the prompt kernel alone, against 4.5 ms for 2,048 prompt tokens).
-    n1 = ctx.n_single if (tcgen05 or mma) and fast and kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype) else 0
+    n1 = ctx.n_single if (tcgen05 or mma) and fast and \
+        (wants_tokens(ctx.n_single) or kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype)) else 0
     out = None
     if n1:
-        import torch
         out = torch.empty((q.shape[0], n_heads * head_dim), dtype=q.dtype, device=q.device)
-        pages = tensor and wants_pages(n1) and \
+        pages = tensor and not wants_tokens(n1) and wants_pages(n1) and \
             kernels.attention_decode_pages_supported(n_heads, kv_heads, head_dim, page_size, q.dtype)
         if pages:
             splits = kernels.attention_decode_pages_splits(n1, n_heads, page_size, ctx.split_context, q.device)
@@ -117,10 +135,15 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
         else:
             splits = ctx.key_splits(n_heads, keys_per_block=tune.row_keys_per_block, blocks_per_sm=tune.row_blocks_per_sm,
                                     n_tokens=n1)
-        kernels.attention_decode(q[:n1], kv, None, ctx.positions[:n1], table, n_heads, scale, window, n_splits=splits,
-                                 out=out[:n1], k_new=None if k_new is None else k_new[:n1],
-                                 v_new=None if v_new is None else v_new[:n1], kernel="pages" if pages else "rows",
-                                 chunk=chunk, gate=None if gate is None else gate[:n1], **exact)
+        if wants_tokens(n1):
+            kernels.attention_tokens(q[:n1], kv, ctx.positions[:n1], table, n_heads, scale, window, n_splits=token_splits(ctx, n1, n_heads),
+                                     out=out[:n1], k_new=None if k_new is None else k_new[:n1], v_new=None if v_new is None else v_new[:n1],
+                                     chunk=chunk, gate=None if gate is None else gate[:n1])
+        else:
+            kernels.attention_decode(q[:n1], kv, None, ctx.positions[:n1], table, n_heads, scale, window, n_splits=splits,
+                                     out=out[:n1], k_new=None if k_new is None else k_new[:n1],
+                                     v_new=None if v_new is None else v_new[:n1], kernel="pages" if pages else "rows",
+                                     chunk=chunk, gate=None if gate is None else gate[:n1], **exact)
         if n1 == ctx.n_entries:
             return out
     # the tcgen05 prompt kernel writes the cache itself when no key block of its entries mixes cached and new keys
@@ -143,14 +166,13 @@ def float32_attention(ctx, q, k_new, v_new, kv, table, n_heads, scale, window, c
     value, portions to the one that shares key blocks among 64 queries."""
     n1 = ctx.n_entries if ctx.decode_only else ctx.n_single
     if n1 == q.shape[0]:
-        return kernels.attention_f32_decode(q, kv, ctx.positions, table, n_heads, scale, window, n_splits=float32_splits(ctx, n1, n_heads),
+        return kernels.attention_tokens(q, kv, ctx.positions, table, n_heads, scale, window, n_splits=token_splits(ctx, n1, n_heads),
                                             k_new=k_new, v_new=v_new, chunk=chunk, gate=gate)
-    import torch
     out = torch.empty_like(q, memory_format=torch.contiguous_format)
     if k_new is not None:
         kernels.kv_store(k_new[n1:], v_new[n1:], ctx.token_entry[n1:], ctx.positions[n1:], table, kv)
     if n1:
-        kernels.attention_f32_decode(q[:n1], kv, ctx.positions[:n1], table, n_heads, scale, window, n_splits=float32_splits(ctx, n1, n_heads),
+        kernels.attention_tokens(q[:n1], kv, ctx.positions[:n1], table, n_heads, scale, window, n_splits=token_splits(ctx, n1, n_heads),
                                      out=out[:n1], k_new=None if k_new is None else k_new[:n1], v_new=None if v_new is None else v_new[:n1],
                                      chunk=chunk, gate=None if gate is None else gate[:n1])
     # A tile's keys are shared among blocks while tiles x heads leave SMs without their three blocks: few in all, or long
@@ -164,11 +186,13 @@ def float32_attention(ctx, q, k_new, v_new, kv, table, n_heads, scale, window, c
                                         n_splits=min(splits, max(1, ctx.split_context // 128)), chunk=chunk, gate=gate)
 
 
-def float32_splits(ctx, n_tokens, n_heads, keys_per_block=128):
+def token_splits(ctx, n_tokens, n_heads, keys_per_block=128):
     """Blocks that share a token's keys: as many as are resident at once (two an SM; a second wave costs more than longer
-    pieces: 200 (token, head) pairs of 70 keys in one and in two pieces), each with at least two rounds of its eight warps."""
+    pieces: 200 (token, head) pairs of 70 keys in one and in two pieces 5.6 and 10.9 us), each with at least half a round of
+    its eight warps, and at most four but for long contexts (25 pairs, 1,000 keys of bfloat16: 15.6, 7.3, 4.0 and 7.4 us in
+    1, 2, 4 and 8)."""
     want = 2 * ctx.sm_count // max(1, n_tokens * n_heads)
-    return max(1, min(want, -(-ctx.split_context // keys_per_block), 8))
+    return max(1, min(want, -(-ctx.split_context // keys_per_block), 4 if ctx.split_context <= 4096 else 8))
 
 
 def general_attention(ctx, q, kv, table, n_heads, scale, window, kv_heads, head_dim, value_dim, exact_weights=False, gate=None, **mask):
@@ -181,7 +205,6 @@ def general_attention(ctx, q, kv, table, n_heads, scale, window, kv_heads, head_
             not kernels.attention_prefill_padded_supported(n_heads, kv_heads, head_dim, value_dim, q.dtype):
         return kernels.attention_rows(q, kv, ctx.token_entry, ctx.positions, table, n_heads, scale, window,
                                       n_splits=ctx.key_splits(n_heads), gate=gate, **mask, **sizes)
-    import torch
     out = torch.empty((q.shape[0], n_heads * value_dim), dtype=q.dtype, device=q.device)
     n1 = ctx.n_single
     if n1:

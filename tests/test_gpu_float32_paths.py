@@ -100,7 +100,7 @@ SIZES = [(3, 3, 16, 16), (4, 2, 48, 8), (5, 5, 64, 16), (6, 2, 32, 12), (2, 1, 1
 def test_prompt_attention(K, heads, kv_heads, d, page, window):
     lengths, new = [64, 1, 65, 200, 331], [64, 1, 1, 129, 64]
     c = paged_case(K, torch.float32, heads, kv_heads, d, page, lengths, new, window, 1)
-    assert K.attention_f32_supported(c["q"], c["cache"])
+    assert K.attention_cores_supported(c["q"], c["cache"])
     start = torch.tensor([0] + torch.tensor(new).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
     pos0 = torch.tensor([n - m for n, m in zip(lengths, new)], dtype=torch.int32, device=DEV)
     for splits in (1, 2, 3, 4):
@@ -114,26 +114,55 @@ def test_prompt_attention(K, heads, kv_heads, d, page, window):
     assert (got - want).abs().max() < 2e-5 and K.read_error_flag(DEV) == 0
 
 
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-5), (torch.bfloat16, 2e-2)])
 @pytest.mark.parametrize("heads,kv_heads,d,page", SIZES)
 @pytest.mark.parametrize("splits", [1, 3, 8])
-def test_single_token_attention(K, heads, kv_heads, d, page, splits):
+def test_single_token_attention(K, heads, kv_heads, d, page, splits, dtype, tol):
+    if d * dtype.itemsize % 16:
+        pytest.skip("rows that are not whole 16-byte pieces")
     lengths = [1, 2, 63, 64, 65, 300, 517]
     for window, chunk in ((None, None), (70, None), (None, 40)):
-        c = paged_case(K, torch.float32, heads, kv_heads, d, page, lengths, [1] * len(lengths), window, 1, store=False)
+        c = paged_case(K, dtype, heads, kv_heads, d, page, lengths, [1] * len(lengths), window, 1, store=False)
+        assert K.attention_cores_supported(c["q"], c["cache"])
         k = c["packed"][:, heads * d:(heads + kv_heads) * d]
         v = c["packed"][:, (heads + kv_heads) * d:]
         stored = c["cache"].clone()
         K.kv_store(k, v, c["ent"], c["pos"], c["table"], stored)
-        gate = torch.randn(len(lengths), heads, device=DEV) if chunk else None
-        got = K.attention_f32_decode(c["q"], c["cache"], c["pos"], c["table"], heads, c["scale"], window, n_splits=splits, k_new=k, v_new=v,
-                                     chunk=chunk, gate=gate)
+        gate = torch.randn(len(lengths), heads, device=DEV).to(dtype) if chunk else None
+        got = K.attention_tokens(c["q"], c["cache"], c["pos"], c["table"], heads, c["scale"], window, n_splits=splits, k_new=k, v_new=v,
+                                 chunk=chunk, gate=gate)
         assert torch.equal(torch.nan_to_num(c["cache"], nan=5.0), torch.nan_to_num(stored, nan=5.0)), "the new keys and values are in the cache"
         if chunk is None:
-            assert (got.cpu().double() - c["ref"]).abs().max() < 2e-5
+            assert (got.cpu().double() - c["ref"]).abs().max() < tol
         want = K.attention_rows(c["q"], stored, c["ent"], c["pos"], c["table"], heads, c["scale"], window, chunk=chunk, gate=gate)
-        assert (got - want).abs().max() < 2e-5
-        again = K.attention_f32_decode(c["q"], stored, c["pos"], c["table"], heads, c["scale"], window, n_splits=splits, chunk=chunk, gate=gate)
+        assert (got.float() - want.float()).abs().max() < tol
+        again = K.attention_tokens(c["q"], stored, c["pos"], c["table"], heads, c["scale"], window, n_splits=splits, chunk=chunk, gate=gate)
         assert torch.equal(got, again) and K.read_error_flag(DEV) == 0
+
+
+@pytest.mark.parametrize("heads,kv_heads,d,dtype,tokens,kernel", [
+    (25, 25, 64, torch.bfloat16, 1, "attention_tokens"), (25, 25, 64, torch.bfloat16, 8, "attention_decode"),
+    (10, 2, 64, torch.bfloat16, 8, "attention_tokens"), (3, 3, 16, torch.bfloat16, 5, "attention_tokens"),
+    (25, 25, 64, torch.float32, 8, "attention_tokens"), (2, 1, 132, torch.float32, 3, "attention_rows")])
+def test_which_kernel_a_decode_step_takes(K, monkeypatch, heads, kv_heads, d, dtype, tokens, kernel):
+    """Few pairs, groups and small heads: the kernel of whole rows; the rest as before. Whichever it is, the result is the
+    general kernel's."""
+    from types import SimpleNamespace
+    from damendaemon_b200.engine.context import StepContext
+    from damendaemon_b200.parts import paged_attention as pa
+    lengths = [40 + 7 * i for i in range(tokens)]
+    c = paged_case(K, dtype, heads, kv_heads, d, 16, lengths, [1] * tokens, None, 1, store=False)
+    q, k, v = c["packed"].split([heads * d, kv_heads * d, kv_heads * d], dim=1)
+    ctx = StepContext(tokens, tokens, 0, None, c["pos"], c["ent"], None, None, torch.arange(tokens + 1, dtype=torch.int32, device=DEV), c["pos"],
+                      {"all": c["table"]}, decode_only=True, split_context=1024, n_single=tokens,
+                      runtime=SimpleNamespace(attention="auto", attention_tuning=pa.AttentionTuning()))
+    cache = SimpleNamespace(kv=c["cache"], group=SimpleNamespace(name="all"), writable=True)
+    called = []
+    for name in ("attention_tokens", "attention_decode", "attention_rows"):
+        monkeypatch.setattr(K, name, lambda *a, _f=getattr(K, name), _n=name, **m: (called.append(_n), _f(*a, **m))[1])
+    got = pa.paged_attention(ctx, q, k, v, cache, heads, c["scale"])
+    assert called == [kernel]
+    assert (got.cpu().double() - c["ref"]).abs().max() < (2e-5 if dtype == torch.float32 else 2e-2) and K.read_error_flag(DEV) == 0
 
 
 def test_a_missing_page_is_reported(K):
@@ -141,12 +170,12 @@ def test_a_missing_page_is_reported(K):
     c = paged_case(K, torch.float32, 2, 2, 64, 16, lengths, [1, 1], None, 1)
     table = c["table"].clone()
     table[1, 2] = -1
-    got = K.attention_f32_decode(c["q"], c["cache"], c["pos"], table, 2, c["scale"])
+    got = K.attention_tokens(c["q"], c["cache"], c["pos"], table, 2, c["scale"])
     assert K.read_error_flag(DEV) == 4 and torch.isfinite(got).all()
     start, pos0 = (torch.tensor(x, dtype=torch.int32, device=DEV) for x in ([0, 1, 2], [39, 89]))
     got = K.attention_f32_prompt(c["q"], c["cache"], start, pos0, table, 2, c["scale"])
     assert K.read_error_flag(DEV) == 4 and torch.isfinite(got).all()
     table[0, 2] = 1000
     packed = c["packed"]
-    K.attention_f32_decode(c["q"], c["cache"], c["pos"], table, 2, c["scale"], k_new=packed[:, 128:256], v_new=packed[:, 256:])
+    K.attention_tokens(c["q"], c["cache"], c["pos"], table, 2, c["scale"], k_new=packed[:, 128:256], v_new=packed[:, 256:])
     assert K.read_error_flag(DEV) & 2
