@@ -1154,8 +1154,9 @@ def gemm_simt(a, w, bias=None, residual=None, activation=None, out_dtype=None, o
 
 
 def gemm_split_fits(a, w):
-    """Whether gemm_split takes these operands: float32, 16-byte aligned rows, a reduction width that is a multiple of 4."""
-    return a.dtype == torch.float32 and w.dtype == torch.float32 and not (a.shape[1] % 4 or a.stride(0) % 4 or w.stride(0) % 4) and \
+    """Whether gemm_split takes these operands: float32, 16-byte aligned rows, a reduction width that is a multiple of 4 (and
+    within the 65,535 k blocks of the kernel that writes the tokens' planes)."""
+    return a.dtype == torch.float32 and w.dtype == torch.float32 and a.shape[1] <= 65535 * 32 and not (a.shape[1] % 4 or a.stride(0) % 4 or w.stride(0) % 4) and \
         not (a.data_ptr() | w.data_ptr()) & 15
 
 
