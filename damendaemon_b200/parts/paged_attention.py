@@ -93,11 +93,11 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
         pairs = n_tokens * n_heads
         return pairs >= tune.pages_from_pairs or pairs * ctx.split_context >= tune.pages_from_pair_keys
     def wants_tokens(n_tokens):
-        # few pairs; or heads and sizes that the other decode kernels do not take: key/value groups (8 requests x 25 heads on 5,
+        # few pairs in a step without portions (beside portions the row kernel is as good); or heads and sizes that the other decode kernels do not take: key/value groups (8 requests x 25 heads on 5,
         # 400 keys: 9 us, 32 through the general kernel and the cache write; 32 x 16 on 4, 600 keys: 37 / 69; 8 x 32 heads of 128
         # on 8: 32 / 41) and small heads
         pairs = n_tokens * n_heads
-        few = pairs <= tune.tokens_to_pairs and pairs * ctx.split_context <= tune.tokens_to_pair_keys
+        few = ctx.decode_only and pairs <= tune.tokens_to_pairs and pairs * ctx.split_context <= tune.tokens_to_pair_keys
         return cores and tensor and (few or not kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype))
     if ctx.decode_only and wants_tokens(ctx.n_tokens):
         return kernels.attention_tokens(q, kv, ctx.positions, table, n_heads, scale, window, n_splits=token_splits(ctx, ctx.n_tokens, n_heads),
