@@ -1,19 +1,14 @@
-// Paged causal attention for float32 caches: a kernel for prompt portions and one for single tokens. Both take head
-// sizes that are multiples of 4 up to 128, any key/value groups, a window, a chunked mask and a gate per head, with the
-// meaning that attention_rows.cu gives them (that kernel serves all other sizes and options and is the reference of
-// these two). Everything is float32 multiply-add on the CUDA cores: scores, softmax (expf) and the weighted value sum.
+// Paged causal attention of prompt portions over float32 caches: head sizes that are multiples of 4 up to 128, any
+// key/value groups, a window, a chunked mask and a gate per head, with the meaning that attention_rows.cu gives them (that
+// kernel serves all other sizes and options and is the reference; single tokens go to attention_tokens.cu). Everything is
+// float32 multiply-add on the CUDA cores: scores, softmax (expf) and the weighted value sum.
 //
 // The general kernel spends a warp on one query of one head and reads every key and value row again for each of them:
-// 1,100 us for 1,000 tokens x 20 heads of 64, where the multiply-adds alone need 38. Here a block of a prompt owns 64
-// queries of a head and reads each block of 64 keys once for all of them into shared memory (cp.async, the next block's
-// keys under this block's softmax and values, its values under the next scores); a thread holds 4 x 8 scores and 4
-// queries' pieces of the output in registers: 106 us. What bounds it now are the reads of shared memory (12 of 16 bytes
-// for 128 multiply-adds a thread, 56 us) and the few warps that hide them (registers: three blocks an SM). A single
-// token's block reads whole rows by groups of lanes, eight key and eight value rows of a group in flight at once, every
-// group with a running maximum and sum of its own; a token's keys may be cut over the blocks of a cluster, whose results
-// meet in the shared memory of the first (no scratch, no second launch), and the step's own key and value are taken from
-// the projection and written to the cache here: 8 requests x 25 heads, 70 keys, in a graph 5.7 us against 34 for the
-// general kernel, its merge and the cache write; at 1,000 keys 31 us (3.3 TB/s).
+// 1,100 us for 1,000 tokens x 20 heads of 64, where the multiply-adds alone need 38. Here a block owns 64 queries of a head
+// and reads each block of 64 keys once for all of them into shared memory (cp.async, the next block's keys under this
+// block's softmax and values, its values under the next scores); a thread holds 4 x 8 scores and 4 queries' pieces of the
+// output in registers: 106 us. What bounds it now are the reads of shared memory (12 of 16 bytes for 128 multiply-adds a
+// thread, 56 us) and the few warps that hide them (registers: three blocks an SM).
 #include "attention_cores.cuh"
 
 namespace {

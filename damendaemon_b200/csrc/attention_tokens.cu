@@ -8,8 +8,9 @@
 // warp by shuffles, in the block through shared memory). A token's keys may be cut over the blocks of a cluster, whose
 // results meet in the shared memory of the first: no scratch, no second launch. The step's own key and value are taken
 // from the projection and written to the cache here, and all other keys are earlier steps': the first eight rows of every
-// group (512 bytes a lane group of 16 float32; 2,048 keys' worth a block in bfloat16) are requested before the kernel
-// waits for the projection. What bounds it is the chain position -> page -> rows -> merge with few tokens and the
+// group (of heads of 64: 128 keys of a block in float32, 256 in bfloat16) are requested before the kernel waits for the
+// projection. Beside that projection, us: float32, 8 requests x 25 heads at 70 keys 34 -> 6 (the general kernel, its merge
+// and the cache write before); bfloat16, 8 requests x 25 heads on 5 at 400 keys 32 -> 9. What bounds it is the chain position -> page -> rows -> merge with few tokens and the
 // memory's rate with many; figures are beside the rule that chooses it (parts/paged_attention.py).
 #include "attention_cores.cuh"
 

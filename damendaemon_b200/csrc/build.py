@@ -1,7 +1,7 @@
 """Compile the CUDA sources of this folder for sm_100a into shared libraries, on first use.
 
 Two libraries: ``core`` (plain CUDA-core kernels of both engine dtypes: embedding,
-LayerNorm, RMS norm (plain, in groups, blended with the token before), rotary positions, per-head norm, retention, the gated delta rule, latent rows and per-head products, weighted sums of streams, the token-pair embedding, the tanh norm and other row operations, the state-space scan, the gated linear recurrence, time mixing, the matrix memory, the post-norm, float32 GEMM, cache writes, general attention, expert routing, sampling) and ``tensor``
+LayerNorm, RMS norm (plain, in groups, blended with the token before), rotary positions, per-head norm, retention, the gated delta rule, latent rows and per-head products, weighted sums of streams, the token-pair embedding, the tanh norm and other row operations, the state-space scan, the gated linear recurrence, time mixing, the matrix memory, the post-norm, float32 GEMM, also on the tensor cores in three bfloat16 parts, cache writes, general, single-token and float32 prompt attention, expert routing, sampling) and ``tensor``
 (tcgen05/TMA GEMM, tensor-core attention, also over latent rows, and per-head products, bfloat16 only). A float32 engine needs
 only ``core``; what is compiled at the first call is what the model needs.
 
