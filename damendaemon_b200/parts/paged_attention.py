@@ -28,11 +28,6 @@ class AttentionTuning:
     pages_per_block: int = 128            # a block of the page-streaming kernel holds the ids of this many pages
     row_keys_per_block: int = 128         # key split of the row decode kernel: keys per block ...
     row_blocks_per_sm: int = 2            # ... and blocks wanted per SM
-    tokens_to_pairs: int = 50             # bfloat16 steps of at most this many (token, head) pairs: whole rows on the CUDA cores, four
-                                          # blocks a pair, all requested before the projection is done (25 pairs, us beside the product
-                                          # before it, against rows: 100 keys 3.4 / 5.5, 544 keys 3.5 / 6.2, 1,000 keys 4.0 / 6.5; 50
-                                          # pairs at 544 keys 7.0 / 7.6; 100 pairs 13.1 / 10.7, pages 9.6) ...
-    tokens_to_pair_keys: int = 60_000     # ... and at most this many pairs x keys of context (measured up to 25 x 1,000)
 
 
 def prompt_key_block(n_heads, kv_heads, head_dim, page_size, dtype):
@@ -92,14 +87,11 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
     def wants_pages(n_tokens):
         pairs = n_tokens * n_heads
         return pairs >= tune.pages_from_pairs or pairs * ctx.split_context >= tune.pages_from_pair_keys
-    def wants_tokens(n_tokens):
-        # few pairs in a step without portions (beside portions the row kernel is as good); or heads and sizes that the other decode kernels do not take: key/value groups (8 requests x 25 heads on 5,
-        # 400 keys: 9 us, 32 through the general kernel and the cache write; 32 x 16 on 4, 600 keys: 37 / 69; 8 x 32 heads of 128
-        # on 8: 32 / 41) and small heads
-        pairs = n_tokens * n_heads
-        few = ctx.decode_only and pairs <= tune.tokens_to_pairs and pairs * ctx.split_context <= tune.tokens_to_pair_keys
-        return cores and tensor and (few or not kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype))
-    if ctx.decode_only and wants_tokens(ctx.n_tokens):
+    # in bfloat16 for the single tokens of sizes that the tensor-core decode kernels do not take: key/value groups (8 requests x
+    # 25 heads on 5, 400 keys: 9 us, 32 through the general kernel and the cache write; 32 x 16 on 4, 600 keys: 37 / 69; 8 x 32
+    # heads of 128 on 8: 32 / 41) and small heads
+    wants_tokens = cores and tensor and not kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype)
+    if ctx.decode_only and wants_tokens:
         return kernels.attention_tokens(q, kv, ctx.positions, table, n_heads, scale, window, n_splits=token_splits(ctx, ctx.n_tokens, n_heads),
                                         k_new=k_new, v_new=v_new, **masked)
     if ctx.decode_only and tensor and wants_pages(ctx.n_tokens) and \
@@ -123,11 +115,11 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
     # key blocks on a single token (measured with 56 decoding requests beside 8 portions of 249 tokens, 36 layers:
     # 8.3 ms a step through the prompt kernel alone, against 4.5 ms for 2,048 prompt tokens).
     n1 = ctx.n_single if (tcgen05 or mma) and fast and \
-        (wants_tokens(ctx.n_single) or kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype)) else 0
+        (wants_tokens or kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype)) else 0
     out = None
     if n1:
         out = torch.empty((q.shape[0], n_heads * head_dim), dtype=q.dtype, device=q.device)
-        pages = tensor and not wants_tokens(n1) and wants_pages(n1) and \
+        pages = tensor and not wants_tokens and wants_pages(n1) and \
             kernels.attention_decode_pages_supported(n_heads, kv_heads, head_dim, page_size, q.dtype)
         if pages:
             splits = kernels.attention_decode_pages_splits(n1, n_heads, page_size, ctx.split_context, q.device)
@@ -135,7 +127,7 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
         else:
             splits = ctx.key_splits(n_heads, keys_per_block=tune.row_keys_per_block, blocks_per_sm=tune.row_blocks_per_sm,
                                     n_tokens=n1)
-        if wants_tokens(n1):
+        if wants_tokens:
             kernels.attention_tokens(q[:n1], kv, ctx.positions[:n1], table, n_heads, scale, window, n_splits=token_splits(ctx, n1, n_heads),
                                      out=out[:n1], k_new=None if k_new is None else k_new[:n1], v_new=None if v_new is None else v_new[:n1],
                                      chunk=chunk, gate=None if gate is None else gate[:n1])

@@ -141,12 +141,13 @@ def test_single_token_attention(K, heads, kv_heads, d, page, splits, dtype, tol)
 
 
 @pytest.mark.parametrize("heads,kv_heads,d,dtype,tokens,kernel", [
-    (25, 25, 64, torch.bfloat16, 1, "attention_tokens"), (25, 25, 64, torch.bfloat16, 8, "attention_decode"),
+    (25, 25, 64, torch.bfloat16, 1, "attention_decode"), (25, 25, 64, torch.bfloat16, 8, "attention_decode"),
+    (2, 2, 128, torch.bfloat16, 1, "attention_decode"),
     (10, 2, 64, torch.bfloat16, 8, "attention_tokens"), (3, 3, 16, torch.bfloat16, 5, "attention_tokens"),
     (25, 25, 64, torch.float32, 8, "attention_tokens"), (2, 1, 132, torch.float32, 3, "attention_rows")])
 def test_which_kernel_a_decode_step_takes(K, monkeypatch, heads, kv_heads, d, dtype, tokens, kernel):
-    """Few pairs, groups and small heads: the kernel of whole rows; the rest as before. Whichever it is, the result is the
-    general kernel's."""
+    """Groups and small heads: the kernel of whole rows; sizes that the tensor-core decode kernels take go to those, however
+    few tokens there are. Whichever it is, the result is the general kernel's."""
     from types import SimpleNamespace
     from damendaemon_b200.engine.context import StepContext
     from damendaemon_b200.parts import paged_attention as pa
