@@ -55,6 +55,9 @@ constexpr int PROMPT_SPLITS = 4;                            // blocks that may s
 // The blocks of a cluster take a tile's key blocks in turn; what they found meets in the first one's shared memory. (One
 // block a tile left 1.6 of three possible blocks on an SM for 1,000 tokens x 20 heads and the SMs with the last tiles busy
 // twice as long as the others: 148 us.)
+// A key that a query does not see is not part of its sum, whatever its row holds: a weight of zero would make NaN of an
+// infinite value. Blocks of keys that some query of the tile does not see are looked through for such values (each thread
+// its own copies, the answer rides on the barrier that is there anyway) and then added pair by pair.
 template <int D>
 __global__ void __launch_bounds__(THREADS, D <= 64 ? 3 : 1)
 attention_f32_prompt_kernel(const float* q, int q_stride, const float* cache, const int* entry_start, const int* entry_pos0, int n_entries,
@@ -82,7 +85,7 @@ attention_f32_prompt_kernel(const float* q, int q_stride, const float* cache, co
     const int h = blockIdx.x / S % H, kh = h / (H / pages.kv_heads), d = pages.d;
     const int q0 = tile * BQ, rows = min(BQ, len - q0), row0 = entry_start[e] + q0;
     const int pos_first = entry_pos0[e] + q0, pos_last = pos_first + rows - 1;
-    const int kv_lo = mask.first_seen(pos_first);
+    const int kv_lo = mask.first_seen(pos_first), lo_last = mask.first_seen(pos_last);
     const int n_blocks = (pos_last - kv_lo) / BKV + 1;
     const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
     const long long value_plane = pages.value_plane();
@@ -209,7 +212,31 @@ attention_f32_prompt_kernel(const float* q, int q_stride, const float* cache, co
             for (int j = 0; j < 2 * OJ; ++j) mul2(o[i][j], pair_of(corr, corr));
         }
         cp_wait<1>();
-        __syncthreads();                                    // this block's values and weights are there
+        const int first = kv_lo + b * BKV, last = min(first + BKV - 1, pos_last);
+        bool odd = false;
+        if (last > pos_first || first < lo_last) {          // a mask's border runs through the block
+            float test = 0.f;
+            for (int i = tid; i < BKV * NC; i += THREADS) {
+                const float4 v = *reinterpret_cast<const float4*>(sV + i / NC * LD + i % NC * 4);
+                test = fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, fmaf(v.w, 0.f, test))));
+            }
+            odd = test != 0.f;                              // 0, or NaN if some value is not finite
+        }
+        if (__syncthreads_or(odd)) {                        // this block's values and weights are there
+#pragma unroll 1
+            for (int k = 0; k < BKV; ++k)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (first + k < lo[i] || first + k > hi[i]) continue;
+                    const float w = sP[(ty + 16 * i) * LP + k];
+#pragma unroll
+                    for (int j = 0; j < OJ; ++j) {
+                        const Quad v = load_quad(sV + k * LD + 4 * tx + 32 * j);
+                        fma2(o[i][2 * j], pair_of(w, w), v.lo);
+                        fma2(o[i][2 * j + 1], pair_of(w, w), v.hi);
+                    }
+                }
+        } else
 #pragma unroll 2
         for (int k = 0; k < BKV; k += 4) {
             float4 p[4];

@@ -180,3 +180,59 @@ def test_a_missing_page_is_reported(K):
     packed = c["packed"]
     K.attention_tokens(c["q"], c["cache"], c["pos"], table, 2, c["scale"], k_new=packed[:, 128:256], v_new=packed[:, 256:])
     assert K.read_error_flag(DEV) & 2
+
+
+def run_of_entries(dtype, entries, keys, heads, kv_heads, d, page=16, seed=11):
+    """Queries of `entries` requests with `keys` tokens each, their caches and block tables: q [entries * keys, ...] is what a
+    prompt of whole requests brings, its last row of every entry what a decode step brings."""
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    blocks = -(-keys // page)
+    q = torch.randn(entries * keys, heads * d, generator=g, device=DEV).to(dtype)
+    k, v = (torch.randn(entries, keys, kv_heads, d, generator=g, device=DEV).to(dtype) for _ in range(2))
+    table = torch.randperm(entries * blocks, generator=g, device=DEV).to(torch.int32).view(entries, blocks)
+
+    def cache(k, v):
+        pages = torch.zeros(entries * blocks, 2, kv_heads, page, d, dtype=dtype, device=DEV)
+        for side, x in enumerate((k, v)):
+            padded = torch.nn.functional.pad(x, (0, 0, 0, 0, 0, blocks * page - keys)).view(entries, blocks, page, kv_heads, d)
+            pages[table.long(), side] = padded.transpose(2, 3)
+        return pages
+    return q, k, v, table, cache
+
+
+MASKS = [(None, None), (40, None), (None, 48)]
+
+
+def seen(keys, window, chunk):
+    i, j = torch.arange(keys, device=DEV)[:, None], torch.arange(keys, device=DEV)[None, :]
+    visible = j <= i
+    if window:
+        visible &= j > i - window
+    if chunk:
+        visible &= j // chunk == i // chunk
+    return visible
+
+
+@pytest.mark.parametrize("window,chunk", MASKS)
+@pytest.mark.parametrize("heads,kv_heads,d", [(2, 2, 64), (2, 1, 16), (1, 1, 128)])
+def test_a_value_that_is_not_finite_reaches_only_queries_that_see_it(K, heads, kv_heads, d, window, chunk):
+    """Prompts of 150 tokens, each with one infinite or NaN value row at another place: queries that do not see it have the
+    bits of the run without it, queries that do are not finite."""
+    keys, places = 150, [0, 1, 30, 63, 64, 65, 100, 127, 128, 148, 149]
+    q, k, v, table, cache = run_of_entries(torch.float32, len(places), keys, heads, kv_heads, d)
+    start = torch.arange(len(places) + 1, dtype=torch.int32, device=DEV) * keys
+    pos0 = torch.zeros(len(places), dtype=torch.int32, device=DEV)
+    visible = seen(keys, window, chunk)
+    for splits in (1, 3):
+        more = dict(n_splits=splits, chunk=chunk)
+        clean = K.attention_f32_prompt(q, cache(k, v), start, pos0, table, heads, d ** -0.5, window, **more).view(len(places), keys, -1)
+        for value in (float("inf"), -float("inf"), float("nan")):
+            spoilt = v.clone()
+            for e, j in enumerate(places):
+                spoilt[e, j] = value
+            got = K.attention_f32_prompt(q, cache(k, spoilt), start, pos0, table, heads, d ** -0.5, window, **more).view(len(places), keys, -1)
+            for e, j in enumerate(places):
+                sees = visible[:, j]
+                assert torch.equal(got[e, ~sees], clean[e, ~sees])
+                assert not bool(torch.isfinite(got[e, sees]).any())
+    assert K.read_error_flag(DEV) == 0
