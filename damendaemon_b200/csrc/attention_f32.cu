@@ -200,7 +200,7 @@ attention_f32_prompt_kernel(const float* q, int q_stride, const float* cache, co
             float sum = 0.f;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const float p = none ? 0.f : expf(s[i][j] - m_new);
+                const float p = s[i][j] == -CUDART_INF_F ? 0.f : expf(s[i][j] - m_new);     // (a NaN stays one, also where it is alone)
                 sum += p;
                 sP[(ty + 16 * i) * LP + tx + 8 * j] = p;
             }
@@ -292,7 +292,7 @@ attention_f32_prompt_kernel(const float* q, int q_stride, const float* cache, co
             const float ms[4] = {m4.x, m4.y, m4.z, m4.w}, ls[4] = {l4.x, l4.y, l4.z, l4.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                if (ms[i] == -CUDART_INF_F) continue;
+                if (ls[i] == 0.f) continue;                // no key seen there (a sum of NaN counts)
                 const float top = fmaxf(m[i], ms[i]);
                 const float mine = expf(m[i] - top), theirs = expf(ms[i] - top);
                 m[i] = top;

@@ -152,6 +152,10 @@ attention_tokens_kernel(const T* q, const T* k_new, const T* v_new, int q_stride
                 for (int i = 0; i < E; ++i) o[i] = fmaf(p, v[i], o[i]);
             }
             m = top;
+        } else {                                            // no score above -infinity: none at all, or NaN, which must not get lost
+#pragma unroll
+            for (int u = 0; u < BATCH; ++u)
+                if (isnan(s[u])) l = s[u];
         }
         __syncwarp();
         base += WARPS * KEYS;

@@ -236,3 +236,55 @@ def test_a_value_that_is_not_finite_reaches_only_queries_that_see_it(K, heads, k
                 assert torch.equal(got[e, ~sees], clean[e, ~sees])
                 assert not bool(torch.isfinite(got[e, sees]).any())
     assert K.read_error_flag(DEV) == 0
+
+
+@pytest.mark.parametrize("window,chunk", MASKS)
+@pytest.mark.parametrize("heads,kv_heads,d", [(2, 2, 64), (2, 1, 16), (1, 1, 128)])
+def test_a_score_that_is_not_a_number_shows_in_a_prompt(K, heads, kv_heads, d, window, chunk):
+    """One NaN key: every query that sees it has no result, the others have theirs; a NaN query alone has none."""
+    keys, places = 150, [0, 1, 30, 63, 64, 65, 100, 127, 128, 148, 149]
+    q, k, v, table, cache = run_of_entries(torch.float32, len(places), keys, heads, kv_heads, d)
+    start = torch.arange(len(places) + 1, dtype=torch.int32, device=DEV) * keys
+    pos0 = torch.zeros(len(places), dtype=torch.int32, device=DEV)
+    visible, spoilt, odd = seen(keys, window, chunk), k.clone(), q.clone().view(len(places), keys, -1)
+    for e, j in enumerate(places):
+        spoilt[e, j] = odd[e, j] = float("nan")
+    for splits in (1, 2, 4):
+        more = dict(n_splits=splits, chunk=chunk)
+        clean = K.attention_f32_prompt(q, cache(k, v), start, pos0, table, heads, d ** -0.5, window, **more).view(len(places), keys, -1)
+        bad_key = K.attention_f32_prompt(q, cache(spoilt, v), start, pos0, table, heads, d ** -0.5, window, **more).view(len(places), keys, -1)
+        bad_query = K.attention_f32_prompt(odd.view(q.shape), cache(k, v), start, pos0, table, heads, d ** -0.5, window, **more).view(len(places), keys, -1)
+        for e, j in enumerate(places):
+            sees, itself = visible[:, j], torch.arange(keys, device=DEV) == j
+            assert torch.equal(bad_key[e, ~sees], clean[e, ~sees]) and bool(torch.isnan(bad_key[e, sees]).all())
+            assert torch.equal(bad_query[e, ~itself], clean[e, ~itself]) and bool(torch.isnan(bad_query[e, j]).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,kv_heads,d", [(2, 2, 64), (2, 1, 16), (1, 1, 128)])
+def test_a_score_that_is_not_a_number_shows_in_a_single_token(K, heads, kv_heads, d, dtype):
+    """70 requests of 70 keys, request j with a NaN key at j: no result, wherever the key falls among warps, groups of lanes and
+    blocks; in requests of one key as well, and for a NaN query."""
+    for keys in (70, 1):
+        q, k, v, table, cache = run_of_entries(dtype, 70, keys, heads, kv_heads, d)
+        q = q.view(70, keys, -1)[:, -1].contiguous()
+        pos = torch.full((70,), keys - 1, dtype=torch.int32, device=DEV)
+        bad, odd = k.clone(), q.clone()
+        bad[torch.arange(70), torch.arange(70) % keys] = float("nan")
+        odd[::2] = float("nan")
+        for splits in (1, 2, 3, 8):
+            for window in (None, 69):
+                clean = K.attention_tokens(q, cache(k, v), pos, table, heads, d ** -0.5, window, n_splits=splits)
+                got = K.attention_tokens(q, cache(bad, v), pos, table, heads, d ** -0.5, window, n_splits=splits)
+                hidden = window is not None and keys > window                 # then request 0 does not see its NaN key
+                assert bool(torch.isnan(got[1 if hidden else 0:]).all()) and (not hidden or torch.equal(got[0], clean[0]))
+                got = K.attention_tokens(odd, cache(k, v), pos, table, heads, d ** -0.5, window, n_splits=splits)
+                assert bool(torch.isnan(got[::2]).all()) and torch.equal(got[1::2], clean[1::2])
+            # the step's own key, which comes from the projection
+            packed = torch.cat([q, bad[:, -1].reshape(70, -1), v[:, -1].reshape(70, -1)], dim=1)
+            parts = packed.split([heads * d, kv_heads * d, kv_heads * d], dim=1)
+            got = K.attention_tokens(parts[0], cache(k, v), pos, table, heads, d ** -0.5, n_splits=splits, k_new=parts[1], v_new=parts[2])
+            clean = K.attention_tokens(q, cache(k, v), pos, table, heads, d ** -0.5, n_splits=splits)
+            last = torch.arange(70, device=DEV) % keys == keys - 1
+            assert bool(torch.isnan(got[last]).all()) and torch.equal(got[~last], clean[~last])
+    assert K.read_error_flag(DEV) == 0
