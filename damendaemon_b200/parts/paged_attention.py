@@ -77,9 +77,11 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
     k_new, v_new = (k, v) if cache.writable else (None, None)
     fast = runtime.attention != "rows"
     masked = dict(chunk=chunk, gate=gate)      # every kernel takes the chunked mask and the gate on its output
-    # the kernels that read whole rows on the CUDA cores (CUDA tensors only: they ask for the rows' alignment)
-    cores = q.is_cuda and fast and not special and kernels.attention_cores_supported(q, kv, k_new, v_new)
-    if cores and q.dtype == torch.float32:
+    # the kernels that read whole rows on the CUDA cores (CUDA tensors only: they ask for the rows' alignment). For float32 they
+    # serve every step; in bfloat16 one of them takes the single tokens of the sizes that the tensor-core decode kernels refuse
+    def cores():
+        return q.is_cuda and fast and not special and kernels.attention_cores_supported(q, kv, k_new, v_new)
+    if q.dtype == torch.float32 and cores():
         return float32_attention(ctx, q, k_new, v_new, kv, table, n_heads, scale, window, **masked)
     tensor = fast and runtime.attention != "mma" and not special
     # a sink alone (no kept first keys, no cap, no weights in two terms) the tcgen05 prompt kernel takes as well
@@ -87,13 +89,6 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
     def wants_pages(n_tokens):
         pairs = n_tokens * n_heads
         return pairs >= tune.pages_from_pairs or pairs * ctx.split_context >= tune.pages_from_pair_keys
-    # in bfloat16 for the single tokens of sizes that the tensor-core decode kernels do not take: key/value groups (8 requests x
-    # 25 heads on 5, 400 keys: 9 us, 32 through the general kernel and the cache write; 32 x 16 on 4, 600 keys: 37 / 69; 8 x 32
-    # heads of 128 on 8: 32 / 41) and small heads
-    wants_tokens = cores and tensor and not kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype)
-    if ctx.decode_only and wants_tokens:
-        return kernels.attention_tokens(q, kv, ctx.positions, table, n_heads, scale, window, n_splits=token_splits(ctx, ctx.n_tokens, n_heads),
-                                        k_new=k_new, v_new=v_new, **masked)
     if ctx.decode_only and tensor and wants_pages(ctx.n_tokens) and \
             kernels.attention_decode_pages_supported(n_heads, kv_heads, head_dim, page_size, q.dtype):
         # whole pages of a group of heads by TMA; it takes the new keys and values from the projection and writes them
@@ -107,6 +102,11 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
         splits = ctx.key_splits(n_heads, keys_per_block=tune.row_keys_per_block, blocks_per_sm=tune.row_blocks_per_sm)
         return kernels.attention_decode(q, kv, None, ctx.positions, table, n_heads, scale, window,
                                         n_splits=splits, k_new=k_new, v_new=v_new, **masked, **exact)
+    # key/value groups and small heads (8 requests x 25 heads on 5, 400 keys: 9 us, 32 through the general kernel and the cache
+    # write; 32 x 16 on 4, 600 keys: 37 / 69; 8 x 32 heads of 128 on 8: 32 / 41)
+    if ctx.decode_only and tensor and cores():
+        return kernels.attention_tokens(q, kv, ctx.positions, table, n_heads, scale, window, n_splits=token_splits(ctx, ctx.n_tokens, n_heads),
+                                        k_new=k_new, v_new=v_new, **masked)
     tcgen05 = not ctx.decode_only and (tensor or (sink_only and fast and runtime.attention != "mma")) and \
         kernels.attention_prefill_tcgen05_supported(n_heads, kv_heads, head_dim, page_size, q.dtype)
     mma = not tcgen05 and not ctx.decode_only and fast and kernels.attention_prefill_supported(n_heads, kv_heads, head_dim, q.dtype)
@@ -114,20 +114,22 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
     # kernel, the portions to a prompt kernel. A prompt kernel spends a tile of 64 or 128 query rows and a walk over all
     # key blocks on a single token (measured with 56 decoding requests beside 8 portions of 249 tokens, 36 layers:
     # 8.3 ms a step through the prompt kernel alone, against 4.5 ms for 2,048 prompt tokens).
-    n1 = ctx.n_single if (tcgen05 or mma) and fast and \
-        (wants_tokens or kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype)) else 0
+    n1 = ctx.n_single if tcgen05 or mma else 0
+    rows = n1 and kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype)
+    if n1 and not rows and not (tensor and cores()):
+        n1 = 0
     out = None
     if n1:
         out = torch.empty((q.shape[0], n_heads * head_dim), dtype=q.dtype, device=q.device)
-        pages = tensor and not wants_tokens and wants_pages(n1) and \
+        pages = rows and tensor and wants_pages(n1) and \
             kernels.attention_decode_pages_supported(n_heads, kv_heads, head_dim, page_size, q.dtype)
         if pages:
             splits = kernels.attention_decode_pages_splits(n1, n_heads, page_size, ctx.split_context, q.device)
             splits = max(splits, -(-table.shape[1] // tune.pages_per_block))
-        else:
+        elif rows:
             splits = ctx.key_splits(n_heads, keys_per_block=tune.row_keys_per_block, blocks_per_sm=tune.row_blocks_per_sm,
                                     n_tokens=n1)
-        if wants_tokens:
+        if not rows:
             kernels.attention_tokens(q[:n1], kv, ctx.positions[:n1], table, n_heads, scale, window, n_splits=token_splits(ctx, n1, n_heads),
                                      out=out[:n1], k_new=None if k_new is None else k_new[:n1], v_new=None if v_new is None else v_new[:n1],
                                      chunk=chunk, gate=None if gate is None else gate[:n1])

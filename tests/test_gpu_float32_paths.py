@@ -166,6 +166,30 @@ def test_which_kernel_a_decode_step_takes(K, monkeypatch, heads, kv_heads, d, dt
     assert (got.cpu().double() - c["ref"]).abs().max() < (2e-5 if dtype == torch.float32 else 2e-2) and K.read_error_flag(DEV) == 0
 
 
+@pytest.mark.parametrize("heads,kv_heads,d,tokens,single,most", [(25, 25, 64, 8, 8, 1), (25, 25, 64, 1, 1, 1), (2, 2, 128, 2, 2, 1),
+                                                                 (25, 25, 64, 40, 4, 2), (25, 25, 64, 40, 0, 1), (25, 5, 64, 40, 0, 1)])
+def test_steps_of_the_tensor_core_sizes_ask_for_no_other_kernel(K, monkeypatch, heads, kv_heads, d, tokens, single, most):
+    """An eager step asks these questions for every layer, on the host: what a decode step, a mixed one and a prompt may ask
+    about the kernels of sizes that the tensor-core ones refuse is nothing, and about the decode kernels once each."""
+    from types import SimpleNamespace
+    from damendaemon_b200.engine.context import StepContext
+    from damendaemon_b200.parts import paged_attention as pa
+    new = [1] * single + ([tokens - single] if tokens > single else [])
+    c = paged_case(K, torch.bfloat16, heads, kv_heads, d, 16, [40 + n for n in new], new, None, 1, store=False)
+    q, k, v = c["packed"].split([heads * d, kv_heads * d, kv_heads * d], dim=1)
+    start = torch.tensor([0] + torch.tensor(new).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    pos0 = torch.full((len(new),), 40, dtype=torch.int32, device=DEV)
+    ctx = StepContext(tokens, len(new), 0, None, c["pos"], c["ent"], None, None, start, pos0, {"all": c["table"]}, decode_only=tokens == single,
+                      split_context=1024, n_single=single, runtime=SimpleNamespace(attention="auto", attention_tuning=pa.AttentionTuning()))
+    cache = SimpleNamespace(kv=c["cache"], group=SimpleNamespace(name="all"), writable=True)
+    asked = []
+    for name in ("attention_cores_supported", "attention_decode_supported", "attention_decode_pages_supported"):
+        monkeypatch.setattr(K, name, lambda *a, _f=getattr(K, name), _n=name, **m: (asked.append(_n), _f(*a, **m))[1])
+    got = pa.paged_attention(ctx, q, k, v, cache, heads, c["scale"])
+    assert asked.count("attention_cores_supported") == 0 and len(asked) <= most
+    assert (got.cpu().double() - c["ref"]).abs().max() < 2e-2 and K.read_error_flag(DEV) == 0
+
+
 def test_a_missing_page_is_reported(K):
     lengths = [40, 90]
     c = paged_case(K, torch.float32, 2, 2, 64, 16, lengths, [1, 1], None, 1)
