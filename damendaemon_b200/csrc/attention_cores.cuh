@@ -10,13 +10,18 @@ struct Pages {
     const int* block_table;      // [entries, max_blocks]
     int max_blocks, page_size, n_pages, kv_heads, d;
     int page_shift;              // log2 of the page size where that is a power of two, else -1
-    // element offset of a key's row in the cache (its head kh), -1 without a page; the value row lies value_plane() further on
-    __device__ __forceinline__ long long key_row(int entry, int key, int kh) const {
+    // a key's page, as the table has it (negative or past the last page: there is none), and its place in the page
+    struct Place { int page, row; };
+    __device__ __forceinline__ Place place(int entry, int key) const {
         const int blk = page_shift >= 0 ? key >> page_shift : key / page_size;
-        const int page = blk < max_blocks ? block_table[(size_t)entry * max_blocks + blk] : -1;
-        if (page < 0 || page >= n_pages) return -1;
-        return ((long long)page * 2 * kv_heads + kh) * page_size * d + (long long)(key - blk * page_size) * d;
+        return {blk < max_blocks ? block_table[(size_t)entry * max_blocks + blk] : -1, key - blk * page_size};
     }
+    // element offset of the row of head kh there, -1 without a page; the value row lies value_plane() further on
+    __device__ __forceinline__ long long row_at(const Place& at, int kh) const {
+        if (at.page < 0 || at.page >= n_pages) return -1;
+        return at.page * (2 * value_plane()) + (long long)(kh * page_size + at.row) * d;
+    }
+    __device__ __forceinline__ long long key_row(int entry, int key, int kh) const { return row_at(place(entry, key), kh); }
     __device__ __forceinline__ long long value_plane() const { return (long long)kv_heads * page_size * d; }
 };
 

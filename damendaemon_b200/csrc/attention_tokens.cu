@@ -10,8 +10,11 @@
 // from the projection and written to the cache here, and all other keys are earlier steps': the first eight rows of every
 // group (of heads of 64: 128 keys of a block in float32, 256 in bfloat16) are requested before the kernel waits for the
 // projection. Beside that projection, us: float32, 8 requests x 25 heads at 70 keys 34 -> 6 (the general kernel, its merge
-// and the cache write before); bfloat16, 8 requests x 25 heads on 5 at 400 keys 32 -> 9. What bounds it is the chain position -> page -> rows -> merge with few tokens and the
-// memory's rate with many; figures are beside the rule that chooses it (parts/paged_attention.py).
+// and the cache write before); bfloat16, 8 requests x 25 heads on 5 at 400 keys 32 -> 6.4. What bounds it is the chain
+// position -> page -> rows -> merge with few tokens; with long contexts a batch's instructions and the wait for its rows,
+// which two blocks an SM do not hide: bfloat16, 8 requests x 32 heads of 128 on 8, 4,000 and 16,000 keys 99 and 374 (general
+// kernel 175 and 618), float32 180 and 709 (797 for the longer); 8 x 25 heads of 64 in float32, 4,000 keys 106 (222). The
+// figures of the rule for the pieces are beside it (parts/paged_attention.py).
 #include "attention_cores.cuh"
 
 namespace {
@@ -74,6 +77,11 @@ attention_tokens_kernel(const T* q, const T* k_new, const T* v_new, int q_stride
     uint4 kv[BATCH], vv[BATCH];
     uint32_t live = 0;                                      // bit u: key u of the batch exists
     auto fetch = [&](int base) {                            // a batch's rows, but for the step's own key's
+        // all pages are asked for before the first of them is looked at (with a look between, the answers come one after the
+        // other), and a key's place in its page is worked out once: a batch of 128 keys of 128 elements takes 2.6 us, 5.7 before
+        Pages::Place place[BATCH];
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) place[u] = pages.place(t, min(base + u * GROUPS, k_end - 1));
         live = 0;
 #pragma unroll
         for (int u = 0; u < BATCH; ++u) {
@@ -84,7 +92,7 @@ attention_tokens_kernel(const T* q, const T* k_new, const T* v_new, int q_stride
                 live |= 1u << u;
                 continue;
             }
-            const long long at = pages.key_row(t, key, kh);
+            const long long at = pages.row_at(place[u], kh);
             if (at < 0) {
                 atomicOr(error_flag, 4);
                 continue;

@@ -183,8 +183,8 @@ def float32_attention(ctx, q, k_new, v_new, kv, table, n_heads, scale, window, c
 def token_splits(ctx, n_tokens, n_heads, keys_per_block=128):
     """Blocks that share a token's keys: as many as are resident at once (two an SM; a second wave costs more than longer
     pieces: 200 (token, head) pairs of 70 keys in one and in two pieces 5.6 and 10.9 us), each with at least half a round of
-    its eight warps, and at most four but for long contexts (25 pairs, 1,000 keys of bfloat16: 15.6, 7.3, 4.0 and 7.4 us in
-    1, 2, 4 and 8)."""
+    its eight warps, and at most four but for long contexts (us in 1 / 2 / 4 / 8 pieces, bfloat16, 25 pairs on 5 heads: 1,000
+    keys 7.8 / 5.2 / 4.3 / 4.8, 16,000 keys 140 / 77 / 42 / 24; 128 pairs of 128 on 32, 16,000 keys 328 / 188 / 193 / 197)."""
     want = 2 * ctx.sm_count // max(1, n_tokens * n_heads)
     return max(1, min(want, -(-ctx.split_context // keys_per_block), 4 if ctx.split_context <= 4096 else 8))
 

@@ -92,6 +92,24 @@ def test_which_float32_products_are_split(K):
     assert torch.equal(linear(auto, shifted, w), K.gemm_simt(shifted, w))
 
 
+def run_of_entries(dtype, entries, keys, heads, kv_heads, d, page=16, seed=11):
+    """Queries of `entries` requests with `keys` tokens each, their caches and block tables: q [entries * keys, ...] is what a
+    prompt of whole requests brings, its last row of every entry what a decode step brings."""
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    blocks = -(-keys // page)
+    q = torch.randn(entries * keys, heads * d, generator=g, device=DEV).to(dtype)
+    k, v = (torch.randn(entries, keys, kv_heads, d, generator=g, device=DEV).to(dtype) for _ in range(2))
+    table = torch.randperm(entries * blocks, generator=g, device=DEV).to(torch.int32).view(entries, blocks)
+
+    def cache(k, v):
+        pages = torch.zeros(entries * blocks, 2, kv_heads, page, d, dtype=dtype, device=DEV)
+        for side, x in enumerate((k, v)):
+            padded = torch.nn.functional.pad(x, (0, 0, 0, 0, 0, blocks * page - keys)).view(entries, blocks, page, kv_heads, d)
+            pages[table.long(), side] = padded.transpose(2, 3)
+        return pages
+    return q, k, v, table, cache
+
+
 SIZES = [(3, 3, 16, 16), (4, 2, 48, 8), (5, 5, 64, 16), (6, 2, 32, 12), (2, 1, 128, 32), (2, 2, 20, 4), (3, 1, 100, 16)]
 
 
@@ -138,6 +156,63 @@ def test_single_token_attention(K, heads, kv_heads, d, page, splits, dtype, tol)
         assert (got.float() - want.float()).abs().max() < tol
         again = K.attention_tokens(c["q"], stored, c["pos"], c["table"], heads, c["scale"], window, n_splits=splits, chunk=chunk, gate=gate)
         assert torch.equal(got, again) and K.read_error_flag(DEV) == 0
+
+
+def plain_decode(q, k, v, heads, lengths, scale):
+    """One query an entry in 64 bits: q [entries, heads * d], k and v [entries, keys, kv_heads, d] with `lengths` keys of each."""
+    q, k, v = q.double().view(len(lengths), heads, -1), k.double(), v.double()
+    rep = heads // k.shape[2]
+    s = torch.einsum("ehd,ekhd->ehk", q, k.repeat_interleave(rep, 2)) * scale
+    s = s.masked_fill(torch.arange(k.shape[1], device=DEV)[None, None] >= torch.tensor(lengths, device=DEV)[:, None, None], float("-inf"))
+    return torch.einsum("ehk,ekhd->ehd", torch.softmax(s, -1), v.repeat_interleave(rep, 2)).reshape(len(lengths), -1)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,kv_heads,d,page", [(4, 1, 64, 16), (2, 2, 48, 24), (2, 1, 128, 64)])
+def test_single_token_attention_over_long_contexts(K, heads, kv_heads, d, page, dtype):
+    """Contexts around and beyond 4,096 keys, where the rule cuts a token's keys into more pieces, pages of a power of two and
+    others; in every number of pieces. Weights and sums are float32: a bfloat16 result is off by its own rounding alone."""
+    from types import SimpleNamespace
+    from damendaemon_b200.parts.paged_attention import token_splits
+    lengths = [4095, 4096, 4097, 9001, 17]
+    q, k, v, table, cache = run_of_entries(dtype, len(lengths), max(lengths), heads, kv_heads, d, page=page)
+    q, cache = q.view(len(lengths), max(lengths), -1)[:, -1].contiguous(), cache(k, v)
+    pos = torch.tensor(lengths, dtype=torch.int32, device=DEV) - 1
+    want = plain_decode(q, k, v, heads, lengths, d ** -0.5)
+    for context, most in ((4096, 4), (4097, 8)):
+        assert token_splits(SimpleNamespace(sm_count=148, split_context=context), len(lengths), heads) == most
+    for splits in (1, 4, 8):
+        got = K.attention_tokens(q, cache, pos, table, heads, d ** -0.5, n_splits=splits)
+        allowed = 2e-6 if dtype == torch.float32 else 2.0 ** -8 * want.abs() + 2e-5
+        assert ((got.double() - want).abs() <= allowed).all()
+    assert K.read_error_flag(DEV) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_long_contexts_are_not_slower_than_through_the_general_kernel(K, dtype):
+    """8 requests x 32 heads of 128 in groups of four at long contexts, which the general kernel read faster while the
+    single-token kernel looked its pages up one after the other."""
+    heads, kv_heads, d, keys = 32, 8, 128, 4000 if dtype == torch.bfloat16 else 8000
+    q, k, v, table, cache = run_of_entries(dtype, 8, keys, heads, kv_heads, d)
+    q, cache = q.view(8, keys, -1)[:, -1].contiguous(), cache(k, v)
+    pos, ent = torch.full((8,), keys - 1, dtype=torch.int32, device=DEV), torch.arange(8, dtype=torch.int32, device=DEV)
+
+    def fastest(call):
+        times = []
+        for _ in range(10):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(10):
+                call()
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    tokens = fastest(lambda: K.attention_tokens(q, cache, pos, table, heads, d ** -0.5))
+    general = fastest(lambda: K.attention_rows(q, cache, ent, pos, table, heads, d ** -0.5, n_splits=10))
+    print(f"{tokens * 100:.1f} us, general kernel {general * 100:.1f} us")
+    assert tokens < general
 
 
 @pytest.mark.parametrize("heads,kv_heads,d,dtype,tokens,kernel", [
@@ -204,24 +279,6 @@ def test_a_missing_page_is_reported(K):
     packed = c["packed"]
     K.attention_tokens(c["q"], c["cache"], c["pos"], table, 2, c["scale"], k_new=packed[:, 128:256], v_new=packed[:, 256:])
     assert K.read_error_flag(DEV) & 2
-
-
-def run_of_entries(dtype, entries, keys, heads, kv_heads, d, page=16, seed=11):
-    """Queries of `entries` requests with `keys` tokens each, their caches and block tables: q [entries * keys, ...] is what a
-    prompt of whole requests brings, its last row of every entry what a decode step brings."""
-    g = torch.Generator(device=DEV).manual_seed(seed)
-    blocks = -(-keys // page)
-    q = torch.randn(entries * keys, heads * d, generator=g, device=DEV).to(dtype)
-    k, v = (torch.randn(entries, keys, kv_heads, d, generator=g, device=DEV).to(dtype) for _ in range(2))
-    table = torch.randperm(entries * blocks, generator=g, device=DEV).to(torch.int32).view(entries, blocks)
-
-    def cache(k, v):
-        pages = torch.zeros(entries * blocks, 2, kv_heads, page, d, dtype=dtype, device=DEV)
-        for side, x in enumerate((k, v)):
-            padded = torch.nn.functional.pad(x, (0, 0, 0, 0, 0, blocks * page - keys)).view(entries, blocks, page, kv_heads, d)
-            pages[table.long(), side] = padded.transpose(2, 3)
-        return pages
-    return q, k, v, table, cache
 
 
 MASKS = [(None, None), (40, None), (None, 48)]
