@@ -74,14 +74,14 @@ __device__ __forceinline__ unsigned long long now_ns() {
 
 template <int D>
 __global__ void __launch_bounds__(WARPS * 32)
-attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const __nv_bfloat16* k_new,
+attention_decode_kernel(const __nv_bfloat16* q, int q_stride, const __nv_bfloat16* k_new,
                         const __nv_bfloat16* v_new, __nv_bfloat16* cache,
-                        const int* __restrict__ tok_entry, const int* __restrict__ tok_pos,
-                        const int* __restrict__ block_table, int max_blocks, __nv_bfloat16* __restrict__ out,
-                        int out_stride, float* __restrict__ part_o, float* __restrict__ part_ml,
-                        int* __restrict__ counters, int H, int P, int n_pages, int window, float scale_log2e,
-                        int* __restrict__ error_flag, int chunk, const __nv_bfloat16* __restrict__ gate, int gate_stride,
-                        int keep_first, float cap_log2e, float scale_over_cap, const float* __restrict__ sink,
+                        const int* tok_entry, const int* tok_pos,
+                        const int* block_table, int max_blocks, __nv_bfloat16* out,
+                        int out_stride, float* part_o, float* part_ml,
+                        int* counters, int H, int P, int n_pages, int window, float scale_log2e,
+                        int* error_flag, int chunk, const __nv_bfloat16* gate, int gate_stride,
+                        int keep_first, float cap_log2e, float scale_over_cap, const float* sink,
                         int exact_weights) {
     constexpr int C = D / 8;            // 16-byte chunks (and lanes) per key row
     constexpr int KPL = 32 / C;         // keys per copy instruction of a warp

@@ -50,12 +50,12 @@ __device__ __forceinline__ float bf16_high(uint32_t v) { return __uint_as_float(
 // block (4 for prompts; 2 for steps of single tokens with at most 32 heads, whose one token fills half a tile of 64).
 template <int VT, int RG>
 __global__ void __launch_bounds__(256)
-attention_latent_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const __nv_bfloat16* __restrict__ cache,
-                        const int* __restrict__ entry_start, const int* __restrict__ entry_pos0, int n_entries,
-                        const int* __restrict__ block_table, int max_blocks, __nv_bfloat16* __restrict__ out,
-                        int out_stride, float* __restrict__ part_o, float* __restrict__ part_ml, int H, int DK, int DV,
-                        int P, int n_pages, float scale_log2e, int n_splits, int* __restrict__ error_flag,
-                        const float* __restrict__ sink, int n_bufs, int window, const __nv_bfloat16* __restrict__ gate,
+attention_latent_kernel(const __nv_bfloat16* q, int q_stride, const __nv_bfloat16* cache,
+                        const int* entry_start, const int* entry_pos0, int n_entries,
+                        const int* block_table, int max_blocks, __nv_bfloat16* out,
+                        int out_stride, float* part_o, float* part_ml, int H, int DK, int DV,
+                        int P, int n_pages, float scale_log2e, int n_splits, int* error_flag,
+                        const float* sink, int n_bufs, int window, const __nv_bfloat16* gate,
                         int gate_stride) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int BQ = RG * 16;
@@ -289,9 +289,9 @@ attention_latent_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const
 // One warp a (token, head): the splits' partial sums, brought to one maximum (the sink's too), added and normed. Lane s
 // holds split s's weight (at most 32 splits); a lane adds four neighbouring columns, 16 bytes a load, several in flight.
 __global__ void __launch_bounds__(128)
-attention_latent_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                              __nv_bfloat16* __restrict__ out, int out_stride, int n_tokens, int H, int DV, int n_splits,
-                              const float* __restrict__ sink, const __nv_bfloat16* __restrict__ gate, int gate_stride) {
+attention_latent_merge_kernel(const float* part_o, const float* part_ml,
+                              __nv_bfloat16* out, int out_stride, int n_tokens, int H, int DV, int n_splits,
+                              const float* sink, const __nv_bfloat16* gate, int gate_stride) {
     dd_launch_dependents();
     dd_grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -336,8 +336,8 @@ attention_latent_merge_kernel(const float* __restrict__ part_o, const float* __r
 // copied behind its outputs. A block: 64 tokens x 128 outputs of one head, the inputs walked in pieces of 32.
 constexpr int PM = 64, PN = 128, PK = 32, PRB = PK * 2 + 16;
 __global__ void __launch_bounds__(128)
-per_head_mma_kernel(const __nv_bfloat16* __restrict__ in, int in_stride, int in_head, const __nv_bfloat16* __restrict__ w,
-                    __nv_bfloat16* __restrict__ out, int out_stride, int out_head, int n, int I, int J, int tail, DdTailTurn turn) {
+per_head_mma_kernel(const __nv_bfloat16* in, int in_stride, int in_head, const __nv_bfloat16* w,
+                    __nv_bfloat16* out, int out_stride, int out_head, int n, int I, int J, int tail, DdTailTurn turn) {
     __shared__ __align__(128) uint8_t sA[2][PM * PRB];
     __shared__ __align__(128) uint8_t sB[2][PN * PRB];
     dd_launch_dependents();

@@ -47,12 +47,12 @@ template <int D> __device__ __forceinline__ uint32_t tile_off(int r, int c) {
 // D, DV: columns of a key and a value tile. PADDED: a key head has dk <= D and a value head dv <= DV elements.
 template <int D, int DV, bool PADDED>
 __global__ void __launch_bounds__(THREADS)
-attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const __nv_bfloat16* __restrict__ cache,
-                         const int* __restrict__ entry_start, const int* __restrict__ entry_pos0, int n_entries,
-                         const int* __restrict__ block_table, int max_blocks, __nv_bfloat16* __restrict__ out,
+attention_prefill_kernel(const __nv_bfloat16* q, int q_stride, const __nv_bfloat16* cache,
+                         const int* entry_start, const int* entry_pos0, int n_entries,
+                         const int* block_table, int max_blocks, __nv_bfloat16* out,
                          int out_stride, int H, int KH, int P, int n_pages, int window, float scale_log2e,
-                         int* __restrict__ error_flag, int chunk, const __nv_bfloat16* __restrict__ gate, int gate_stride,
-                         int keep_first, float cap_log2e, float scale_over_cap, const float* __restrict__ sink,
+                         int* error_flag, int chunk, const __nv_bfloat16* gate, int gate_stride,
+                         int keep_first, float cap_log2e, float scale_over_cap, const float* sink,
                          int exact_weights, int dk_arg, int dv_arg) {
     constexpr int NC = D / 8, NV = DV / 8;    // 16-byte chunks per row
     constexpr int KS = D / 16;                // k-steps over the head dimension

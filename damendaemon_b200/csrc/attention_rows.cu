@@ -61,13 +61,13 @@ template <> struct Vec<__nv_bfloat16> {
 
 template <typename T, int DPL>
 __global__ void __launch_bounds__(WARPS * 32)
-attention_rows_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ cache,
-                      const int* __restrict__ tok_entry, const int* __restrict__ tok_pos,
-                      const int* __restrict__ block_table, int max_blocks,
-                      T* __restrict__ out, int out_stride, float* __restrict__ part_o, float* __restrict__ part_ml,
+attention_rows_kernel(const T* q, int q_stride, const T* cache,
+                      const int* tok_entry, const int* tok_pos,
+                      const int* block_table, int max_blocks,
+                      T* out, int out_stride, float* part_o, float* part_ml,
                       int n_tokens, int H, int KH, int d, int P, int n_pages, int window, float scale,
-                      int n_splits, int* __restrict__ error_flag, int dv, int chunk,
-                      const T* __restrict__ gate, int gate_stride, RowsExtra extra) {
+                      int n_splits, int* error_flag, int dv, int chunk,
+                      const T* gate, int gate_stride, RowsExtra extra) {
     extern __shared__ float q_smem[];
     dd_launch_dependents();
     dd_grid_wait();
@@ -206,9 +206,9 @@ attention_rows_kernel(const T* __restrict__ q, int q_stride, const T* __restrict
 
 template <typename T>
 __global__ void __launch_bounds__(WARPS * 32)
-attention_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                       T* __restrict__ out, int out_stride, int n_tokens, int H, int d, int n_splits,
-                       const T* __restrict__ gate, int gate_stride, const float* __restrict__ sink) {
+attention_merge_kernel(const float* part_o, const float* part_ml,
+                       T* out, int out_stride, int n_tokens, int H, int d, int n_splits,
+                       const T* gate, int gate_stride, const float* sink) {
     dd_launch_dependents();
     dd_grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

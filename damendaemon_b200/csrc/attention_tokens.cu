@@ -48,7 +48,6 @@ template <typename T, int D>
 __global__ void __launch_bounds__(32 * WARPS, 2)
 attention_tokens_kernel(const T* q, const T* k_new, const T* v_new, int q_stride, T* cache, const int* positions, T* out, int out_stride, int H,
                         Pages pages, Mask mask, float scale, const T* gate, int gate_stride, int* error_flag) {
-    // (no __restrict__ on what the kernel before writes: loads through such pointers may be moved above the wait)
     constexpr int E = Piece<T>::N, LANES = D / E, GROUPS = 32 / LANES;      // GROUPS keys a warp reads at once
     constexpr int KEYS = GROUPS * BATCH;                    // keys of a warp's batch
     __shared__ __align__(16) float part_o[WARPS][D];

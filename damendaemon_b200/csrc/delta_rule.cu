@@ -29,12 +29,12 @@ template <int BYTES> __device__ __forceinline__ void dr_cp_async(float* dst, con
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-delta_prepare_kernel(const T* __restrict__ proj, int proj_stride, const T* __restrict__ beta_in, int beta_stride,
-                     const float* __restrict__ step_in, const float* __restrict__ conv_w, int taps,
-                     const float* __restrict__ conv_state, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
-                     const int* __restrict__ tok_entry, const int* __restrict__ entry_start, const int* __restrict__ entry_slot,
-                     float* __restrict__ q_out, float* __restrict__ k_out, float* __restrict__ v_out,
-                     float* __restrict__ decay_out, float* __restrict__ beta_out, int H, int G, int dk, int dv) {
+delta_prepare_kernel(const T* proj, int proj_stride, const T* beta_in, int beta_stride,
+                     const float* step_in, const float* conv_w, int taps,
+                     const float* conv_state, const float* a_log, const float* dt_bias,
+                     const int* tok_entry, const int* entry_start, const int* entry_slot,
+                     float* q_out, float* k_out, float* v_out,
+                     float* decay_out, float* beta_out, int H, int G, int dk, int dv) {
     // A token's work is dealt out over the gridDim.y blocks of its row: the value channels, decays and step sizes element
     // by element over all their threads, the head vectors of q and k a warp each (convolution, silu and the unit norm stay
     // inside the warp). An element is computed by the same instructions wherever it lands.
@@ -91,8 +91,8 @@ delta_prepare_kernel(const T* __restrict__ proj, int proj_stride, const T* __res
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-conv_state_update_kernel(const T* __restrict__ proj, int proj_stride, float* __restrict__ conv_state, int taps,
-                         const int* __restrict__ entry_start, const int* __restrict__ entry_slot, int C) {
+conv_state_update_kernel(const T* proj, int proj_stride, float* conv_state, int taps,
+                         const int* entry_start, const int* entry_slot, int C) {
     dd_launch_dependents();
     dd_grid_wait();
     const int e = blockIdx.y;
@@ -114,9 +114,9 @@ constexpr int DR_TOKENS = 16;          // tokens staged together
 
 template <int LPC>
 __global__ void __launch_bounds__(DR_THREADS)
-delta_rule_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                  const float* __restrict__ decay, const float* __restrict__ beta, const int* __restrict__ entry_start,
-                  const int* __restrict__ entry_slot, float* __restrict__ state, float* __restrict__ out,
+delta_rule_kernel(const float* q, const float* k, const float* v,
+                  const float* decay, const float* beta, const int* entry_start,
+                  const int* entry_slot, float* state, float* out,
                   int H, int G, int dk, int dv) {
     constexpr int DKP = 8 * LPC, COLS = DR_THREADS / LPC;
     constexpr int BUF = DR_TOKENS * (3 * DKP + COLS) + DR_TOKENS;       // floats of one buffer: q, k, decay, v, beta
@@ -245,8 +245,8 @@ delta_rule_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
 
 template <typename TO>
 __global__ void __launch_bounds__(128)
-delta_finish_kernel(const float* __restrict__ o, const float* __restrict__ gate, const float* __restrict__ weight,
-                    TO* __restrict__ out, int out_stride, int n, int H, int dv, float eps) {
+delta_finish_kernel(const float* o, const float* gate, const float* weight,
+                    TO* out, int out_stride, int n, int H, int dv, float eps) {
     dd_launch_dependents();
     dd_grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -7,24 +7,34 @@
 
 namespace {
 __global__ void __launch_bounds__(256)
-weighted_sum4_kernel(const float4* __restrict__ stack, size_t plane4, const float* __restrict__ w, int n,
-                     float4* __restrict__ out, size_t count4) {
+weighted_sum4_kernel(const float4* stack, size_t plane4, const float* w, int n,
+                     float4* out, size_t count4) {
     dd_launch_dependents();
     dd_grid_wait();
     const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
     if (i >= count4) return;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int j = 0; j < n; ++j) {
-        const float4 v = stack[(size_t)j * plane4 + i];
-        const float f = w[j];
-        acc.x = fmaf(f, v.x, acc.x); acc.y = fmaf(f, v.y, acc.y); acc.z = fmaf(f, v.z, acc.z); acc.w = fmaf(f, v.w, acc.w);
+    for (int j0 = 0; j0 < n; j0 += 4) {                      // four planes requested together, added in order
+        float4 v[4];
+        float f[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (j0 + u >= n) break;
+            v[u] = stack[(size_t)(j0 + u) * plane4 + i];
+            f[u] = w[j0 + u];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (j0 + u >= n) break;
+            acc.x = fmaf(f[u], v[u].x, acc.x); acc.y = fmaf(f[u], v[u].y, acc.y); acc.z = fmaf(f[u], v[u].z, acc.z); acc.w = fmaf(f[u], v[u].w, acc.w);
+        }
     }
     out[i] = acc;
 }
 
 __global__ void __launch_bounds__(256)
-weighted_sum_kernel(const float* __restrict__ stack, size_t plane, const float* __restrict__ w, int n,
-                    float* __restrict__ out, size_t count) {
+weighted_sum_kernel(const float* stack, size_t plane, const float* w, int n,
+                    float* out, size_t count) {
     dd_launch_dependents();
     dd_grid_wait();
     const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
@@ -36,8 +46,8 @@ weighted_sum_kernel(const float* __restrict__ stack, size_t plane, const float* 
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-blend_rows_kernel(T* __restrict__ v, int v_stride, const T* __restrict__ other, int other_stride,
-                  const float* __restrict__ lambda, int rows, int width) {
+blend_rows_kernel(T* v, int v_stride, const T* other, int other_stride,
+                  const float* lambda, int rows, int width) {
     dd_launch_dependents();
     const float lam = lambda[0];
     dd_grid_wait();

@@ -4,10 +4,10 @@
 #include "common.cuh"
 
 template <typename T>
-__global__ void embed_kernel(const int* __restrict__ ids, const int* __restrict__ pos,
-                             const T* __restrict__ wte, const T* __restrict__ wpe,
-                             float* __restrict__ out, int width, int vocab, int n_positions, float scale,
-                             int* __restrict__ error_flag) {
+__global__ void embed_kernel(const int* ids, const int* pos,
+                             const T* wte, const T* wpe,
+                             float* out, int width, int vocab, int n_positions, float scale,
+                             int* error_flag) {
     dd_launch_dependents();
     dd_grid_wait();
     const int row = blockIdx.x;

@@ -5,11 +5,11 @@
 #include "common.cuh"
 
 template <typename T>
-__global__ void embed_pairs_kernel(const int* __restrict__ ids, const int* __restrict__ pos, const int* __restrict__ tok_entry,
-                                   const int* __restrict__ entry_start, const int* __restrict__ entry_slot,
-                                   const T* __restrict__ tokens, const T* __restrict__ pairs, int* __restrict__ last_id,
-                                   float* __restrict__ out, int width, int vocab, int buckets, long long mul_prev,
-                                   long long mul_cur, int* __restrict__ error_flag) {
+__global__ void embed_pairs_kernel(const int* ids, const int* pos, const int* tok_entry,
+                                   const int* entry_start, const int* entry_slot,
+                                   const T* tokens, const T* pairs, int* last_id,
+                                   float* out, int width, int vocab, int buckets, long long mul_prev,
+                                   long long mul_cur, int* error_flag) {
     dd_launch_dependents();
     dd_grid_wait();
     __shared__ int row_of_pair;
@@ -37,7 +37,19 @@ __global__ void embed_pairs_kernel(const int* __restrict__ ids, const int* __res
     const T* a = tokens + (size_t)id * width;
     const T* b = pairs + (size_t)row_of_pair * width;
     float* o = out + (size_t)t * width;
-    for (int c = threadIdx.x; c < width; c += blockDim.x) o[c] = dd_to_f32(a[c]) + dd_to_f32(b[c]);
+    constexpr int P = 4;                         // elements of a thread that are requested before the first of them is written
+    for (int c0 = threadIdx.x; c0 < width; c0 += P * blockDim.x) {
+        float x[P], y[P];
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const int c = c0 + p * blockDim.x;
+            x[p] = c < width ? dd_to_f32(a[c]) : 0.f;
+            y[p] = c < width ? dd_to_f32(b[c]) : 0.f;
+        }
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+            if (c0 + p * blockDim.x < width) o[c0 + p * blockDim.x] = x[p] + y[p];
+    }
 }
 
 // last_id: int32 [slots]; pairs: [buckets + 1, width] in the token table's dtype.

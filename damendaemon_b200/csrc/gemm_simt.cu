@@ -11,10 +11,10 @@ constexpr int BM = 64, BN = 64, BK = 16, THREADS = 256;
 
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(THREADS)
-gemm_simt_kernel(const TI* __restrict__ A, int lda, const TI* __restrict__ W, int ldw,
-                 const float* __restrict__ bias, const float* residual, int ldr,
+gemm_simt_kernel(const TI* A, int lda, const TI* W, int ldw,
+                 const float* bias, const float* residual, int ldr,
                  TO* C, int ldc, int M, int N, int K, int act,
-                 const int* __restrict__ tile_group, long long group_stride, const float* __restrict__ row_scale) {
+                 const int* tile_group, long long group_stride, const float* row_scale) {
     __shared__ float As[BK][BM + 4];
     __shared__ float Ws[BK][BN + 4];
     dd_launch_dependents();
@@ -94,8 +94,8 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool live
 
 template <int MR, int RB_N, typename TO>
 __global__ void __launch_bounds__(RB_THREADS)
-gemm_simt_rows_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw,
-                      const float* __restrict__ bias, const float* residual, int ldr,
+gemm_simt_rows_kernel(const float* A, int lda, const float* W, int ldw,
+                      const float* bias, const float* residual, int ldr,
                       TO* C, int ldc, int M, int N, int K, int act) {
     constexpr int PER = MR * RB_N / RB_THREADS;             // rows of A per thread (1 to 8)
     static_assert(PER >= 1 && MR * RB_N % RB_THREADS == 0, "a thread owns whole rows");
@@ -183,8 +183,8 @@ constexpr int BG = 128, BG_K = 16, BG_LD = BG_K + 4, BG_STAGES = 3, BG_THREADS =
 constexpr int BG_SMEM = BG_STAGES * 2 * BG * BG_LD * 4;
 
 __global__ void __launch_bounds__(BG_THREADS)
-gemm_simt_big_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw,
-                     const float* __restrict__ bias, const float* residual, int ldr,
+gemm_simt_big_kernel(const float* A, int lda, const float* W, int ldw,
+                     const float* bias, const float* residual, int ldr,
                      float* C, int ldc, int M, int N, int K, int act) {
     extern __shared__ __align__(16) float big_smem[];
     float (*As)[BG][BG_LD] = reinterpret_cast<float (*)[BG][BG_LD]>(big_smem);

@@ -18,9 +18,9 @@ constexpr int WARPS = 8;
 
 template <typename T>
 __global__ void __launch_bounds__(WARPS * 32)
-head_norm_rotary_kernel(T* __restrict__ q, T* __restrict__ k, int stride, const int* __restrict__ positions,
-                        const float* __restrict__ freqs, const float* __restrict__ q_weight,
-                        const float* __restrict__ k_weight, float eps, int q_heads, int k_heads, int head_dim,
+head_norm_rotary_kernel(T* q, T* k, int stride, const int* positions,
+                        const float* freqs, const float* q_weight,
+                        const float* k_weight, float eps, int q_heads, int k_heads, int head_dim,
                         int n_pairs, int interleaved, int heads_per_block) {
     extern __shared__ float staged[];             // [n_pairs] cosines, [n_pairs] sines, [WARPS][head_dim] a head per warp
     float* cosines = staged;
@@ -102,9 +102,9 @@ template <> struct Piece<__nv_bfloat16> {
 // computed once; one pass of the block covers THREADS / G heads. About a thirteenth of the general kernel's instructions.
 template <typename T, int G>
 __global__ void __launch_bounds__(WARPS * 32)
-head_norm_rotary_pieces_kernel(T* __restrict__ q, T* __restrict__ k, int stride, const int* __restrict__ positions,
-                               const float* __restrict__ freqs, const float* __restrict__ q_weight,
-                               const float* __restrict__ k_weight, float eps, int q_heads, int k_heads, int head_dim,
+head_norm_rotary_pieces_kernel(T* q, T* k, int stride, const int* positions,
+                               const float* freqs, const float* q_weight,
+                               const float* k_weight, float eps, int q_heads, int k_heads, int head_dim,
                                int n_pairs, int heads_per_block) {
     constexpr int V = Piece<T>::N;
     extern __shared__ __align__(16) float table[];       // [n_pairs] cosines, [n_pairs] sines

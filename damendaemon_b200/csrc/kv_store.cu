@@ -8,11 +8,11 @@
 #include "common.cuh"
 
 template <typename T>
-__global__ void kv_store_kernel(const T* __restrict__ k_src, const T* __restrict__ v_src, int src_stride,
-                                const int* __restrict__ tok_entry, const int* __restrict__ tok_pos,
-                                const int* __restrict__ block_table, int max_blocks,
-                                T* __restrict__ cache, int n_pages, int kv_heads, int page_size, int head_dim,
-                                int v_dim, int* __restrict__ error_flag) {
+__global__ void kv_store_kernel(const T* k_src, const T* v_src, int src_stride,
+                                const int* tok_entry, const int* tok_pos,
+                                const int* block_table, int max_blocks,
+                                T* cache, int n_pages, int kv_heads, int page_size, int head_dim,
+                                int v_dim, int* error_flag) {
     dd_launch_dependents();
     // positions, entries and the block table are the step's inputs: the page is known before the projection has finished
     const int t = blockIdx.x;

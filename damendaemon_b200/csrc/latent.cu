@@ -18,14 +18,32 @@
 #include "common.cuh"
 
 namespace {
+// out[c] = in[c] * r * weight[c], four elements of a thread requested before the first of them is written
 template <typename T>
-__global__ void __launch_bounds__(128)
-latent_prepare_kernel(T* __restrict__ q, int q_stride, int H, int dk, int dr, const T* __restrict__ down, int down_stride,
-                      int R, const float* __restrict__ weight, float eps, const float* __restrict__ freqs, int n_pairs,
-                      const int* __restrict__ tok_entry, const int* __restrict__ tok_pos, const int* __restrict__ block_table,
-                      int max_blocks, T* __restrict__ cache, int n_pages, int page_size, int* __restrict__ error_flag,
-                      int interleaved, const T* __restrict__ second, int second_stride, int S,
-                      const float* __restrict__ second_weight, T* __restrict__ second_out, int second_out_stride) {
+__device__ __forceinline__ void scale_row(const T* in, T* out, int n, float r, const float* weight) {
+    for (int c0 = threadIdx.x; c0 < n; c0 += 4 * 128) {
+        float x[4], w[4];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const int c = c0 + 128 * p;
+            x[p] = c < n ? dd_to_f32(in[c]) : 0.f;
+            w[p] = c < n ? weight[c] : 0.f;
+        }
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+            if (c0 + 128 * p < n) out[c0 + 128 * p] = dd_from_f32<T>(x[p] * r * w[p]);
+    }
+}
+
+// (sixteen blocks an SM: with four registers more, 2,048 rows took 14.3 instead of 10.1 us)
+template <typename T>
+__global__ void __launch_bounds__(128, 16)
+latent_prepare_kernel(T* q, int q_stride, int H, int dk, int dr, const T* down, int down_stride,
+                      int R, const float* weight, float eps, const float* freqs, int n_pairs,
+                      const int* tok_entry, const int* tok_pos, const int* block_table,
+                      int max_blocks, T* cache, int n_pages, int page_size, int* error_flag,
+                      int interleaved, const T* second, int second_stride, int S,
+                      const float* second_weight, T* second_out, int second_out_stride) {
     __shared__ float scratch[4];
     __shared__ float cs[2 * 128];                   // cosines, then sines, of this token's angles
     dd_launch_dependents();
@@ -60,8 +78,7 @@ latent_prepare_kernel(T* __restrict__ q, int q_stride, int H, int dk, int dr, co
         if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = sum;
         __syncthreads();
         const float r = 1.0f / sqrtf((scratch[0] + scratch[1] + scratch[2] + scratch[3]) / (float)S + eps);
-        for (int c = threadIdx.x; c < S; c += 128)
-            second_out[(size_t)t * second_out_stride + c] = dd_from_f32<T>(dd_to_f32(from[c]) * r * second_weight[c]);
+        scale_row(from, second_out + (size_t)t * second_out_stride, S, r, second_weight);
         __syncthreads();
     }
     if (page < 0 || page >= n_pages) {
@@ -93,7 +110,7 @@ constexpr int PH_TOKENS = 8;
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-per_head_linear_kernel(const T* __restrict__ in, int in_stride, int in_head, const T* __restrict__ w, T* __restrict__ out,
+per_head_linear_kernel(const T* in, int in_stride, int in_head, const T* w, T* out,
                        int out_stride, int out_head, int n, int I, int J, int tail, int j_per_block, DdTailTurn turn) {
     extern __shared__ float rows[];                 // [PH_TOKENS][I]
     dd_launch_dependents();

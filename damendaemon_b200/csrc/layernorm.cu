@@ -20,9 +20,9 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 // Rows up to THREADS * PER elements are read once and kept in registers; wider rows are re-read.
 template <typename TO, int THREADS, int PER>
 __global__ void __launch_bounds__(THREADS)
-layernorm_kernel(const float* __restrict__ x, const int* __restrict__ row_index,
-                 const float* __restrict__ gamma, const float* __restrict__ beta,
-                 TO* __restrict__ out, int width, float eps) {
+layernorm_kernel(const float* x, const int* row_index,
+                 const float* gamma, const float* beta,
+                 TO* out, int width, float eps) {
     __shared__ float scratch[THREADS / 32];
     dd_launch_dependents();
     dd_grid_wait();
@@ -93,9 +93,9 @@ template <> struct Pack4<__nv_bfloat16> {
 
 template <typename TO, int VPT>
 __global__ void __launch_bounds__(128)
-layernorm_vec_kernel(const float* __restrict__ x, const int* __restrict__ row_index,
-                     const float* __restrict__ gamma, const float* __restrict__ beta,
-                     TO* __restrict__ out, int width, float eps) {
+layernorm_vec_kernel(const float* x, const int* row_index,
+                     const float* gamma, const float* beta,
+                     TO* out, int width, float eps) {
     __shared__ float scratch[4];
     dd_launch_dependents();
     const int row = blockIdx.x;

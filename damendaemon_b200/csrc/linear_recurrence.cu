@@ -19,9 +19,9 @@ __device__ __forceinline__ float rg_softplus(float x) { return x > 20.f ? x : lo
 __device__ __forceinline__ float rg_sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 __global__ void __launch_bounds__(RG_OUTS)
-recurrence_gates_kernel(const float* __restrict__ u, const float* __restrict__ wa, const float* __restrict__ ba,
-                        const float* __restrict__ wi, const float* __restrict__ bi, const float* __restrict__ lam, float gain,
-                        float* __restrict__ a_out, float* __restrict__ drive_out, int n_tokens, int width, int bw) {
+recurrence_gates_kernel(const float* u, const float* wa, const float* ba,
+                        const float* wi, const float* bi, const float* lam, float gain,
+                        float* a_out, float* drive_out, int n_tokens, int width, int bw) {
     __shared__ float us[RG_TOKENS][RG_K];
     __shared__ float was[RG_OUTS][RG_K + 1];
     __shared__ float wis[RG_OUTS][RG_K + 1];
@@ -77,9 +77,9 @@ constexpr int LS_TOKENS = 16;     // tokens whose operands a thread of the scan 
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-linear_scan_kernel(const float* __restrict__ a, const float* __restrict__ drive, const T* __restrict__ y, int y_stride,
-                   const int* __restrict__ entry_start, const int* __restrict__ entry_slot, float* __restrict__ state,
-                   T* __restrict__ out, int out_stride, int width, int act) {
+linear_scan_kernel(const float* a, const float* drive, const T* y, int y_stride,
+                   const int* entry_start, const int* entry_slot, float* state,
+                   T* out, int out_stride, int width, int act) {
     dd_launch_dependents();
     const int e = blockIdx.y, c = blockIdx.x * 128 + threadIdx.x;
     if (c >= width) return;
@@ -126,9 +126,9 @@ linear_scan_kernel(const float* __restrict__ a, const float* __restrict__ drive,
 constexpr int RG_FEW = 16, RG_FEW_OUTS = 32;
 
 __global__ void __launch_bounds__(RG_FEW * RG_FEW_OUTS)
-recurrence_gates_few_kernel(const float* __restrict__ u, const float* __restrict__ wa, const float* __restrict__ ba,
-                            const float* __restrict__ wi, const float* __restrict__ bi, const float* __restrict__ lam, float gain,
-                            float* __restrict__ a_out, float* __restrict__ drive_out, int n_tokens, int width, int bw) {
+recurrence_gates_few_kernel(const float* u, const float* wa, const float* ba,
+                            const float* wi, const float* bi, const float* lam, float gain,
+                            float* a_out, float* drive_out, int n_tokens, int width, int bw) {
     extern __shared__ float us[];                   // [n_tokens][bw]
     __shared__ float was[2][RG_FEW_OUTS][RG_K + 1];
     __shared__ float wis[2][RG_FEW_OUTS][RG_K + 1];

@@ -56,9 +56,9 @@ __device__ __forceinline__ MemoryGates mm_gates(float i, float f, float before, 
 constexpr int MG_TOKENS = 128;
 
 __global__ void __launch_bounds__(MG_TOKENS)
-memory_gates_kernel(const float* __restrict__ z, int z_stride, float cap, const int* __restrict__ entry_start,
-                    const int* __restrict__ entry_slot, float* __restrict__ peak, float* __restrict__ fade,
-                    float* __restrict__ take, float* __restrict__ floor_out, int H) {
+memory_gates_kernel(const float* z, int z_stride, float cap, const int* entry_start,
+                    const int* entry_slot, float* peak, float* fade,
+                    float* take, float* floor_out, int H) {
     __shared__ __align__(16) float2 logs[MG_TOKENS];     // (i, f) of a token
     __shared__ float maxima[MG_TOKENS + 1];              // M before the first token, then after every one
     dd_launch_dependents();
@@ -124,9 +124,9 @@ __device__ __forceinline__ float4 mm_load4(const T* row, int c, int n) {
 // A thread owns four neighbouring elements of a head's q, k or v; the blocks of grid column t share token t.
 template <typename T, bool WIDE>
 __global__ void __launch_bounds__(256)
-memory_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int stride, float q_scale,
-                      int silu, const float* __restrict__ take, float* __restrict__ q_out, float* __restrict__ k_out,
-                      float* __restrict__ v_out, int H, int dk, int dv, int ones, int qk_row, int v_row) {
+memory_prepare_kernel(const T* q, const T* k, const T* v, int stride, float q_scale,
+                      int silu, const float* take, float* q_out, float* k_out,
+                      float* v_out, int H, int dk, int dv, int ones, int qk_row, int v_row) {
     dd_launch_dependents();
     dd_grid_wait();
     const int t = blockIdx.x, qk4 = qk_row / 4, v4 = v_row / 4;
@@ -386,8 +386,8 @@ struct StepArgs {
 constexpr int ST_THREADS = 256, ST_AHEAD = 2;
 template <typename T, int LPC, bool FUSED>
 __global__ void __launch_bounds__(ST_THREADS)
-memory_step_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ gate,
-                   T* __restrict__ out, const StepArgs a) {
+memory_step_kernel(const T* q, const T* k, const T* v, const T* gate,
+                   T* out, const StepArgs a) {
     constexpr int DKP = 8 * LPC, COLS = ST_THREADS / LPC;
     extern __shared__ __align__(16) float sh[];          // q, k [DKP] each, then v and o of the block's columns
     __shared__ float scratch[8], n_parts[8], parts[8];
@@ -535,7 +535,7 @@ struct FinishArgs {
 // kept in registers (beyond, it reads again).
 template <typename T, int TEAM, int V, int KEEP>
 __global__ void __launch_bounds__(256)
-memory_finish_kernel(const T* __restrict__ gate, T* __restrict__ out, const FinishArgs a) {
+memory_finish_kernel(const T* gate, T* out, const FinishArgs a) {
     __shared__ float scratch[8];
     dd_launch_dependents();
     const int sub = threadIdx.x % TEAM, per_token = a.H / a.heads;

@@ -135,10 +135,10 @@ template <> struct RoutePiece<__nv_bfloat16> {
 // arg-max over the warp, the lowest index winning a tie.
 template <typename T>
 __global__ void __launch_bounds__(128)
-route_by_score_kernel(const T* __restrict__ y, int ldy, const T* __restrict__ router, int ldr, int width, int n_tokens,
+route_by_score_kernel(const T* y, int ldy, const T* router, int ldr, int width, int n_tokens,
                       int n_experts, int top, int groups, int keep, float weight_scale, int gate_row,
-                      int* __restrict__ chosen, float* __restrict__ pair_weight, float* __restrict__ shared_scale,
-                      int softmax, const float* __restrict__ correction, int renormalize) {
+                      int* chosen, float* pair_weight, float* shared_scale,
+                      int softmax, const float* correction, int renormalize) {
     extern __shared__ float route_smem[];        // [E] choice scores, [E] scores, [groups] worths, [4][rows] the warps' sums
     dd_launch_dependents();
     dd_grid_wait();
@@ -277,7 +277,7 @@ route_by_score_kernel(const T* __restrict__ y, int ldy, const T* __restrict__ ro
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-gather_rows_kernel(const T* __restrict__ x, const int* __restrict__ row_token, T* __restrict__ out, int width) {
+gather_rows_kernel(const T* x, const int* row_token, T* out, int width) {
     dd_launch_dependents();
     dd_grid_wait();
     const int row = blockIdx.x;
@@ -295,8 +295,8 @@ gather_rows_kernel(const T* __restrict__ x, const int* __restrict__ row_token, T
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-gated_unit_kernel(const T* __restrict__ gate_up, int stride, T* __restrict__ out, int out_stride, int rows, int inner,
-                  float limit, float alpha, int form, const float* __restrict__ row_scale) {
+gated_unit_kernel(const T* gate_up, int stride, T* out, int out_stride, int rows, int inner,
+                  float limit, float alpha, int form, const float* row_scale) {
     dd_launch_dependents();
     dd_grid_wait();
     constexpr int V = 16 / sizeof(T);          // elements of a 16-byte piece
@@ -328,8 +328,8 @@ gated_unit_kernel(const T* __restrict__ gate_up, int stride, T* __restrict__ out
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-combine_rows_kernel(const float* __restrict__ y, const int* __restrict__ pair_row, float* __restrict__ stream, int width,
-                    int top, float weight, const float* __restrict__ pair_weight, const T* __restrict__ own) {
+combine_rows_kernel(const float* y, const int* pair_row, float* stream, int width,
+                    int top, float weight, const float* pair_weight, const T* own) {
     dd_launch_dependents();
     dd_grid_wait();
     const int t = blockIdx.x;

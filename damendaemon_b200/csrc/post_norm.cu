@@ -49,7 +49,7 @@ template <int V> __device__ __forceinline__ void pn_store(__nv_bfloat16* p, cons
 
 template <typename T, int V, int KEEP>
 __global__ void __launch_bounds__(PN_THREADS)
-post_norm_kernel(const PostNormArgs a, T* __restrict__ rounded) {
+post_norm_kernel(const PostNormArgs a, T* rounded) {
     __shared__ float scratch[PN_THREADS / 32];
     dd_launch_dependents();
     const int t = blockIdx.x, tid = threadIdx.x;
@@ -140,7 +140,7 @@ post_norm_kernel(const PostNormArgs a, T* __restrict__ rounded) {
 
 template <int V>
 __global__ void __launch_bounds__(256)
-round_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ out, long long n) {
+round_rows_kernel(const float* x, __nv_bfloat16* out, long long n) {
     dd_launch_dependents();
     dd_grid_wait();
     const long long c = ((long long)blockIdx.x * 256 + threadIdx.x) * V;

@@ -103,7 +103,7 @@ template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("c
 // A staged token in shared memory: [R L] rotated q (zeros beyond dk), [R L] rotated scaled k, [COLS] this block's v.
 template <typename T, int R, int L, int WARPS, bool PREPARED>
 __global__ void __launch_bounds__(WARPS * 32)
-retention_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const RetentionArgs a) {
+retention_kernel(const T* q, const T* k, const T* v, const RetentionArgs a) {
     constexpr int THREADS = WARPS * 32, PER_WARP = 32 / L, COLS = WARPS * PER_WARP, DKS = R * L;
     constexpr int PER_TOKEN = 2 * DKS + (COLS + 3) / 4 * 4;
     extern __shared__ __align__(16) float staged[];            // [chunk][PER_TOKEN], twice when PREPARED
@@ -255,8 +255,8 @@ retention_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __re
 // zeroed). A block owns a token and a share of its heads; the token's cosines and sines are computed once.
 template <typename T>
 __global__ void __launch_bounds__(PREP_WARPS * 32)
-retention_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const RetentionArgs a,
-                         float* __restrict__ prepared, int heads_per_block) {
+retention_prepare_kernel(const T* q, const T* k, const T* v, const RetentionArgs a,
+                         float* prepared, int heads_per_block) {
     extern __shared__ float table[];             // [n_pairs] cosines, [n_pairs] sines
     dd_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -296,8 +296,8 @@ retention_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
 // A warp owns a (token, head): the head's o in registers (PER values a lane), one pass.
 template <typename T, int PER>
 __global__ void __launch_bounds__(128)
-retention_finish_kernel(const float* __restrict__ o, const T* __restrict__ gate, int gate_stride, T* __restrict__ out,
-                        int out_stride, int n_tokens, int heads, int dv, float eps, const float* __restrict__ weight) {
+retention_finish_kernel(const float* o, const T* gate, int gate_stride, T* out,
+                        int out_stride, int n_tokens, int heads, int dv, float eps, const float* weight) {
     dd_launch_dependents();
     dd_grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

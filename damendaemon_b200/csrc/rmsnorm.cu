@@ -43,8 +43,8 @@ template <> struct RmsPack4<__nv_bfloat16> {
 // Rows whose width is a multiple of 4 and at most 128 * 4 * VPT: the row in registers as float4.
 template <typename TO, int VPT>
 __global__ void __launch_bounds__(128)
-rmsnorm_vec_kernel(const float* __restrict__ x, const int* __restrict__ row_index, const float* __restrict__ weight,
-                   TO* __restrict__ out, int width, float eps, float offset) {
+rmsnorm_vec_kernel(const float* x, const int* row_index, const float* weight,
+                   TO* out, int width, float eps, float offset) {
     __shared__ float scratch[4];
     dd_launch_dependents();
     const int row = blockIdx.x;
@@ -79,8 +79,8 @@ rmsnorm_vec_kernel(const float* __restrict__ x, const int* __restrict__ row_inde
 
 template <typename TO, int THREADS>
 __global__ void __launch_bounds__(THREADS)
-rmsnorm_kernel(const float* __restrict__ x, const int* __restrict__ row_index, const float* __restrict__ weight,
-               TO* __restrict__ out, int width, float eps, float offset) {
+rmsnorm_kernel(const float* x, const int* row_index, const float* weight,
+               TO* out, int width, float eps, float offset) {
     __shared__ float scratch[THREADS / 32];
     dd_launch_dependents();
     dd_grid_wait();
@@ -99,7 +99,7 @@ constexpr int MAX_GROUPS = 64;
 // by lane in a fixed order, and one thread adds a stretch's pieces: the sum of a row does not depend on which of the two
 // rows it is, nor on what the other one is.
 template <int THREADS>
-__device__ __forceinline__ void group_scales(const float* __restrict__ a, float* ra, const float* __restrict__ b, float* rb,
+__device__ __forceinline__ void group_scales(const float* a, float* ra, const float* b, float* rb,
                                              int width, int groups, float eps, float* partial) {
     const int gw = width / groups, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pieces = groups >= 8 ? 1 : 8 / groups, piece = (gw + pieces - 1) / pieces;
@@ -141,8 +141,8 @@ __device__ __forceinline__ void group_scales(const float* __restrict__ a, float*
 
 template <typename TO, int THREADS>
 __global__ void __launch_bounds__(THREADS)
-rmsnorm_groups_kernel(const float* __restrict__ x, const int* __restrict__ row_index, const float* __restrict__ weight,
-                      TO* __restrict__ out, int width, int groups, float eps, float offset) {
+rmsnorm_groups_kernel(const float* x, const int* row_index, const float* weight,
+                      TO* out, int width, int groups, float eps, float offset) {
     __shared__ float partial[2 * MAX_GROUPS];
     __shared__ float r[MAX_GROUPS];
     dd_launch_dependents();
@@ -163,9 +163,9 @@ __device__ __forceinline__ float blended_value(float n, float p, float mu) { ret
 
 template <typename TO, int THREADS>
 __global__ void __launch_bounds__(THREADS)
-rmsnorm_shift_kernel(const float* __restrict__ x, const float* __restrict__ weight, const float* __restrict__ mu,
-                     float* __restrict__ state, const int* __restrict__ tok_entry, const int* __restrict__ entry_start,
-                     const int* __restrict__ entry_slot, TO* __restrict__ out, int width, int groups, float eps, float offset) {
+rmsnorm_shift_kernel(const float* x, const float* weight, const float* mu,
+                     float* state, const int* tok_entry, const int* entry_start,
+                     const int* entry_slot, TO* out, int width, int groups, float eps, float offset) {
     __shared__ float partial[2 * MAX_GROUPS];
     __shared__ float r_own[MAX_GROUPS], r_other[MAX_GROUPS];
     dd_launch_dependents();

@@ -33,8 +33,8 @@ template <> struct Pair<__nv_bfloat16> {
 // between the loads of a pass.
 template <typename T, bool WORDS>
 __global__ void __launch_bounds__(THREADS)
-rotary_kernel(T* __restrict__ q, T* __restrict__ k, int stride, const int* __restrict__ positions,
-              const float* __restrict__ freqs, float magnitude, int q_heads, int k_heads, int head_dim, int n_pairs,
+rotary_kernel(T* q, T* k, int stride, const int* positions,
+              const float* freqs, float magnitude, int q_heads, int k_heads, int head_dim, int n_pairs,
               int interleaved) {
     extern __shared__ float cs[];                 // [n_pairs] cosines, [n_pairs] sines of this token
     dd_launch_dependents();

@@ -92,9 +92,9 @@ __device__ __forceinline__ float unordered(uint32_t k) {
 }
 
 __global__ void __launch_bounds__(THREADS)
-sample_kernel(const float* __restrict__ logits, int ldl, int V, const float* __restrict__ temperature,
-              const int* __restrict__ top_k, const float* __restrict__ top_p,
-              const double* __restrict__ uniform, int* __restrict__ out) {
+sample_kernel(const float* logits, int ldl, int V, const float* temperature,
+              const int* top_k, const float* top_p,
+              const double* uniform, int* out) {
     __shared__ Best sh_best[THREADS / 32];
     __shared__ int sh_nan[THREADS / 32];
     __shared__ double sh_d[THREADS / 32];
@@ -176,11 +176,11 @@ sample_kernel(const float* __restrict__ logits, int ldl, int V, const float* __r
     if (threadIdx.x == 0) out[r] = sh_found == 0x7fffffff ? best.i : sh_found;
 }
 
-__global__ void adjust_kernel(float* __restrict__ logits, int ldl, int V, const int* __restrict__ item_row,
-                              const int* __restrict__ item_token, const float* __restrict__ item_count,
-                              const float* __restrict__ item_bias, const int* __restrict__ item_seen,
-                              const float* __restrict__ repetition, const float* __restrict__ frequency,
-                              const float* __restrict__ presence, int n_items) {
+__global__ void adjust_kernel(float* logits, int ldl, int V, const int* item_row,
+                              const int* item_token, const float* item_count,
+                              const float* item_bias, const int* item_seen,
+                              const float* repetition, const float* frequency,
+                              const float* presence, int n_items) {
     dd_launch_dependents();
     dd_grid_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

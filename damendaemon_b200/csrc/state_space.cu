@@ -20,9 +20,9 @@ __device__ __forceinline__ float ss_softplus(float x) { return x > 20.f ? x : lo
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-conv_channels_kernel(const T* __restrict__ in, int in_stride, const float* __restrict__ taps_w, const float* __restrict__ bias,
-                     int taps, const float* __restrict__ conv_state, const int* __restrict__ tok_entry,
-                     const int* __restrict__ entry_start, const int* __restrict__ entry_slot, float* __restrict__ out,
+conv_channels_kernel(const T* in, int in_stride, const float* taps_w, const float* bias,
+                     int taps, const float* conv_state, const int* tok_entry,
+                     const int* entry_start, const int* entry_slot, float* out,
                      int out_stride, int C, int act) {
     dd_launch_dependents();
     const int t = blockIdx.y;
@@ -54,10 +54,10 @@ constexpr int SS_TOKENS = 16;         // tokens staged together
 // not lie on the chain from token to token. While a chunk is worked on, the next one is already on its way in registers.
 template <typename T, int LPC>
 __global__ void __launch_bounds__(SS_THREADS)
-state_space_scan_kernel(const float* __restrict__ xbc, int xbc_stride, const T* __restrict__ dt_in, int dt_stride,
-                        const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ skip,
-                        const int* __restrict__ entry_start, const int* __restrict__ entry_slot, float* __restrict__ state,
-                        float* __restrict__ out, int H, int G, int N, int dv) {
+state_space_scan_kernel(const float* xbc, int xbc_stride, const T* dt_in, int dt_stride,
+                        const float* dt_bias, const float* a_log, const float* skip,
+                        const int* entry_start, const int* entry_slot, float* state,
+                        float* out, int H, int G, int N, int dv) {
     constexpr int NP = LPC * 8, COLS = SS_THREADS / LPC;
     constexpr int ROW = 2 * NP + COLS;                                   // staged floats of one token: B, C, x
     constexpr int PER_THREAD = (SS_TOKENS * ROW + SS_THREADS - 1) / SS_THREADS;
@@ -164,10 +164,10 @@ constexpr int GN_KEEP = 8;
 // directly. The arithmetic of a token is that of the staged kernel, instruction for instruction.
 template <typename T, int LPC>
 __global__ void __launch_bounds__(SS_THREADS)
-state_space_single_kernel(const float* __restrict__ xbc, int xbc_stride, const T* __restrict__ dt_in, int dt_stride,
-                          const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ skip,
-                          const int* __restrict__ entry_start, const int* __restrict__ entry_slot, float* __restrict__ state,
-                          float* __restrict__ out, int H, int G, int N, int dv) {
+state_space_single_kernel(const float* xbc, int xbc_stride, const T* dt_in, int dt_stride,
+                          const float* dt_bias, const float* a_log, const float* skip,
+                          const int* entry_start, const int* entry_slot, float* state,
+                          float* out, int H, int G, int N, int dv) {
     constexpr int NP = LPC * 8, COLS = SS_THREADS / LPC;
     dd_launch_dependents();
     const int e = blockIdx.z, h = blockIdx.y, g = h / (H / G);
@@ -205,12 +205,14 @@ state_space_single_kernel(const float* __restrict__ xbc, int xbc_stride, const T
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-gated_group_norm_kernel(const float* __restrict__ y, const T* __restrict__ z, int z_stride, const float* __restrict__ w, float eps,
-                        T* __restrict__ out, int out_stride, int groups, int inner) {
+gated_group_norm_kernel(const float* y, const T* z, int z_stride, const float* w, float eps,
+                        T* out, int out_stride, int groups, int inner) {
     __shared__ float scratch[8];
     dd_launch_dependents();
-    dd_grid_wait();
     const int t = blockIdx.x, g = blockIdx.y, size = inner / groups;
+    // the weights do not depend on the kernel before: their lines are brought into L1 while it is running
+    for (int c = threadIdx.x * 32; c < size; c += blockDim.x * 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(w + g * size + c));
+    dd_grid_wait();
     const float* yr = y + (size_t)t * inner + g * size;
     const T* zr = z + (size_t)t * z_stride + g * size;
     auto gated = [&](int c) {
@@ -233,10 +235,21 @@ gated_group_norm_kernel(const float* __restrict__ y, const T* __restrict__ z, in
     for (int i = 0; i < (int)(blockDim.x >> 5); ++i) total += scratch[i];
     const float r = rsqrtf(total / (float)size + eps);
     T* o = out + (size_t)t * out_stride + g * size;
+    // four weights requested before the first result is written (all eight ahead of the sum cost 8 registers more than the
+    // 32 that let eight blocks share an SM: 2 x 1,024 tokens 15.1 instead of 12.2 us)
 #pragma unroll
-    for (int j = 0; j < GN_KEEP; ++j) {
-        const int c = threadIdx.x + j * blockDim.x;
-        if (c < size) o[c] = dd_from_f32<T>(kept[j] * r * w[g * size + c]);
+    for (int j0 = 0; j0 < GN_KEEP; j0 += 4) {
+        float wj[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int c = threadIdx.x + (j0 + j) * blockDim.x;
+            wj[j] = c < size ? w[g * size + c] : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int c = threadIdx.x + (j0 + j) * blockDim.x;
+            if (c < size) o[c] = dd_from_f32<T>(kept[j0 + j] * r * wj[j]);
+        }
     }
     for (int c = threadIdx.x + GN_KEEP * blockDim.x; c < size; c += blockDim.x) o[c] = dd_from_f32<T>(gated(c) * r * w[g * size + c]);
 }

@@ -23,8 +23,8 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-tanh_norm_kernel(const float* __restrict__ x, const int* __restrict__ row_index, const float* __restrict__ alpha,
-                 const float* __restrict__ w, const float* __restrict__ b, T* __restrict__ out, int width) {
+tanh_norm_kernel(const float* x, const int* row_index, const float* alpha,
+                 const float* w, const float* b, T* out, int width) {
     dd_launch_dependents();
     const float a = alpha[0];
     dd_grid_wait();
@@ -47,7 +47,7 @@ tanh_norm_kernel(const float* __restrict__ x, const int* __restrict__ row_index,
 }
 
 __global__ void __launch_bounds__(256)
-add_rows_kernel(float* __restrict__ x, const float* __restrict__ other, const float* __restrict__ vec, int width) {
+add_rows_kernel(float* x, const float* other, const float* vec, int width) {
     dd_launch_dependents();
     dd_grid_wait();
     const size_t at = (size_t)blockIdx.x * width;
@@ -60,8 +60,8 @@ add_rows_kernel(float* __restrict__ x, const float* __restrict__ other, const fl
 }
 
 __global__ void __launch_bounds__(256)
-norm_pair_add_kernel(float* __restrict__ x, const float* __restrict__ left, const float* __restrict__ right,
-                     const float* __restrict__ wl, const float* __restrict__ wr, float eps, float half, int width) {
+norm_pair_add_kernel(float* x, const float* left, const float* right,
+                     const float* wl, const float* wr, float eps, float half, int width) {
     __shared__ float scratch[8];
     dd_launch_dependents();
     dd_grid_wait();
@@ -83,8 +83,8 @@ norm_pair_add_kernel(float* __restrict__ x, const float* __restrict__ left, cons
 // wait for the kernel before.
 template <typename T, int KEEP>
 __global__ void __launch_bounds__(256)
-wide_norm_pieces_kernel(T* __restrict__ q, T* __restrict__ k, int stride, const int* __restrict__ positions,
-                        const float* __restrict__ freqs, const float* __restrict__ qw, const float* __restrict__ kw, float eps,
+wide_norm_pieces_kernel(T* q, T* k, int stride, const int* positions,
+                        const float* freqs, const float* qw, const float* kw, float eps,
                         int nq, int nk, int d, int n_pairs) {
     constexpr int PIECE = 16 / sizeof(T);
     extern __shared__ float wn_turns[];                  // cosine and sine of every pair
@@ -154,8 +154,8 @@ wide_norm_pieces_kernel(T* __restrict__ q, T* __restrict__ k, int stride, const 
 // that do not fit shared memory, or are not 16-byte aligned, are normed and rotated in place from global memory.
 template <typename T, bool STAGED>
 __global__ void __launch_bounds__(256)
-wide_norm_rotary_kernel(T* __restrict__ q, T* __restrict__ k, int stride, const int* __restrict__ positions,
-                        const float* __restrict__ freqs, const float* __restrict__ qw, const float* __restrict__ kw, float eps,
+wide_norm_rotary_kernel(T* q, T* k, int stride, const int* positions,
+                        const float* freqs, const float* qw, const float* kw, float eps,
                         int q_heads, int k_heads, int d, int n_pairs, int interleaved) {
     extern __shared__ __align__(16) float wn_shared[];
     __shared__ float sums[2][8];
@@ -237,7 +237,7 @@ wide_norm_rotary_kernel(T* __restrict__ q, T* __restrict__ k, int stride, const 
 // An item is a 16-byte piece of a row (WIDE) or one element; the grid covers all items of all rows.
 template <typename T, bool WIDE>
 __global__ void __launch_bounds__(256)
-sigmoid_gate_kernel(T* __restrict__ x, int x_stride, const T* __restrict__ gate, int gate_stride, int rows, int width) {
+sigmoid_gate_kernel(T* x, int x_stride, const T* gate, int gate_stride, int rows, int width) {
     constexpr int PIECE = WIDE ? 16 / sizeof(T) : 1;
     dd_launch_dependents();
     dd_grid_wait();
@@ -259,7 +259,7 @@ sigmoid_gate_kernel(T* __restrict__ x, int x_stride, const T* __restrict__ gate,
     }
 }
 
-__global__ void __launch_bounds__(256) tanh_cap_kernel(float* __restrict__ x, long long n, float cap) {
+__global__ void __launch_bounds__(256) tanh_cap_kernel(float* x, long long n, float cap) {
     dd_launch_dependents();
     dd_grid_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -79,7 +79,7 @@ __device__ __forceinline__ void tm_block_sums(float& a, float& b, float* scratch
 // there already. S: the number of blends, -1: any number (their weights are read when they are used).
 template <typename T, int VPT, int S>
 __global__ void __launch_bounds__(256)
-token_mix_vec_kernel(const MixArgs a, T* __restrict__ out1, T* __restrict__ out2, T* __restrict__ mixes, int per_block) {
+token_mix_vec_kernel(const MixArgs a, T* out1, T* out2, T* mixes, int per_block) {
     __shared__ float scratch[16];
     constexpr int SK = S > 0 ? S : 1;
     dd_launch_dependents();
@@ -165,7 +165,7 @@ token_mix_vec_kernel(const MixArgs a, T* __restrict__ out1, T* __restrict__ out2
 // Any width and alignment: a block a token, rows read twice.
 template <typename T>
 __global__ void __launch_bounds__(256)
-token_mix_kernel(const MixArgs a, T* __restrict__ out1, T* __restrict__ out2, T* __restrict__ mixes) {
+token_mix_kernel(const MixArgs a, T* out1, T* out2, T* mixes) {
     __shared__ float scratch[16];
     dd_launch_dependents();
     dd_grid_wait();
@@ -243,10 +243,10 @@ __device__ __forceinline__ float tm_fade(float x) { return -expm1f(-expf(x)); }
 // A warp a (token, head).
 template <typename T>
 __global__ void __launch_bounds__(256)
-time_prepare_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v, int stride,
-                    const float* __restrict__ decay_in, const float* __restrict__ w0, const float* __restrict__ u,
-                    float* __restrict__ r_out, float* __restrict__ k_out, float* __restrict__ v_out, float* __restrict__ fade_out,
-                    float* __restrict__ bonus_out, int n_tokens, int H, int dk, int dv) {
+time_prepare_kernel(const T* r, const T* k, const T* v, int stride,
+                    const float* decay_in, const float* w0, const float* u,
+                    float* r_out, float* k_out, float* v_out, float* fade_out,
+                    float* bonus_out, int n_tokens, int H, int dk, int dv) {
     dd_launch_dependents();
     dd_grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -254,17 +254,34 @@ time_prepare_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* _
     if (item >= (long long)n_tokens * H) return;
     const int t = (int)(item / H), h = (int)(item % H);
     const size_t in = (size_t)t * stride + (size_t)h * dk, at = (size_t)item * dk;
+    // everything a lane reads of two elements is requested before the first of its results is written
+    constexpr int P = 2;
     float bonus = 0.f;
-    for (int i = lane; i < dk; i += 32) {
-        const float rv = dd_to_f32(r[in + i]), kv = dd_to_f32(k[in + i]);
-        r_out[at + i] = rv;
-        k_out[at + i] = kv;
-        fade_out[at + i] = tm_fade(decay_in[at + i] + w0[h * dk + i]);
-        bonus = __fmaf_rn(__fmul_rn(rv, u[h * dk + i]), kv, bonus);
+    for (int i0 = lane; i0 < max(dk, dv); i0 += 32 * P) {
+        float rv[P], kv[P], x[P], uv[P], vv[P];
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const int i = i0 + 32 * p;
+            rv[p] = i < dk ? dd_to_f32(r[in + i]) : 0.f;
+            kv[p] = i < dk ? dd_to_f32(k[in + i]) : 0.f;
+            x[p] = i < dk ? decay_in[at + i] + w0[h * dk + i] : 0.f;
+            uv[p] = i < dk ? u[h * dk + i] : 0.f;
+            vv[p] = i < dv ? dd_to_f32(v[(size_t)t * stride + (size_t)h * dv + i]) : 0.f;
+        }
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const int i = i0 + 32 * p;
+            if (i < dk) {
+                r_out[at + i] = rv[p];
+                k_out[at + i] = kv[p];
+                fade_out[at + i] = tm_fade(x[p]);
+                bonus = __fmaf_rn(__fmul_rn(rv[p], uv[p]), kv[p], bonus);
+            }
+            if (i < dv) v_out[(size_t)item * dv + i] = vv[p];
+        }
     }
     bonus = dd_warp_sum(bonus);
     if (lane == 0) bonus_out[item] = bonus;
-    for (int i = lane; i < dv; i += 32) v_out[(size_t)item * dv + i] = dd_to_f32(v[(size_t)t * stride + (size_t)h * dv + i]);
 }
 
 // One token for a thread's eight rows of its column: the part of S^T r, then the state.
@@ -314,9 +331,9 @@ constexpr int TS_TOKENS = 16;          // tokens staged together
 // lanes apart, so that neighbouring lanes read neighbouring pieces); THREADS / LPC * C columns a block.
 template <int R, int C, int LPC, int THREADS>
 __global__ void __launch_bounds__(THREADS)
-time_scan_kernel(const float* __restrict__ r, const float* __restrict__ k, const float* __restrict__ v, const float* __restrict__ fade,
-                 const float* __restrict__ bonus, const int* __restrict__ entry_start, const int* __restrict__ entry_slot,
-                 float* __restrict__ state, float* __restrict__ out, int H, int dk, int dv) {
+time_scan_kernel(const float* r, const float* k, const float* v, const float* fade,
+                 const float* bonus, const int* entry_start, const int* entry_slot,
+                 float* state, float* out, int H, int dk, int dv) {
     constexpr int DKP = R * LPC, COLS = THREADS / LPC * C, P = R / 4;
     constexpr int BUF = TS_TOKENS * (3 * DKP + COLS) + TS_TOKENS;       // floats of one buffer: r, k, fade, v, bonus
     extern __shared__ __align__(16) float staged[];
@@ -472,10 +489,10 @@ time_scan_kernel(const float* __restrict__ r, const float* __restrict__ k, const
 constexpr int ST_THREADS = 256, ST_AHEAD = 2;
 template <typename T, int LPC>
 __global__ void __launch_bounds__(ST_THREADS)
-time_step_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ gate, int stride,
-                 const float* __restrict__ decay_in, const float* __restrict__ w0, const float* __restrict__ u,
-                 const float* __restrict__ weight, float eps, const int* __restrict__ entry_slot, float* __restrict__ state,
-                 T* __restrict__ out, int out_stride, int H, int dk, int dv) {
+time_step_kernel(const T* r, const T* k, const T* v, const T* gate, int stride,
+                 const float* decay_in, const float* w0, const float* u,
+                 const float* weight, float eps, const int* entry_slot, float* state,
+                 T* out, int out_stride, int H, int dk, int dv) {
     constexpr int DKP = 8 * LPC, COLS = ST_THREADS / LPC;
     extern __shared__ __align__(16) float sh[];          // r, k, fade [DKP] each, then v and o [dv] each
     __shared__ float scratch[8];
