@@ -18,6 +18,7 @@ import torch
 from .. import kernels
 from ..cache import CacheManager, PageCapacityError
 from ..parts import DecoderModel, Runtime, cache_needs, tensor_decls
+from ..parts.linear import splits_float32
 from ..registry import load_config
 from ..weights.loader import DictSource, check_and_place, load_weights
 from .context import StepContext
@@ -92,6 +93,9 @@ class Engine:
         kv_tokens = (kv_tokens + page_size - 1) // page_size * page_size
         self.kv_tokens = kv_tokens
         self.cache = CacheManager(cache_needs(self.spec), kv_tokens, page_size, max_requests, self.max_context)
+        # float32 products on the tensor cores first write their tokens in parts: the widest of them counts
+        self._plane_width = max((t.shape[1] for t in weights.values() if self.dtype == torch.float32 and gemm != "simt" and t.dim() == 2
+                                 and splits_float32(*t.shape)), default=0)
         self._admit_memory()
         self.cache.allocate(self.device, self.dtype)
         self._caches = [self.cache.layer_view(i) if e.cache_of is None else self.cache.layer_view(e.cache_of, writable=False)
@@ -139,7 +143,9 @@ class Engine:
         cache_bytes = self.cache.bytes_needed(element)
         widest = max((getattr(l.feed_forward, "inner", 0) for l in self.spec.layers), default=0)
         per_token = 4 * self.spec.width * 4 + (3 * self.spec.width + widest) * element
-        workspace = min(self.max_context * self.cache.max_requests, 8192) * per_token + self.cache.max_requests * self.spec.vocab_size * 4
+        tokens = min(self.max_context * self.cache.max_requests, 8192)
+        self.workspace_bytes = workspace = tokens * per_token + self.cache.max_requests * self.spec.vocab_size * 4 + \
+            kernels.gemm_split_plane_bytes(tokens, self._plane_width, 128)
         free, total = torch.cuda.mem_get_info(self.device)
         need = cache_bytes + workspace + self.HEADROOM_BYTES
         if need > free:

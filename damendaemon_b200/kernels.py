@@ -7,6 +7,7 @@ cannot be built or loaded, raises ``KernelError``.
 from __future__ import annotations
 
 import ctypes
+import functools
 import threading
 
 import torch
@@ -1160,7 +1161,16 @@ def gemm_split_fits(a, w):
         not (a.data_ptr() | w.data_ptr()) & 15
 
 
-_split_plans = {}
+def gemm_split_plane_bytes(tokens, reduction, token_tile):
+    """Scratch for the tokens' three bfloat16 planes: 192 bytes for every token, rounded up to whole tiles, and k block of 32."""
+    return -(-tokens // token_tile) * token_tile * -(-reduction // 32) * 192
+
+
+@functools.lru_cache(maxsize=4096)
+def _split_plan(M, N, K, sms):
+    """(blocks that share a tile's K, token tile) as the kernel's own plan has them."""
+    tile = ctypes.c_int(0)
+    return library("core").dd_gemm_split_plan(M, N, K, sms, ctypes.byref(tile)), tile.value
 
 
 def gemm_split(a, w, bias=None, residual=None, activation=None, out=None, token_tile=None, splits=None):
@@ -1179,14 +1189,9 @@ def gemm_split(a, w, bias=None, residual=None, activation=None, out=None, token_
     if residual is not None:
         _rows(residual, "residual")
     lib, sms = library("core"), sm_count(a.device)
-    plan = _split_plans.get((M, N, K))
-    if plan is None:
-        tile = ctypes.c_int(0)
-        planned = lib.dd_gemm_split_plan(M, N, K, sms, ctypes.byref(tile))
-        plan = _split_plans[(M, N, K)] = (planned, tile.value)
+    plan = _split_plan(M, N, K, sms)
     token_tile = plan[1] if token_tile is None else token_tile
-    planes = None if token_tile < 64 else \
-        torch.empty((-(-M // token_tile) * token_tile * -(-K // 32) * 192,), dtype=torch.uint8, device=a.device)
+    planes = None if token_tile < 64 else torch.empty((gemm_split_plane_bytes(M, K, token_tile),), dtype=torch.uint8, device=a.device)
     _call(lib, "dd_gemm_split", _ptr(a, "a"), a.stride(0), _ptr(w, "w"), w.stride(0), _ptr(bias, "bias", torch.float32),
           _ptr(residual, "residual", torch.float32), 0 if residual is None else residual.stride(0),
           _ptr(out, "out", torch.float32), out.stride(0), M, N, K, ACTIVATIONS[activation],

@@ -369,3 +369,36 @@ def test_a_score_that_is_not_a_number_shows_in_a_single_token(K, heads, kv_heads
             last = torch.arange(70, device=DEV) % keys == keys - 1
             assert bool(torch.isnan(got[last]).all()) and torch.equal(got[~last], clean[~last])
     assert K.read_error_flag(DEV) == 0
+
+
+def test_admission_counts_the_planes_of_the_split_products(K):
+    """What an engine promises to fit before it allocates its cache covers the largest step: 8,192 tokens of prompts through a
+    layer whose inner products are split take no more than the estimate; and only products that are split count."""
+    from damendaemon_b200.engine import Engine, StepEntry
+    from damendaemon_b200.registry import architecture_of
+    config = {"architectures": ["GPT2LMHeadModel"], "model_type": "gpt2", "n_layer": 1, "n_embd": 512, "n_head": 8, "n_inner": 2048,
+              "vocab_size": 300, "n_positions": 1024}
+    arch = architecture_of(config)
+    tensors = arch.random_tensors(arch.parse_config(config), 1, torch.float32)
+    made = {}
+    for dtype, gemm in (("float32", "auto"), ("float32", "simt"), ("bfloat16", "auto")):
+        made[dtype, gemm] = Engine(config=config, tensors=tensors, dtype=dtype, gemm=gemm, kv_tokens=8192, max_requests=8)
+    engine = made["float32", "auto"]
+    planes = K.gemm_split_plane_bytes(8192, 2048, 128)
+    assert planes == 8192 * 2048 * 6
+    assert engine.workspace_bytes - made["float32", "simt"].workspace_bytes == planes
+    assert made["bfloat16", "auto"].workspace_bytes < made["float32", "simt"].workspace_bytes
+    entries = [StepEntry(r, [(7 * i + r) % 300 for i in range(1024)], [1023]) for r in range(8)]
+    engine.step(entries, end=range(8))                  # (the step's metadata and the error word are allocated)
+    torch.cuda.synchronize()
+    held = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    engine.step(entries, end=range(8))
+    assert planes < torch.cuda.max_memory_allocated() - held <= engine.workspace_bytes
+
+
+def test_plans_that_are_kept_are_bounded(K):
+    assert K._split_plan.cache_info().maxsize <= 4096
+    for M in (1, 16, 17, 33, 65, 128, 129, 300, 5000):
+        splits, tile = K._split_plan(M, 1600, 1600, 148)
+        assert tile == (16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128) and 1 <= splits <= 8
