@@ -535,6 +535,9 @@ DD_API int dd_gemm_split(const float* X, int ldx, const float* W, int ldw, const
                          float* out, int ldo, int M, int N, int K, int act, int token_tile, int splits, int sm_count,
                          void* planes, int* error_flag, void* stream) {
     if (M <= 0 || N <= 0) return 0;
+    if (M == 1) ldx = K;                                         // (the stride of a single row may be anything)
+    if (N == 1) ldw = K;
+    if (ldx < K || ldw < K) return dd_fail("dd_gemm_split: rows of %d elements lie over one another (strides %d, %d)", K, ldx, ldw);
     if (K <= 0 || K % 4 || ldx % 4 || ldw % 4 || (((uintptr_t)X | (uintptr_t)W) & 15))
         return dd_fail("dd_gemm_split: K=%d and the row strides (%d, %d) must be multiples of 4 and the operands 16-byte aligned", K, ldx, ldw);
     const int kblocks = dd_ceil_div(K, BK);

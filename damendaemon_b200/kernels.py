@@ -1156,9 +1156,11 @@ def gemm_simt(a, w, bias=None, residual=None, activation=None, out_dtype=None, o
 
 def gemm_split_fits(a, w):
     """Whether gemm_split takes these operands: float32, 16-byte aligned rows, a reduction width that is a multiple of 4 (and
-    within the 65,535 k blocks of the kernel that writes the tokens' planes)."""
-    return a.dtype == torch.float32 and w.dtype == torch.float32 and a.shape[1] <= 65535 * 32 and not (a.shape[1] % 4 or a.stride(0) % 4 or w.stride(0) % 4) and \
-        not (a.data_ptr() | w.data_ptr()) & 15
+    within the 65,535 k blocks of the kernel that writes the tokens' planes), rows that do not lie over one another (an
+    expanded row's stride of 0 is none that TMA describes)."""
+    K = a.shape[1]
+    return a.dtype == torch.float32 and w.dtype == torch.float32 and K <= 65535 * 32 and not (K % 4 or a.stride(0) % 4 or w.stride(0) % 4) and \
+        (a.stride(0) >= K or a.shape[0] == 1) and (w.stride(0) >= K or w.shape[0] == 1) and not (a.data_ptr() | w.data_ptr()) & 15
 
 
 def gemm_split_plane_bytes(tokens, reduction, token_tile):

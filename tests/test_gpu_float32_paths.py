@@ -90,6 +90,13 @@ def test_which_float32_products_are_split(K):
     # rows that start off a 16-byte boundary stay on the CUDA cores
     shifted = torch.randn(8, 1601, device=DEV)[:, 1:]
     assert torch.equal(linear(auto, shifted, w), K.gemm_simt(shifted, w))
+    # ... and so do rows that lie over one another, which no tensor map describes
+    for rows in (a[:1].expand(8, 1600), torch.randn(8 * 1600, device=DEV).as_strided((8, 1600), (16, 1))):
+        assert not K.gemm_split_fits(rows, w) and torch.equal(linear(auto, rows, w), K.gemm_simt(rows.contiguous(), w))
+    with pytest.raises(K.KernelError, match="over one another"):
+        K.gemm_split(a[:1].expand(8, 1600), w)
+    one = a.as_strided((1, 1600), (0, 1))
+    assert torch.equal(linear(auto, one, w), K.gemm_split(a[:1], w))
 
 
 def run_of_entries(dtype, entries, keys, heads, kv_heads, d, page=16, seed=11):
