@@ -253,3 +253,42 @@ def test_experts_chosen_by_a_table(experts, top, shared, tokens, dtype):
                       runtime=runtime)
     got = part.forward(y.to(dtype).to(DEV), stream.clone().to(DEV), ctx).cpu().double()
     assert (got - want).abs().max() < (2e-5 if dtype == torch.float32 else 0.05)
+
+
+@pytest.mark.parametrize("given", [True, False])
+@pytest.mark.parametrize("tokens,top", [(1, 1), (2048, 2), (4097, 1), (4096, 2), (3000, 3), (2731, 3)])
+def test_routing_of_more_pairs_than_the_block_holds_at_once(tokens, top, given):
+    """Up to 4,096 (token, choice) pairs go through the block's 1,024 threads in one round, more in several (ordinary prompts
+    have 4,098 and more): every pair has one row among its expert's, the unused rows and tiles are marked, with token ids and
+    without; identity experts have no rows; an id outside the vocabulary in an early round is reported."""
+    from damendaemon_b200 import kernels
+    experts, identity, tile, vocab = 7, 2, 16, 500
+    g = torch.Generator().manual_seed(tokens + top)
+    rows = vocab if given else tokens
+    table = torch.rand(rows, experts + identity, generator=g).argsort(1)[:, :top].to(torch.int32).contiguous()
+    ids = torch.randint(0, vocab, (tokens,), generator=g, dtype=torch.int32) if given else None
+    weight = torch.rand(tokens * top, generator=g) + 0.1
+    chosen = (table[ids.long()] if given else table).reshape(-1).long()
+
+    def route(ids):
+        return [x.cpu().long() if x.dtype == torch.int32 else x.cpu() for x in
+                kernels.route_by_table(None if ids is None else ids.to(DEV), table.to(DEV), experts, tile, n_identity=identity, pair_weight=weight.to(DEV))]
+
+    pair_row, row_token, tile_group, row_weight = route(ids)
+    assert kernels.read_error_flag(DEV) == 0
+    own = chosen >= experts
+    assert bool((pair_row[own] == -2).all()) and bool((pair_row[~own] >= 0).all())
+    used = pair_row[~own]
+    assert used.unique().numel() == used.numel()
+    assert torch.equal(row_token[used], torch.arange(tokens).repeat_interleave(top)[~own]) and torch.equal(row_weight[used], weight[~own])
+    assert torch.equal(tile_group[used // tile], chosen[~own])
+    empty = torch.ones(row_token.numel(), dtype=torch.bool)
+    empty[used] = False
+    assert bool((row_token[empty] == -1).all()) and bool((row_weight[empty] == 0).all())
+    tiles = sum(-(-int((chosen == e).sum()) // tile) for e in range(experts))
+    assert bool((tile_group[tiles:] == -1).all()) and bool((tile_group[:tiles] >= 0).all())
+    if given:
+        wrong = ids.clone()
+        wrong[0] = vocab
+        pair_row = route(wrong)[0]
+        assert kernels.read_error_flag(DEV) == 1 and bool((pair_row[:top] == -1).all())
