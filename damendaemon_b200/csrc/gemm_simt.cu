@@ -1,9 +1,10 @@
 // C[M,N] = act(A[M,K] . W[N,K]^T + bias) (+ residual): plain CUDA-core GEMM with
-// float32 multiply-add and no tensor-core or reduced-precision mode. It is the
-// matrix product of the true 32-bit path, and (with bfloat16 operands) the slow
-// stand-in that the tensor-core kernels are checked against. Every output element
-// is summed over k in ascending order by one thread, so a row's result does not
-// depend on how many other rows are in the batch.
+// float32 multiply-add and no tensor-core or reduced-precision mode. It is the float32
+// engine's product for small matrices (larger ones: gemm_split_tcgen05.cu) and where
+// 'simt' is asked for, and (with bfloat16 operands) the slow stand-in that the
+// tensor-core kernels are checked against. Every output element is summed over k in
+// ascending order by one thread, so a row's result does not depend on how many other
+// rows are in the batch.
 #include "common.cuh"
 
 namespace {

@@ -12,7 +12,9 @@ def splits_float32(out, reduction):
     K = 4 to 6,400). Smaller matrices stream through the CUDA-core kernel in fewer steps than the split one needs to
     start (split / CUDA cores, us): 1024 x 256 at 8 rows 7.2 / 3.4, 512 x 512 at 8 and 64 rows 7.3 / 4.8 and 12.4 / 11.9;
     1024 x 1024 7.5 / 8.1 and 11.3 / 21.8, 6400 -> 1600 15 / 41 and 21.5 / 125. The line goes by the matrix alone, so that
-    a row of a small model has the same bits whatever else is in the batch."""
+    a row of a small model has the same bits whatever else is in the batch. The split product cuts its sums by the number of
+    tiles: a row of a larger model has other bits beside more than 128 tokens than alone, within the same error (gemm='simt'
+    keeps them)."""
     return out * reduction >= 1 << 20
 
 
