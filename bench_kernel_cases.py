@@ -7,9 +7,12 @@ the same command with a small N.
 """
 from __future__ import annotations
 
+from types import SimpleNamespace
+
 import torch
 
 from damendaemon_b200 import kernels as K
+from damendaemon_b200.parts.paged_attention import token_splits
 
 H, D, PAGE = 25, 64, 16
 SHAPES = {"qkv": (4800, 1600, "bias"), "proj": (1600, 1600, "residual"), "fc": (6400, 1600, "gelu"),
@@ -39,8 +42,9 @@ def _gemm_case(name, tokens, dev):
     return run, work
 
 
-def _gemm32_case(name, tokens, dev):
-    """The same products in true 32-bit on the CUDA cores (float32 weights, activations and stream)."""
+def _gemm32_case(name, tokens, dev, product=None):
+    """The same products in float32 (weights, activations and stream), on the CUDA cores or by another kernel."""
+    product = product or K.gemm_simt
     features, reduction, epilogue = SHAPES[name]
     copies = max(2, min(12, (300 << 20) // (features * reduction * 4)))
     weights = [torch.randn(features, reduction, device=dev).mul_(0.02) for _ in range(copies)]
@@ -52,9 +56,9 @@ def _gemm32_case(name, tokens, dev):
     def run(i):
         w = weights[i % copies]
         if epilogue == "residual":
-            K.gemm_simt(x, w, bias, residual=stream, out=stream)
+            product(x, w, bias, residual=stream, out=stream)
         else:
-            K.gemm_simt(x, w, bias if epilogue != "none" else None, activation="gelu_new" if epilogue == "gelu" else None, out=out)
+            product(x, w, bias if epilogue != "none" else None, activation="gelu_new" if epilogue == "gelu" else None, out=out)
     return run, {"bytes": features * reduction * 4, "flops": 2 * tokens * features * reduction}
 
 
@@ -701,9 +705,9 @@ def _grouped_case(which, tokens, dev):
     return run, {"bytes": used * INNER * width * 2, "flops": 2 * tokens * TOP * INNER * width}
 
 
-def _cache_case(batch, context, dev, copies):
+def _cache_case(batch, context, dev, copies, dtype=torch.bfloat16):
     n_pages = batch * ((context + PAGE - 1) // PAGE)
-    caches = [torch.randn(n_pages, 2, H, PAGE, D, device=dev).to(torch.bfloat16) for _ in range(copies)]
+    caches = [torch.randn(n_pages, 2, H, PAGE, D, device=dev).to(dtype) for _ in range(copies)]
     table = torch.arange(n_pages, dtype=torch.int32, device=dev).view(batch, -1)
     return caches, table
 
@@ -737,8 +741,27 @@ def _prefill_case(prompts, length, dev, kernel="tcgen05", store=False, masked=Fa
     return run, {"bytes": prompts * length * H * D * 6, "flops": prompts * 4 * (length * (length + 1) // 2) * H * D}
 
 
+def _float32_attention_case(batch, length, dev, decode):
+    """The float32 engine's attention: single tokens at the end of contexts of this length, which bring their own keys and
+    values, or whole prompts whose keys and values are in the cache (one block a tile of queries)."""
+    copies = max(2, min(8, (300 << 20) // (batch * length * H * D * 8)))
+    caches, table = _cache_case(batch, length, dev, copies, torch.float32)
+    if decode:
+        pos = torch.full((batch,), length - 1, dtype=torch.int32, device=dev)
+        q, k, v = torch.randn(batch, 3 * H * D, device=dev).split(H * D, dim=1)
+        splits = token_splits(SimpleNamespace(sm_count=K.sm_count(dev), split_context=length), batch, H)
+        run = lambda i: K.attention_tokens(q, caches[i % copies], pos, table, H, D ** -0.5, n_splits=splits, k_new=k, v_new=v)
+        return run, {"bytes": batch * length * H * D * 8, "flops": 4 * batch * length * H * D, "fp32": True}
+    start = torch.arange(batch + 1, dtype=torch.int32, device=dev) * length
+    pos0 = torch.zeros(batch, dtype=torch.int32, device=dev)
+    q = torch.randn(batch * length, H * D, device=dev)
+    run = lambda i: K.attention_f32_prompt(q, caches[i % copies], start, pos0, table, H, D ** -0.5)
+    return run, {"bytes": batch * length * H * D * 16, "flops": batch * 4 * (length * (length + 1) // 2) * H * D, "fp32": True}
+
+
 def build(name, device="cuda:0"):
-    """name: gemm_<qkv|proj|fc|fc2|head>_m<tokens> | gemm32_<...>_m<tokens> (float32, CUDA cores) | attn_decode_b<batch>[_c<context>] (page streaming) | attn_decode_rows_b<batch>[_c<context>] | attn_prefill_p<prompts>_t<tokens> | attn_prefill | attn_prefill_store (the kernel writes the cache too) | attn_prefill_mma |
+    """name: gemm_<qkv|proj|fc|fc2|head>_m<tokens> | gemm32_<...>_m<tokens> (float32, CUDA cores) | gemmsplit_<...>_m<tokens> (float32 in three bfloat16 parts) |
+    attn32_decode_b<batch>_c<context> | attn32_prefill_p<prompts>_t<tokens> (the float32 kernels) | attn_decode_b<batch>[_c<context>] (page streaming) | attn_decode_rows_b<batch>[_c<context>] | attn_prefill_p<prompts>_t<tokens> | attn_prefill | attn_prefill_store (the kernel writes the cache too) | attn_prefill_mma |
     attn_prefill_long (one prompt of 4,096 tokens) | layernorm_m<rows> | rmsnorm_m<rows> | rotary_m<rows> |
     grouped_<up|upsilu|down|route|score>_m<tokens> (sixteen experts, two per token; upsilu: the silu form of the unit;
     score: routing by a router's scores) | headnorm_m<rows> | gatedact_m<rows> | retention_p<requests>_t<tokens> |
@@ -842,6 +865,14 @@ def build(name, device="cuda:0"):
         return _gemm_case(parts[1], int(parts[2][1:]), device)
     if parts[0] == "gemm32" and len(parts) == 3 and parts[1] in SHAPES and parts[2][0] == "m":
         return _gemm32_case(parts[1], int(parts[2][1:]), device)
+    if parts[0] == "gemmsplit" and len(parts) == 3 and parts[1] in SHAPES and parts[2][0] == "m":
+        return _gemm32_case(parts[1], int(parts[2][1:]), device, K.gemm_split)
+    if name.startswith("attn32_decode_b"):
+        batch, context = name[len("attn32_decode_b"):].split("_c")
+        return _float32_attention_case(int(batch), int(context), device, decode=True)
+    if name.startswith("attn32_prefill_p"):
+        prompts, tokens = name[len("attn32_prefill_p"):].split("_t")
+        return _float32_attention_case(int(prompts), int(tokens), device, decode=False)
     if name.startswith("layernorm_m"):
         return _layernorm_case(int(name[len("layernorm_m"):]), device)
     if name.startswith("attn_decode_rows_b") or name.startswith("attn_decode_b"):
