@@ -3,13 +3,14 @@
 //
 // In the cache a page holds the keys of all heads side by side and then the values ([page][K|V][head][slot][64]):
 // the keys of G neighbouring heads are one run of G x page_size rows of 128 bytes. A block owns (token, group of
-// G <= 8 heads, split of the token's pages); thread 0 asks TMA for one box of G x page_size rows of keys and one
+// G <= 7 heads, split of the token's pages); one warp asks TMA for one box of G x page_size rows of keys and one
 // of values per page, as many pages ahead as the ring holds, so a block moves its bytes in pieces of tens of KB with two instructions
 // each (copying the same bytes 16 at a time, one key row per 8 lanes, the memory system delivered 4.5 TB/s;
 // in boxes of this size it delivers 5.4). The 128-byte swizzle of the tensor map is the layout ldmatrix wants.
-// Each of the 8 warps owns one head of the group for all pages, so nothing is merged inside the block:
-// scores and P.V on mma.sync m16n8k16 with the single query in row 0 (see attention_decode.cu), running maximum
-// and sum in float32, base 2 (damendaemon/kernels.py:147-178; split merge by log-sum-exp kernels.py:190-210).
+// Each of the other warps owns one head of the group for all pages, so nothing is merged inside the block:
+// scores and P.V on mma.sync m16n8k16 with the keys (and then the dimensions of the values) as its 16 rows and the single
+// query (the weights) in every column, running maximum and sum in float32, base 2 (damendaemon/kernels.py:147-178; split
+// merge by log-sum-exp kernels.py:190-210).
 //
 // With k_new/v_new the step's own key and value replace the cache row of the token's position in shared memory
 // and are written to the cache by the warp that owns the head. Rows of the last page beyond the position are
@@ -23,9 +24,9 @@
 #include <math_constants.h>
 
 namespace {
-constexpr int D = 64, TILE = 16, WARPS = 8, THREADS = WARPS * 32, HEADS_PER_WARP = 1, MAX_GROUP = WARPS * HEADS_PER_WARP;
-constexpr int MAX_BLOCK_PAGES = 128;          // pages a block may own (their ids live in shared memory); 1 << 7 below
-constexpr int MAX_STAGES = 6;
+constexpr int D = 64, TILE = 16, MAX_GROUP = 7, MAX_THREADS = (MAX_GROUP + 1) * 32;      // a warp a head, and one that requests pages
+constexpr int MAX_BLOCK_PAGES = 128;          // pages a block may own; 1 << 7 below
+constexpr int MAX_STAGES = 3;                 // deeper rings are no faster and leave fewer blocks an SM (see the kernel)
 
 struct Params {
     const __nv_bfloat16* q;
@@ -59,14 +60,15 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t* r) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
-// The same product when only row 0 of A is not zero: rows 8..15 of the result are zero whatever B holds, so their two
-// accumulators are fed with zeros and dropped instead of being kept in registers from tile to tile.
-__device__ __forceinline__ void mma_bf16_row0(float& c0, float& c1, uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
-    float d2, d3;
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%10,%10};"
-                 : "+f"(c0), "+f"(c1), "=f"(d2), "=f"(d3)
-                 : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1), "f"(0.f));
-    asm volatile("" ::"f"(d2), "f"(d3));      // the two dead accumulators count as used
+// 16 rows of A times one column of B, which every column of B repeats (a lane's fragment does not depend on its column):
+// every column of the result is the same, so one of a row's two accumulators in a lane is kept (row quad in c0, row
+// quad + 8 in c1) and the other is fed with zeros and dropped.
+__device__ __forceinline__ void mma_bf16_column(float& c0, float& c1, const uint32_t* a, uint32_t b0, uint32_t b1) {
+    float d1, d3;
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%2,%1,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%10,%1,%10};"
+                 : "+f"(c0), "+f"(c1), "=f"(d1), "=f"(d3)
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+    asm volatile("" ::"f"(d1), "f"(d3));      // the two dead accumulators count as used
 }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -75,14 +77,25 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 // byte offset of 16-byte chunk c of key row r in a tile of 128-byte rows under the 128-byte swizzle
 __device__ __forceinline__ uint32_t tile_off(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
 
-__global__ void __launch_bounds__(THREADS, 2)
-attention_decode_pages_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p) {
+// What bounds it: a step of a few tokens is a chain of latencies, not a stream (8 tokens x 25 heads x 540 keys are 28 MB, 4.4 us of
+// the memory's rate, and the kernel took 11.6 us of a layer). So nothing but data makes anybody wait: a warp of its own
+// looks the pages up (the first 64 entries of the table are read beside the position, not after it) and requests them,
+// the head warps follow it through full and empty barriers of the ring without a barrier of the block, keys and value
+// dimensions are the 16 rows of mma.sync (8 of them a tile of 16 keys, not 16), and a head's splits are merged by
+// the warp that finishes last, through a counter per head: before, the blocks' barriers, fences and the last block's
+// walk over all its heads were 4.4 us behind the last key. Whole passes, before and now: 8 requests from 512 keys on
+// (xl, 64 steps) 129.7 / 117.8 ms, 64 from 256 keys on 204.1 / 195.8, 32 of 16 to 800 keys (medium) 48.9 / 44.4.
+// 80 registers and three stages leave three blocks an SM: with 104 registers and two blocks the last of these takes 45.9
+// (and the first 118.0), with two stages 44.5 (122.3), with four 46.2; a spilled register costs more than any of them.
+__global__ void __launch_bounds__(MAX_THREADS, 3)
+attention_decode_pages_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_last, const Params p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int box_bytes = p.G * p.P * 128;                 // keys (or values) of the group's heads in one page
     uint64_t* full = reinterpret_cast<uint64_t*>(tiles + (size_t)p.stages * 2 * box_bytes);
-    int* page_ids = reinterpret_cast<int*>(full + MAX_STAGES);
-    __shared__ int abort_flag, sh_last;
+    uint64_t* empty = full + MAX_STAGES;
+    volatile int* stage_page = reinterpret_cast<volatile int*>(empty + MAX_STAGES);     // the page a stage holds, -1: none
+    __shared__ int abort_flag;
     dd_launch_dependents();
 
     // Positions, entries and the block table are this step's inputs, not an earlier kernel's results: they are read
@@ -96,6 +109,33 @@ attention_decode_pages_kernel(const __grid_constant__ CUtensorMap map_kv, const 
     const int split = blockIdx.z, g = blockIdx.y, t = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int quad = lane >> 2, t4 = lane & 3;
+    const int head0 = g * p.G;                              // first head of the group
+    const int group_heads = min(p.G, p.H - head0);
+    const CUtensorMap* map = group_heads == p.G ? &map_kv : &map_last;      // boxes of the last group's few heads
+    const int pos = p.tok_pos[t];
+    // without tok_entry token t is entry t (a step of single tokens in entry order): one trip to L2 less before the pages
+    const int* bt = p.block_table + (size_t)(p.tok_entry ? p.tok_entry[t] : t) * p.max_blocks;
+    int held[2] = {-1, -1};                                 // the page warp: entries lane and 32 + lane of a short table
+    const bool short_table = p.max_blocks <= 64;
+    if (warp == p.G) {
+        if (short_table) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                if (i * 32 + lane < p.max_blocks) held[i] = bt[i * 32 + lane];
+        }
+        if (lane == 0) {
+            for (int s = 0; s < p.stages; ++s) {
+                tc::mbar_init(&full[s], 1);
+                tc::mbar_init(&empty[s], group_heads);
+            }
+            abort_flag = 0;
+            tc::fence_barrier_init();
+            tc::fence_proxy_async();
+            tc::prefetch_tensormap(map);
+        }
+    }
+    __syncthreads();                                        // the only one: from here every warp goes at its own pace
+
     // (page sizes are powers of two, and the block budget's reciprocal comes from the host: a chain of integer
     // divisions here, a hundred cycles each, stood between the positions and the first page request)
     const int span = p.max_blocks << p.log2_P;              // positions the block table can describe
@@ -108,7 +148,6 @@ attention_decode_pages_kernel(const __grid_constant__ CUtensorMap map_kv, const 
     };
     // every warp adds up the pages of all tokens for itself (a load per lane and five shuffles for up to 32 tokens):
     // no barrier and no shared memory stand between the positions and the first page request
-    const int pos = p.tok_pos[t];
     int total_pages = 0;
     if (p.deal) {
         for (int i = lane; i < p.n_tokens; i += 32) total_pages += pages_of(p.tok_pos[i], nullptr);
@@ -133,225 +172,208 @@ attention_decode_pages_kernel(const __grid_constant__ CUtensorMap map_kv, const 
     const int per = (my_pages + n_splits - 1) / n_splits;                // pages per split, rounded up
     const int page0 = first_page + split * per;
     const int n_mine = max(0, min(last_page + 1, page0 + per) - page0);
-    // without tok_entry token t is entry t (a step of single tokens in entry order): one trip to L2 less before the pages
-    const int* bt = p.block_table + (size_t)(p.tok_entry ? p.tok_entry[t] : t) * p.max_blocks;
-    for (int i = threadIdx.x; i < n_mine; i += THREADS) {
-        const int blk = page0 + i;
-        int page = blk < p.max_blocks ? bt[blk] : -1;
-        if (page < 0 || page >= p.n_pages) {
-            atomicOr(p.error_flag, 4);
-            page = -1;
-        }
-        page_ids[i] = page;
-    }
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < p.stages; ++s) tc::mbar_init(&full[s], 1);
-        abort_flag = 0;
-        tc::fence_barrier_init();
-        tc::fence_proxy_async();
-        tc::prefetch_tensormap(&map_kv);
-    }
-    __syncthreads();
 
-    const int head0 = g * p.G;                              // first head of the group
-    const int group_heads = min(p.G, p.H - head0);
-    auto load_page = [&](int i) {                           // thread 0: page i of this block into stage i % stages
-        const int s = i % p.stages, page = page_ids[i];
-        uint8_t* dst = tiles + (size_t)s * 2 * box_bytes;
-        if (page < 0) {                                     // a missing page (error bit set): nothing to wait for
-            tc::mbar_arrive(&full[s]);
-            return;
+    if (warp == p.G) {
+        // ---- the page warp: looks up and requests ----
+        // With k_new/v_new given the pages hold earlier steps' keys and values only (this step's own row is patched in
+        // below), so they are requested while the projection that produces the queries is still running.
+        // Without them the step's row is in the cache already, written by some kernel of this step: then the wait comes first.
+        if (p.k_new == nullptr) dd_grid_wait();
+        bool ok = true;
+        int s = 0, phase = 1;                               // the first round of the ring finds its stages free
+#pragma unroll 1
+        for (int i0 = 0; i0 < n_mine && ok; i0 += 32) {
+            const int blk = page0 + i0 + lane;
+            int page = -1;
+            if (short_table) {
+                const int low = __shfl_sync(0xffffffffu, held[0], blk & 31), high = __shfl_sync(0xffffffffu, held[1], blk & 31);
+                page = blk < 32 ? low : (blk < p.max_blocks ? high : -1);
+            } else if (i0 + lane < n_mine && blk < p.max_blocks) page = bt[blk];
+            if (i0 + lane < n_mine && (page < 0 || page >= p.n_pages)) {
+                atomicOr(p.error_flag, p.k_new != nullptr && blk == last_page ? 6 : 4);     // the token's own row finds no place either
+                page = -1;
+            }
+#pragma unroll 1
+            for (int i = i0; i < min(n_mine, i0 + 32) && ok; ++i) {
+                const int id = __shfl_sync(0xffffffffu, page, i - i0);
+                if (lane == 0) {
+                    ok = tc::mbar_wait(&empty[s], phase, &abort_flag);
+                    if (ok) {
+                        stage_page[s] = id;
+                        if (id < 0) tc::mbar_arrive(&full[s]);                  // a missing page (error bit set): nothing to wait for
+                        else {
+                            uint8_t* dst = tiles + (size_t)s * 2 * box_bytes;
+                            tc::mbar_expect_tx(&full[s], 2 * group_heads * p.P * 128);
+                            tc::tma_load_2d(dst, map, 0, ((id * 2 + 0) * p.H + head0) * p.P, &full[s]);
+                            tc::tma_load_2d(dst + box_bytes, map, 0, ((id * 2 + 1) * p.H + head0) * p.P, &full[s]);
+                        }
+                    }
+                }
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                if (++s == p.stages) { s = 0; phase ^= 1; }
+            }
         }
-        tc::mbar_expect_tx(&full[s], 2 * box_bytes);
-        tc::tma_load_2d(dst, &map_kv, 0, ((page * 2 + 0) * p.H + head0) * p.P, &full[s]);
-        tc::tma_load_2d(dst + box_bytes, &map_kv, 0, ((page * 2 + 1) * p.H + head0) * p.P, &full[s]);
-    };
-    // With k_new/v_new given the pages hold earlier steps' keys and values only (this step's own row is patched in
-    // below), so the first stages are requested while the projection that produces the queries is still running.
-    // Without them the step's row is in the cache already, written by some kernel of this step: then the wait comes first.
-    if (threadIdx.x == 0 && p.k_new != nullptr)
-        for (int i = 0; i < min(n_mine, p.stages); ++i) load_page(i);
+        if (!ok && lane == 0) atomicOr(p.error_flag, 8);
+        return;
+    }
+    if (warp >= group_heads) return;
+
+    // ---- a warp owns a head of the group ----
     dd_grid_wait();              // the queries and this step's keys and values are the kernel before this one's work
-    if (threadIdx.x == 0 && p.k_new == nullptr)
-        for (int i = 0; i < min(n_mine, p.stages); ++i) load_page(i);
-
-    // the queries of this warp's heads as A operands: row 0 of a 16-row tile, every other row zero
-    uint32_t qf[HEADS_PER_WARP][D / 16][2];
-    float m[HEADS_PER_WARP], l[HEADS_PER_WARP], o[HEADS_PER_WARP][D / 8][2];
-#pragma unroll
-    for (int u = 0; u < HEADS_PER_WARP; ++u) {
-        const int hl = warp + u * WARPS;
-        const __nv_bfloat16* qp = p.q + (size_t)t * p.q_stride + (size_t)(head0 + min(hl, group_heads - 1)) * D;
+    const int h = head0 + warp;
+    // the query as the B operand, the same in every column
+    uint32_t qf[D / 16][2];
+    float m = -CUDART_INF_F, l = 0.f, o[D / 16][2];         // o: dimensions 16 j + quad and 16 j + 8 + quad, in every lane of the quad
+    {
+        const __nv_bfloat16* qp = p.q + (size_t)t * p.q_stride + (size_t)h * D;
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
-            qf[u][ks][0] = quad == 0 ? *reinterpret_cast<const uint32_t*>(qp + ks * 16 + 2 * t4) : 0u;
-            qf[u][ks][1] = quad == 0 ? *reinterpret_cast<const uint32_t*>(qp + ks * 16 + 8 + 2 * t4) : 0u;
+            qf[ks][0] = *reinterpret_cast<const uint32_t*>(qp + ks * 16 + 2 * t4);
+            qf[ks][1] = *reinterpret_cast<const uint32_t*>(qp + ks * 16 + 8 + 2 * t4);
+            o[ks][0] = o[ks][1] = 0.f;
         }
-        m[u] = -CUDART_INF_F;
-        l[u] = 0.f;
-#pragma unroll
-        for (int j = 0; j < D / 8; ++j) o[u][j][0] = o[u][j][1] = 0.f;
     }
 
     const size_t head_plane = (size_t)p.P * D, page_stride = 2 * (size_t)p.H * head_plane;
+    bool ok = true;
+    int s = 0, phase = 0;
+#pragma unroll 1
     for (int i = 0; i < n_mine; ++i) {
-        const int s = i % p.stages;
-        // all threads leave together if the wait ran out for any of them
-        if (!__syncthreads_and(tc::mbar_wait(&full[s], (i / p.stages) & 1, &abort_flag) ? 1 : 0)) break;
-        const int page = page_ids[i];
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(&full[s], phase, &abort_flag));
+        if (!ok) break;
+        const int page = stage_page[s];
         const int key0 = (page0 + i) * p.P;                 // first key of the page
-        uint8_t* k_box = tiles + (size_t)s * 2 * box_bytes;
-        uint8_t* v_box = k_box + box_bytes;
+        uint8_t* kh = tiles + (size_t)s * 2 * box_bytes + (size_t)warp * p.P * 128;
+        uint8_t* vh = kh + box_bytes;
         if (page >= 0) {
-#pragma unroll
-            for (int u = 0; u < HEADS_PER_WARP; ++u) {
-                const int hl = warp + u * WARPS;
-                if (hl >= group_heads) continue;
-                uint8_t* kh = k_box + (size_t)hl * p.P * 128;
-                uint8_t* vh = v_box + (size_t)hl * p.P * 128;
-                if (key0 + p.P > pos) {
-                    // the page of the token's own position: its new key and value, and zeros for the unwritten slots
-                    const int slot = pos - key0;
-                    if (p.k_new != nullptr && lane < 16) {
-                        const int c = lane & 7;
-                        const __nv_bfloat16* src = (lane < 8 ? p.k_new : p.v_new) + (size_t)t * p.q_stride + (size_t)(head0 + hl) * D + c * 8;
-                        const uint4 v = *reinterpret_cast<const uint4*>(src);
-                        *reinterpret_cast<uint4*>((lane < 8 ? kh : vh) + tile_off(slot, c)) = v;
-                        __nv_bfloat16* dst = p.cache + (size_t)page * page_stride + (size_t)(head0 + hl) * head_plane + (size_t)slot * D + c * 8;
-                        *reinterpret_cast<uint4*>(lane < 8 ? dst : dst + (size_t)p.H * head_plane) = v;
-                    }
-                    for (int r = slot + 1 + (lane >> 3); r < p.P; r += 4)
-                        *reinterpret_cast<uint4*>(vh + tile_off(r, lane & 7)) = make_uint4(0, 0, 0, 0);
-                    __syncwarp();
+            if (key0 + p.P > pos) {
+                // the page of the token's own position: its new key and value, and zeros for the unwritten slots
+                const int slot = pos - key0;
+                if (p.k_new != nullptr && lane < 16) {
+                    const int c = lane & 7;
+                    const __nv_bfloat16* src = (lane < 8 ? p.k_new : p.v_new) + (size_t)t * p.q_stride + (size_t)h * D + c * 8;
+                    const uint4 v = *reinterpret_cast<const uint4*>(src);
+                    *reinterpret_cast<uint4*>((lane < 8 ? kh : vh) + tile_off(slot, c)) = v;
+                    __nv_bfloat16* dst = p.cache + (size_t)page * page_stride + (size_t)h * head_plane + (size_t)slot * D + c * 8;
+                    *reinterpret_cast<uint4*>(lane < 8 ? dst : dst + (size_t)p.H * head_plane) = v;
                 }
-                for (int tt = 0; tt < p.P / TILE; ++tt) {
-                    const int base = key0 + tt * TILE;
-                    if (base > pos || base + TILE <= lo) continue;          // no live key in this tile
-                    const uint8_t* kt = kh + tt * TILE * 128;
-                    const uint8_t* vt = vh + tt * TILE * 128;
-                    // scores of 16 keys against the query (row 0)
-                    float sc[2][2];
-                    sc[0][0] = sc[0][1] = sc[1][0] = sc[1][1] = 0.f;
-                    const int mi = lane >> 3;
+                for (int r = slot + 1 + (lane >> 3); r < p.P; r += 4)
+                    *reinterpret_cast<uint4*>(vh + tile_off(r, lane & 7)) = make_uint4(0, 0, 0, 0);
+                tc::fence_proxy_async();                    // (the token's last page: no later request writes over it, as it stands)
+                __syncwarp();
+            }
+#pragma unroll 1
+            for (int tt = 0; tt < p.P / TILE; ++tt) {
+                const int base = key0 + tt * TILE;
+                if (base > pos || base + TILE <= lo) continue;          // no live key in this tile
+                const uint8_t* kt = kh + tt * TILE * 128;
+                const uint8_t* vt = vh + tt * TILE * 128;
+                // scores of 16 keys (the rows of A), in two independent parts: keys quad and quad + 8 in each lane of the quad
+                float part[2][2];
+                const int mi = lane >> 3;
 #pragma unroll
-                    for (int ks = 0; ks < D / 16; ++ks) {
-                        uint32_t b[4];
-                        ldmatrix_x4(smem_addr(kt + tile_off((mi >> 1) * 8 + (lane & 7), 2 * ks + (mi & 1))), b);
-                        mma_bf16_row0(sc[0][0], sc[0][1], qf[u][ks][0], qf[u][ks][1], b[0], b[1]);
-                        mma_bf16_row0(sc[1][0], sc[1][1], qf[u][ks][0], qf[u][ks][1], b[2], b[3]);
-                    }
-                    // row 0 lives in lanes 0..3 (elements 0 and 1 of each 8-key tile); the other rows are idle
-                    float mx = -CUDART_INF_F;
+                for (int ks = 0; ks < D / 16; ++ks) {
+                    uint32_t a[4];
+                    ldmatrix_x4(smem_addr(kt + tile_off((mi & 1) * 8 + (lane & 7), 2 * ks + (mi >> 1))), a);
+                    float* c = part[ks & 1];
+                    if (ks < 2) c[0] = c[1] = 0.f;
+                    mma_bf16_column(c[0], c[1], a, qf[ks][0], qf[ks][1]);
+                }
+                const int key = base + quad;
+                const float s0 = key <= pos && key >= lo ? (part[0][0] + part[1][0]) * p.scale_log2e : -CUDART_INF_F;
+                const float s1 = key + 8 <= pos && key + 8 >= lo ? (part[0][1] + part[1][1]) * p.scale_log2e : -CUDART_INF_F;
+                float mx = fmaxf(s0, s1);
 #pragma unroll
-                    for (int nt = 0; nt < 2; ++nt)
+                for (int x = 4; x < 32; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+                const float m_new = fmaxf(m, mx);               // the tile holds at least one live key
+                const float corr = exp2f(m - m_new);
+                m = m_new;
+                const float p0 = exp2f(s0 - m_new), p1 = exp2f(s1 - m_new);
+                l = l * corr + (p0 + p1);
+                // the weights as the B operand: a lane gets keys 2 t4, 2 t4 + 1 and the same + 8 from the quads that hold them
+                const uint32_t mine = pack_bf16(p0, p1);
+                const uint32_t even = __shfl_sync(0xffffffffu, mine, 8 * t4), odd = __shfl_sync(0xffffffffu, mine, 8 * t4 + 4);
+                const uint32_t w0 = __byte_perm(even, odd, 0x5410), w1 = __byte_perm(even, odd, 0x7632);
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            const int key = base + nt * 8 + 2 * t4 + e;
-                            const float v = (key <= pos && key >= lo) ? sc[nt][e] * p.scale_log2e : -CUDART_INF_F;
-                            sc[nt][e] = v;
-                            mx = fmaxf(mx, v);
-                        }
-                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                    const float m_new = fmaxf(m[u], mx);               // the tile holds at least one live key
-                    const float corr = exp2f(m[u] - m_new);
-                    m[u] = m_new;
-                    l[u] *= corr;
-                    uint32_t pf[2];
-                    {
-                        const float p00 = exp2f(sc[0][0] - m_new), p01 = exp2f(sc[0][1] - m_new);
-                        const float p10 = exp2f(sc[1][0] - m_new), p11 = exp2f(sc[1][1] - m_new);
-                        l[u] += (p00 + p01) + (p10 + p11);
-                        pf[0] = quad == 0 ? pack_bf16(p00, p01) : 0u;
-                        pf[1] = quad == 0 ? pack_bf16(p10, p11) : 0u;
-                    }
-#pragma unroll
-                    for (int j = 0; j < D / 8; ++j) { o[u][j][0] *= corr; o[u][j][1] *= corr; }
-#pragma unroll
-                    for (int dp = 0; dp < D / 16; ++dp) {
-                        uint32_t b[4];
-                        ldmatrix_x4_trans(smem_addr(vt + tile_off((mi & 1) * 8 + (lane & 7), 2 * dp + (mi >> 1))), b);
-                        mma_bf16_row0(o[u][2 * dp][0], o[u][2 * dp][1], pf[0], pf[1], b[0], b[1]);
-                        mma_bf16_row0(o[u][2 * dp + 1][0], o[u][2 * dp + 1][1], pf[0], pf[1], b[2], b[3]);
-                    }
+                for (int j = 0; j < D / 16; ++j) {
+                    uint32_t a[4];
+                    ldmatrix_x4_trans(smem_addr(vt + tile_off((mi >> 1) * 8 + (lane & 7), 2 * j + (mi & 1))), a);
+                    o[j][0] *= corr;
+                    o[j][1] *= corr;
+                    mma_bf16_column(o[j][0], o[j][1], a, w0, w1);
                 }
             }
         }
-        __syncthreads();                                    // every warp is done with the stage
-        if (threadIdx.x == 0 && i + p.stages < n_mine) load_page(i + p.stages);
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&empty[s]);          // this warp is done with the stage
+        if (++s == p.stages) { s = 0; phase ^= 1; }
     }
+    if (!ok && lane == 0) atomicOr(p.error_flag, 8);
 
-    // row 0: lanes 0..3 hold dims 8j + 2*t4 + {0,1}; their sums of l differ by the keys each saw
+    // every lane of a quad holds the same: lane t4 stores dimensions 16 t4 + quad and 16 t4 + 8 + quad
 #pragma unroll
-    for (int u = 0; u < HEADS_PER_WARP; ++u) {
-        const int hl = warp + u * WARPS;
-        float lu = l[u];
-        lu += __shfl_xor_sync(0xffffffffu, lu, 1);
-        lu += __shfl_xor_sync(0xffffffffu, lu, 2);
-        if (hl >= group_heads || quad != 0) continue;
-        const int h = head0 + hl;
-        if (n_splits == 1) {
-            float inv = lu > 0.f ? 1.f / lu : 0.f;
-            if (p.gate) inv *= 1.0f / (1.0f + __expf(-__bfloat162float(p.gate[(size_t)t * p.gate_stride + h])));
-            __nv_bfloat16* dst = p.out + (size_t)t * p.out_stride + (size_t)h * D + 2 * t4;
-#pragma unroll
-            for (int j = 0; j < D / 8; ++j) *reinterpret_cast<uint32_t*>(dst + j * 8) = pack_bf16(o[u][j][0] * inv, o[u][j][1] * inv);
-        } else {
-            const size_t item = ((size_t)t * p.H + h) * gridDim.z + split;     // the scratch is laid out for the most splits
-            float* dst = p.part_o + item * D + 2 * t4;
-#pragma unroll
-            for (int j = 0; j < D / 8; ++j) *reinterpret_cast<float2*>(dst + j * 8) = make_float2(o[u][j][0], o[u][j][1]);
-            if (t4 == 0) { p.part_ml[2 * item] = m[u]; p.part_ml[2 * item + 1] = lu; }
-        }
+    for (int x = 4; x < 32; x <<= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
+    const int d = 16 * t4 + quad;
+    const float o0 = t4 == 0 ? o[0][0] : (t4 == 1 ? o[1][0] : (t4 == 2 ? o[2][0] : o[3][0]));
+    const float o1 = t4 == 0 ? o[0][1] : (t4 == 1 ? o[1][1] : (t4 == 2 ? o[2][1] : o[3][1]));
+    if (n_splits == 1) {
+        float inv = l > 0.f ? 1.f / l : 0.f;
+        if (p.gate) inv *= 1.0f / (1.0f + __expf(-__bfloat162float(p.gate[(size_t)t * p.gate_stride + h])));
+        __nv_bfloat16* dst = p.out + (size_t)t * p.out_stride + (size_t)h * D + d;
+        dst[0] = __float2bfloat16_rn(o0 * inv);
+        dst[8] = __float2bfloat16_rn(o1 * inv);
+        return;
     }
-    if (threadIdx.x == 0 && abort_flag) atomicOr(p.error_flag, 8);
-    if (n_splits == 1) return;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int prev = atomicAdd(&p.counters[t * gridDim.y + g], 1);
-        sh_last = prev == n_splits - 1;
+    const size_t first = ((size_t)t * p.H + h) * gridDim.z;     // the scratch is laid out for the most splits
+    {
+        float* dst = p.part_o + (first + split) * D + d;
+        dst[0] = o0;
+        dst[8] = o1;
+        if (lane == 0) *reinterpret_cast<float2*>(p.part_ml + 2 * (first + split)) = make_float2(m, l);
+        __threadfence();
     }
-    __syncthreads();
-    if (!sh_last) return;
+    __syncwarp();
+    int last = 0;
+    if (lane == 0) last = atomicAdd(&p.counters[t * p.H + h], 1) == n_splits - 1;
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
     __threadfence();
-    // The block that finished last merges the group's heads: a thread per output dimension, the partial maxima, sums
-    // and outputs of eight splits requested together and merged with a running maximum.
-    for (int idx = threadIdx.x; idx < group_heads * D; idx += THREADS) {
-        const int h = head0 + idx / D, d = idx % D;
-        const size_t first = ((size_t)t * p.H + h) * gridDim.z;
-        float Mx = -CUDART_INF_F, Lx = 0.f, acc = 0.f;
-        for (int sp0 = 0; sp0 < n_splits; sp0 += 8) {
-            float mm[8], ll[8], oo[8];
+    // The warp that finished last merges the head: a lane per two output dimensions, the partial maxima and sums of eight
+    // splits in eight lanes, everything of eight splits requested together and merged with a running maximum.
+    float Mx = -CUDART_INF_F, Lx = 0.f, a0 = 0.f, a1 = 0.f;
+    for (int sp0 = 0; sp0 < n_splits; sp0 += 8) {
+        const int mine = sp0 + (lane & 7);
+        float2 ml = make_float2(-CUDART_INF_F, 0.f), oo[8];
+        if (mine < n_splits) ml = __ldcg(reinterpret_cast<const float2*>(p.part_ml + 2 * (first + mine)));
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const bool live = sp0 + u < n_splits;
-                const size_t it = first + sp0 + (live ? u : 0);
-                mm[u] = live ? __ldcg(p.part_ml + 2 * it) : -CUDART_INF_F;
-                ll[u] = live ? __ldcg(p.part_ml + 2 * it + 1) : 0.f;
-                oo[u] = live ? __ldcg(p.part_o + it * D + d) : 0.f;
+        for (int u = 0; u < 8; ++u)
+            oo[u] = sp0 + u < n_splits ? __ldcg(reinterpret_cast<const float2*>(p.part_o + (first + sp0 + u) * D) + lane) : make_float2(0.f, 0.f);
+        float cm = ml.y > 0.f ? ml.x : -CUDART_INF_F;
+#pragma unroll
+        for (int x = 4; x > 0; x >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, x));
+        cm = fmaxf(cm, Mx);
+        if (cm == -CUDART_INF_F) continue;                  // nothing live so far
+        const float keep = Mx == -CUDART_INF_F ? 0.f : exp2f(Mx - cm);
+        Mx = cm;
+        const float w = ml.y > 0.f ? exp2f(ml.x - Mx) : 0.f;
+        float sum = ml.y > 0.f ? ml.y * w : 0.f;
+#pragma unroll
+        for (int x = 4; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
+        Lx = Lx * keep + sum;
+        a0 *= keep;
+        a1 *= keep;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const float wu = __shfl_sync(0xffffffffu, w, u);
+            if (wu > 0.f) {                                 // a split without a live key adds nothing, whatever its scratch holds
+                a0 += oo[u].x * wu;
+                a1 += oo[u].y * wu;
             }
-            float cm = Mx;
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (ll[u] > 0.f) cm = fmaxf(cm, mm[u]);
-            if (cm == -CUDART_INF_F) continue;            // nothing live so far
-            const float keep = Mx == -CUDART_INF_F ? 0.f : exp2f(Mx - cm);
-            acc *= keep;
-            Lx *= keep;
-            Mx = cm;
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (ll[u] > 0.f) {
-                    const float w = exp2f(mm[u] - Mx);
-                    Lx += ll[u] * w;
-                    acc += oo[u] * w;
-                }
         }
-        const float gated = p.gate ? 1.0f / (1.0f + __expf(-__bfloat162float(p.gate[(size_t)t * p.gate_stride + h]))) : 1.0f;
-        p.out[(size_t)t * p.out_stride + (size_t)h * D + d] = __float2bfloat16_rn(Lx > 0.f ? acc / Lx * gated : 0.f);
     }
-    if (threadIdx.x == 0) p.counters[t * gridDim.y + g] = 0;
+    const float gated = p.gate ? 1.0f / (1.0f + __expf(-__bfloat162float(p.gate[(size_t)t * p.gate_stride + h]))) : 1.0f;
+    const float inv = Lx > 0.f ? gated / Lx : 0.f;
+    *reinterpret_cast<uint32_t*>(p.out + (size_t)t * p.out_stride + (size_t)h * D + 2 * lane) = pack_bf16(a0 * inv, a1 * inv);
+    if (lane == 0) p.counters[t * p.H + h] = 0;
 }
 
 typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -370,9 +392,13 @@ EncodeTiled encode_fn() {
     return fn;
 }
 
-// heads per block: as many as two per warp and 256 box rows allow, spread evenly over the groups
-void grouping(int n_heads, int page_size, int* group, int* n_groups) {
-    const int most = MAX_GROUP < 256 / page_size ? MAX_GROUP : 256 / page_size;
+// Heads per block, spread evenly over the groups: up to seven (a warp each, 256 box rows at most), since the fewer and
+// larger the boxes the better they stream (64 tokens x 25 heads: a step of 195 ms in groups of 7, 214 in groups of 5);
+// up to four while a step has so few tokens that its blocks, in eight splits, stay below 1.35 an SM: then it is the
+// chain of a block's pages that counts (1 token x 16 heads: 0.5 to 2 % of a whole step, 5 tokens 2 %).
+void grouping(int n_tokens, int n_heads, int page_size, int sm_count, int* group, int* n_groups) {
+    int most = MAX_GROUP < 256 / page_size ? MAX_GROUP : 256 / page_size;
+    if (most > 4 && (long long)n_tokens * dd_ceil_div(n_heads, 4) * 8 * 20 <= 27ll * sm_count) most = 4;
     *n_groups = dd_ceil_div(n_heads, most);
     *group = dd_ceil_div(n_heads, *n_groups);
 }
@@ -390,7 +416,7 @@ DD_API int dd_attention_decode_pages_supported(int n_heads, int n_kv_heads, int 
 // keys: 8 splits, all blocks resident, 13 us; a second wave of blocks 18 us).
 DD_API int dd_attention_decode_pages_splits(int n_tokens, int n_heads, int page_size, int context, int sm_count) {
     int group = 0, n_groups = 0;
-    grouping(n_heads, page_size, &group, &n_groups);
+    grouping(n_tokens < 1 ? 1 : n_tokens, n_heads, page_size, sm_count, &group, &n_groups);
     const int pages = dd_ceil_div(context < 1 ? 1 : context, page_size);
     // A token gets pages / (all pages x groups / resident blocks) splits: with equal contexts that is resident blocks
     // / (tokens x groups); a token 2.5 times as long as the average gets 2.5 times as many, and the grid allows for
@@ -429,15 +455,6 @@ DD_API int dd_attention_decode_pages(const void* q, int q_stride, const void* k_
     EncodeTiled enc = encode_fn();
     if (!enc) return dd_fail("dd_attention_decode_pages: cuTensorMapEncodeTiled is not available from this driver");
     Params p;
-    int n_groups = 0;
-    grouping(n_heads, page_size, &p.G, &n_groups);
-    const int box_rows = p.G * page_size, box_bytes = box_rows * 128;
-    p.stages = (106 * 1024) / (2 * box_bytes);            // two blocks per SM
-    int blocks_per_sm = 2;
-    if (p.stages < 2) {                                               // large pages: one block per SM
-        p.stages = (210 * 1024) / (2 * box_bytes);
-        blocks_per_sm = 1;
-    }
     static int sm_count = 0;
     if (!sm_count) {
         int dev = 0;
@@ -445,26 +462,38 @@ DD_API int dd_attention_decode_pages(const void* q, int q_stride, const void* k_
         cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
         if (sm_count <= 0) sm_count = 148;
     }
+    int n_groups = 0;
+    grouping(n_tokens, n_heads, page_size, sm_count, &p.G, &n_groups);
+    const int box_bytes = p.G * page_size * 128;
+    p.stages = (106 * 1024) / (2 * box_bytes);            // two blocks per SM
+    int blocks_per_sm = 2;
+    if (p.stages < 2) {                                               // large pages: one block per SM
+        p.stages = (210 * 1024) / (2 * box_bytes);
+        blocks_per_sm = 1;
+    }
     p.inv_block_budget = 1.0f / (float)(blocks_per_sm * sm_count);
     p.deal = (long long)n_tokens * n_groups * n_splits > (long long)blocks_per_sm * sm_count;
     p.log2_P = page_size == 16 ? 4 : (page_size == 32 ? 5 : (page_size == 64 ? 6 : 7));
     if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
     if (p.stages < 2) return dd_fail("dd_attention_decode_pages: a page of %d heads x %d tokens does not fit twice into shared memory", p.G, page_size);
-    const int smem = p.stages * 2 * box_bytes + 1024 + MAX_STAGES * 8 + MAX_BLOCK_PAGES * 4;
+    const int smem = p.stages * 2 * box_bytes + 1024 + MAX_STAGES * (2 * 8 + 4);
     static int configured = 0;
     if (configured < smem) {
         cudaError_t e = cudaFuncSetAttribute(attention_decode_pages_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return dd_fail("dd_attention_decode_pages: shared memory of %d bytes refused: %s", smem, cudaGetErrorString(e));
         configured = smem;
     }
-    CUtensorMap map;
+    CUtensorMap maps[2];
     cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)n_pages * 2 * n_heads * page_size};
     cuuint64_t strides[1] = {(cuuint64_t)D * 2};
-    cuuint32_t box[2] = {(cuuint32_t)D, (cuuint32_t)box_rows};
     cuuint32_t elem[2] = {1, 1};
-    CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, cache, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return dd_fail("dd_attention_decode_pages: cannot describe the cache to TMA (driver error %d)", (int)r);
+    for (int i = 0; i < 2; ++i) {
+        // the last group may hold fewer heads: a box of its own reads no neighbour's rows (25 heads in groups of 7: 28 were read)
+        cuuint32_t box[2] = {(cuuint32_t)D, (cuuint32_t)((i ? n_heads - (n_groups - 1) * p.G : p.G) * page_size)};
+        CUresult r = enc(&maps[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, cache, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return dd_fail("dd_attention_decode_pages: cannot describe the cache to TMA (driver error %d)", (int)r);
+    }
     p.q = (const __nv_bfloat16*)q; p.k_new = (const __nv_bfloat16*)k_new; p.v_new = (const __nv_bfloat16*)v_new;
     p.cache = (__nv_bfloat16*)cache; p.tok_entry = tok_entry; p.tok_pos = tok_pos; p.block_table = block_table;
     p.out = (__nv_bfloat16*)out; p.part_o = part_o; p.part_ml = part_ml; p.counters = counters; p.error_flag = error_flag;
@@ -472,6 +501,6 @@ DD_API int dd_attention_decode_pages(const void* q, int q_stride, const void* k_
     p.n_pages = n_pages; p.window = window; p.chunk = chunk; p.gate = (const __nv_bfloat16*)gate; p.gate_stride = gate_stride;
     p.scale_log2e = scale * 1.4426950408889634f;
     p.n_tokens = n_tokens;
-    dd_launch(attention_decode_pages_kernel, dim3(n_tokens, n_groups, n_splits), dim3(THREADS), (size_t)smem, (cudaStream_t)stream, map, p);
+    dd_launch(attention_decode_pages_kernel, dim3(n_tokens, n_groups, n_splits), dim3((p.G + 1) * 32), (size_t)smem, (cudaStream_t)stream, maps[0], maps[1], p);
     return dd_check_launch("dd_attention_decode_pages");
 }

@@ -19,12 +19,11 @@ from .. import kernels
 
 @dataclass(frozen=True)
 class AttentionTuning:
-    """Thresholds of the kernel choice. The defaults were measured on a B200 with 25 heads of 64 and 768 keys per
-    request: the page-streaming decode kernel wins from 8 requests on (11.6 against 14.0 us; 54 against 68 us at 64
-    requests) and loses at 4 and below (11.0 against 9.8 us; 9.1 against 5.5 us at one request)."""
-    pages_from_pairs: int = 150           # decode steps with at least this many (token, head) pairs stream whole pages,
-    pages_from_pair_keys: int = 200_000   # ... or with this many pairs x keys of context (one request of 16,384 keys:
-                                          # 36 us in pages, 45 us in rows; two of 4,096: 25 us either way; one: 22 / 15)
+    """Thresholds of the kernel choice, measured on a B200 with 25 heads of 64: from pages_from_pairs on the key splits are those
+    of the page-streaming decode kernel, which deals them out by the contexts; below, a token's keys are cut by
+    row_keys_per_block (the launcher of the row kernel gives sizes that page streaming takes to that kernel all the same)."""
+    pages_from_pairs: int = 150           # decode steps with at least this many (token, head) pairs deal the splits out,
+    pages_from_pair_keys: int = 200_000   # ... or with this many pairs x keys of context (one request of 16,384 keys)
     pages_per_block: int = 128            # a block of the page-streaming kernel holds the ids of this many pages
     row_keys_per_block: int = 128         # key split of the row decode kernel: keys per block ...
     row_blocks_per_sm: int = 2            # ... and blocks wanted per SM

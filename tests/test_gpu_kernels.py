@@ -242,6 +242,25 @@ def test_attention_decode_pages(K, heads, page, n_splits, window):
     assert 1 <= K.attention_decode_pages_splits(8, heads, page, 1000, DEV) <= (1000 + page - 1) // page
 
 
+@pytest.mark.parametrize("heads,page,lengths", [(25, 16, [540]), (25, 16, [3, 1000, 64]), (5, 32, [17, 129, 1, 300]), (9, 16, [77] * 9),
+                                                (3, 128, [1000])])
+@pytest.mark.parametrize("n_splits", [1, 4, 9])
+def test_attention_decode_of_few_tokens(K, heads, page, lengths, n_splits):
+    """Few (token, head) pairs are page-streamed in groups of at most four heads (the last group smaller), whichever kernel is
+    asked for; a page that is missing is reported, as a write too where the token's own key belongs there."""
+    c = paged_case(K, torch.bfloat16, heads, heads, 64, page, lengths=lengths, new=[1] * len(lengths), window=None, n_splits=n_splits, spike=5)
+    args = (None, c["pos"], c["table"], heads, c["scale"])
+    out, pages = (K.attention_decode(c["q"], c["cache"], *args, n_splits=n_splits, kernel=k) for k in ("rows", "pages"))
+    assert K.read_error_flag(DEV) == 0 and torch.equal(out, pages)
+    assert (out.double().cpu() - c["ref"]).abs().max() < tol(torch.bfloat16)
+    for own, bits in ((False, 4), (True, 6)):
+        if len(lengths) == 1 and (own or lengths[0] > page):
+            args[2][0, (lengths[0] - 1) // page if own else 0] = -1
+            new = {} if not own else dict(k_new=c["packed"][:, heads * 64:2 * heads * 64], v_new=c["packed"][:, 2 * heads * 64:])
+            K.attention_decode(c["q"], c["cache"], *args, n_splits=n_splits, **new)
+            assert K.read_error_flag(DEV) == bits
+
+
 @pytest.mark.parametrize("heads,page", [(25, 16), (8, 64), (20, 32)])
 @pytest.mark.parametrize("n_splits", [3, 8])
 @pytest.mark.parametrize("window", [None, 100])
