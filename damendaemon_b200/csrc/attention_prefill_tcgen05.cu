@@ -11,7 +11,7 @@
 //               O_t += P_t V (128 x 64, accumulated in TMEM over all blocks) for whichever tile has its P ready
 //               first, with P read from tensor memory (64 columns of its own per tile) and V read as it lies in
 //               memory, as an MN-major operand;
-//   warps 2..5 and 6..9  softmax of the lower and of the upper tile: a thread owns one query row (its TMEM lane),
+//   warps 4..7 and 8..11 softmax of the lower and of the upper tile: a thread owns one query row (its TMEM lane),
 //               takes the row's 128 scores of a block into registers with four TMEM loads in flight, and writes
 //               P as bfloat16 pairs into tensor memory. Scaling and row sums use float32 pair instructions and
 //               the maximum a three-input instruction: the warps are bound by what they can issue as much as by
@@ -32,7 +32,7 @@
 #include <math_constants.h>
 
 namespace {
-constexpr int BQ = 128, TILES = 2, BKV = 128, D = 64, THREADS = 64 + TILES * 128, STAGES = 4;
+constexpr int BQ = 128, TILES = 2, BKV = 128, D = 64, THREADS = 128 + TILES * 128, STAGES = 4;
 constexpr int TILE_BYTES = BKV * D * 2;             // one 128 x 64 bf16 tile: 16 KB
 constexpr int Q_BYTES = TILES * TILE_BYTES;         // the two query tiles, one after the other
 constexpr int STAGE_BYTES = 2 * TILE_BYTES;         // keys, then values
@@ -181,305 +181,314 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     const uint32_t tmem_base = *tmem_slot;
     dd_grid_wait();              // queries and the cache are earlier kernels' results
 
-    if (warp == 0) {
-        // ---- TMA ----
-        if (lane == 0) {
-            tc::mbar_expect_tx(q_full, Q_BYTES);
-            tc::tma_load_2d(sQ, &map_q, h * D, row0, q_full);       // rows past the last token read as zeros
+    // A softmax thread holds its row's 128 scores and wants more than the 168 registers that twelve warps may have each (ten
+    // warps: 168 too, an SM's quarter holds three of them; the spills cost 12 %, one prompt of 4,096 tokens 107 us, now 93.5):
+    // the warpgroup of the fetching and the issuing warp gives some up. 128 x 72 + 256 x 216 are the launch's 384 x 168.
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+        if (warp == 0) {
+            // ---- TMA ----
+            if (lane == 0) {
+                tc::mbar_expect_tx(q_full, Q_BYTES);
+                tc::tma_load_2d(sQ, &map_q, h * D, row0, q_full);       // rows past the last token read as zeros
+            }
+            const int pages_per_block = BKV / p.P;
+            const int* bt = p.block_table + (size_t)e * p.max_blocks;
+            const uint32_t page_bytes = (uint32_t)p.P * D * 2;
+            const int kv_lo = tile_lo(0);
+            // The warp holds 32 consecutive entries of the request's block table, one per lane, and the next 32 already
+            // requested: a key block's pages never straddle such a window (its first entry is a multiple of the pages
+            // per block, which divide 32), and no block waits for a table read of its own.
+            auto table_window = [&](int w) { const int i = w * 32 + lane; return i < p.max_blocks ? bt[i] : -1; };
+            int window_at = (kb_first / p.P) / 32;
+            int held = table_window(window_at), ahead = table_window(window_at + 1);
+            for (int j = 0; j < n_blocks; ++j) {
+                const int s = j % STAGES;
+                if (j >= STAGES) {
+                    bool ok = true;
+                    if (lane == 0) ok = tc::mbar_wait(&kv_empty[s], ((j / STAGES) - 1) & 1, abort_flag);
+                    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                    if (!ok) break;
+                }
+                const int kb = kb_first + j * BKV;
+                uint8_t* k_dst = sKV + s * STAGE_BYTES;
+                uint8_t* v_dst = k_dst + TILE_BYTES;
+                if (p.new_rows && kb >= pos0) {
+                    // Every key of this block is one of this step's own: they lie row after row beside the queries, so one
+                    // box of 128 rows brings the keys and one the values (a box per cache page costs the TMA unit about
+                    // 60 ns each, 1 us per block with pages of 16 tokens, which is what bounded whole prompts). Rows past
+                    // the entry are other requests' tokens or zeros: masked by position like any key after the query.
+                    if (lane == 0) {
+                        const int row = (row0 - q0) + kb - pos0;       // the entry's first row + (key - its first position)
+                        tc::mbar_expect_tx(&kv_full[s], STAGE_BYTES);
+                        tc::tma_load_2d(k_dst, &map_k_new, kh * D, row, &kv_full[s]);
+                        tc::tma_load_2d(v_dst, &map_v_new, kh * D, row, &kv_full[s]);
+                    }
+                    continue;
+                }
+                const int first_entry = kb / p.P;
+                if (first_entry / 32 != window_at) {
+                    window_at = first_entry / 32;
+                    held = ahead;
+                    ahead = table_window(window_at + 1);
+                }
+                // lanes 0 .. pages-1 fetch the key boxes of the block's pages, the next `pages` lanes the value boxes
+                const int slot = lane < pages_per_block ? lane : lane - pages_per_block;
+                const bool values = lane >= pages_per_block;
+                const int page = __shfl_sync(0xffffffffu, held, (first_entry + slot) & 31);
+                bool valid = false;
+                if (lane < 2 * pages_per_block) {
+                    const int key0 = kb + slot * p.P;
+                    valid = key0 <= pos_last && key0 + p.P > kv_lo;
+                    if (valid && (page < 0 || page >= p.n_pages)) {
+                        atomicOr(p.error_flag, 4);
+                        valid = false;
+                    }
+                }
+                const int n_valid = __popc(__ballot_sync(0xffffffffu, valid));          // boxes, keys and values counted apart
+                if (lane < 2 * pages_per_block) {
+                    if (valid) {
+                        const int row = ((page * 2 + (values ? 1 : 0)) * p.KH + kh) * p.P;
+                        tc::tma_load_2d((values ? v_dst : k_dst) + slot * page_bytes, &map_kv, 0, row, &kv_full[s]);
+                    } else if (values) {
+                        // no live key in this page: its scores are all masked; its value rows must be zeros
+                        uint4* z = reinterpret_cast<uint4*>(v_dst + slot * page_bytes);
+                        for (uint32_t i = 0; i < page_bytes / 16; ++i) z[i] = make_uint4(0, 0, 0, 0);
+                        tc::fence_proxy_async();
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) tc::mbar_expect_tx(&kv_full[s], (uint32_t)n_valid * page_bytes);
+            }
+            if (p.store_new && h % (p.H / p.KH) == 0) {
+                // The pair's own keys and values are its last key blocks (one per tile), and they lie in shared memory in
+                // the layout of the cache's tensor map: TMA writes them into their pages, one box per page, while the block
+                // works on them. No block of this launch reads these cache rows: with every entry starting on a key-block
+                // boundary, the key blocks that hold this step's tokens are read from k_new/v_new. A page that the entry
+                // fills only in part receives whatever follows the entry's last token in its other slots; slots past a
+                // request's length are never read by anyone.
+                if (pos0 % BKV != 0) {
+                    if (lane == 0) atomicOr(p.error_flag, 2);        // the caller broke the rule: nothing is written
+                } else {
+                    for (int j = n_blocks - n_tiles; j < n_blocks; ++j) {
+                        const int s = j % STAGES, kb = kb_first + j * BKV;
+                        if (!tc::mbar_wait(&kv_full[s], (j / STAGES) & 1, abort_flag)) break;
+                        if (lane < 2 * pages_per_block) {
+                            const int slot = lane < pages_per_block ? lane : lane - pages_per_block;
+                            const bool values = lane >= pages_per_block;
+                            const int key0 = kb + slot * p.P;
+                            if (key0 <= pos_last) {
+                                const int page = bt[key0 / p.P];
+                                if (page < 0 || page >= p.n_pages) atomicOr(p.error_flag, 2);
+                                else
+                                    tc::tma_store_2d(&map_kv, 0, ((page * 2 + (values ? 1 : 0)) * p.KH + kh) * p.P,
+                                                     sKV + s * STAGE_BYTES + (values ? TILE_BYTES : 0) + slot * page_bytes);
+                            }
+                        }
+                    }
+                    tc::bulk_commit();
+                    tc::bulk_wait_all();         // shared memory has been read and the cache written before the block leaves
+                }
+            }
+        } else if (warp == 1) {
+            // ---- MMA ----
+            if (tc::elect_one()) {
+                constexpr uint32_t idesc_s = tc::idesc_bf16_f32(BQ, BKV);
+                constexpr uint32_t idesc_o = tc::idesc_bf16_f32_b_mn(BQ, D);
+                const uint32_t q_addr = tc::smem_u32(sQ);
+                int first[TILES], last[TILES], scored[TILES], added[TILES];
+#pragma unroll
+                for (int t = 0; t < TILES; ++t) {
+                    first[t] = block_first(t);
+                    last[t] = t < n_tiles ? block_last(t) : -1;
+                    scored[t] = added[t] = 0;
+                }
+                bool ok = tc::mbar_wait(q_full, 0, abort_flag);
+                tc::fence_after_sync();
+                // S_t = Q_t K_j^T for the tiles that take part in key block j, as soon as a tile's softmax warps have taken
+                // its previous scores into registers
+                auto issue_scores = [&](int j) {
+                    const int s = j % STAGES;
+                    if (!tc::mbar_wait(&kv_full[s], (j / STAGES) & 1, abort_flag)) { ok = false; return; }
+                    const uint32_t k_addr = tc::smem_u32(sKV + s * STAGE_BYTES);
+#pragma unroll
+                    for (int t = 0; t < TILES; ++t) {
+                        if (j < first[t] || j > last[t]) continue;
+                        if (scored[t] > 0 && !tc::mbar_wait(&s_free[t], (scored[t] - 1) & 1, abort_flag)) { ok = false; return; }
+                        tc::fence_after_sync();
+#pragma unroll
+                        for (int k = 0; k < D / 16; ++k)
+                            tc::mma_bf16(tmem_base + s_col(t), tc::smem_desc_sw128(q_addr + t * TILE_BYTES + k * 32),
+                                         tc::smem_desc_sw128(k_addr + k * 32), idesc_s, k > 0 ? 1u : 0u);
+                        tc::mma_commit(&s_full[t]);
+                        ++scored[t];
+                    }
+                };
+                if (ok) issue_scores(0);
+                for (int j = 0; j < n_blocks && ok; ++j) {
+                    if (j + 1 < n_blocks) issue_scores(j + 1);
+                    if (!ok) break;
+                    // O_t += P_t V_j, for each tile as soon as its P is there, whichever comes first
+                    const int s = j % STAGES;
+                    const uint32_t v_addr = tc::smem_u32(sKV + s * STAGE_BYTES + TILE_BYTES);
+                    uint32_t pending = 0;
+#pragma unroll
+                    for (int t = 0; t < TILES; ++t)
+                        if (j >= first[t] && j <= last[t]) pending |= 1u << t;
+                    const unsigned long long start = tc::global_ns();
+                    uint32_t spins = 0;
+                    while (pending && ok) {
+#pragma unroll
+                        for (int t = 0; t < TILES; ++t) {
+                            if (!(pending & (1u << t)) || !tc::mbar_try_wait(&p_ready[t], added[t] & 1)) continue;
+                            tc::fence_after_sync();
+#pragma unroll
+                            for (int k = 0; k < BKV / 16; ++k)
+                                tc::mma_bf16_a_tmem(tmem_base + o_col(t), tmem_base + p_col(t) + k * 8,
+                                                    tc::smem_desc_sw128_mn(v_addr + k * 16 * D * 2, 1024), idesc_o,
+                                                    (added[t] > 0 || k > 0) ? 1u : 0u);
+                            tc::mma_commit(&o_full[t]);
+                            ++added[t];
+                            pending &= ~(1u << t);
+                        }
+                        if (pending && (++spins & 0x3ff) == 0 && (*abort_flag || tc::global_ns() - start > tc::WAIT_LIMIT_NS)) {
+                            *abort_flag = 1;
+                            ok = false;
+                        }
+                    }
+                    if (ok) tc::mma_commit(&kv_empty[s]);            // keys and values of this block have been read
+                }
+            }
         }
-        const int pages_per_block = BKV / p.P;
-        const int* bt = p.block_table + (size_t)e * p.max_blocks;
-        const uint32_t page_bytes = (uint32_t)p.P * D * 2;
-        const int kv_lo = tile_lo(0);
-        // The warp holds 32 consecutive entries of the request's block table, one per lane, and the next 32 already
-        // requested: a key block's pages never straddle such a window (its first entry is a multiple of the pages
-        // per block, which divide 32), and no block waits for a table read of its own.
-        auto table_window = [&](int w) { const int i = w * 32 + lane; return i < p.max_blocks ? bt[i] : -1; };
-        int window_at = (kb_first / p.P) / 32;
-        int held = table_window(window_at), ahead = table_window(window_at + 1);
-        for (int j = 0; j < n_blocks; ++j) {
-            const int s = j % STAGES;
-            if (j >= STAGES) {
-                bool ok = true;
-                if (lane == 0) ok = tc::mbar_wait(&kv_empty[s], ((j / STAGES) - 1) & 1, abort_flag);
-                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-                if (!ok) break;
-            }
-            const int kb = kb_first + j * BKV;
-            uint8_t* k_dst = sKV + s * STAGE_BYTES;
-            uint8_t* v_dst = k_dst + TILE_BYTES;
-            if (p.new_rows && kb >= pos0) {
-                // Every key of this block is one of this step's own: they lie row after row beside the queries, so one
-                // box of 128 rows brings the keys and one the values (a box per cache page costs the TMA unit about
-                // 60 ns each, 1 us per block with pages of 16 tokens, which is what bounded whole prompts). Rows past
-                // the entry are other requests' tokens or zeros: masked by position like any key after the query.
-                if (lane == 0) {
-                    const int row = (row0 - q0) + kb - pos0;       // the entry's first row + (key - its first position)
-                    tc::mbar_expect_tx(&kv_full[s], STAGE_BYTES);
-                    tc::tma_load_2d(k_dst, &map_k_new, kh * D, row, &kv_full[s]);
-                    tc::tma_load_2d(v_dst, &map_v_new, kh * D, row, &kv_full[s]);
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+        if (((warp - 4) >> 2) < n_tiles) {
+            // ---- softmax and output: four warps per tile, a thread owns one query row (its TMEM lane) ----
+            const int t = (warp - 4) >> 2, quarter = warp & 3;
+            const int r = quarter * 32 + lane;
+            const int t_first = tile_first(t), rows = tile_last(t) - t_first + 1;
+            const int qpos = t_first + r;
+            const int qlo = first_seen(qpos);
+            const int j_first = block_first(t), j_last = block_last(t);
+            const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+            // m: the maximum the row's exponentials, sum and output are relative to. It follows the true running maximum only
+            // when that has moved ahead by more than 8 (a factor of 256, harmless in float32 and bfloat16): only then is the
+            // output row in TMEM rescaled, which is rare after the first blocks. l: the row's sum.
+            float m = -CUDART_INF_F, l = 0.f;
+            bool alive = true;
+            for (int j = j_first, c = 0; j <= j_last && alive; ++j, ++c) {
+                const int kb = kb_first + j * BKV;
+                alive = __all_sync(0xffffffffu, tc::mbar_wait(&s_full[t], c & 1, abort_flag));
+                if (!alive) break;
+                tc::fence_after_sync();
+                // the row's 128 scores of the block into registers: four loads in flight, one wait; then the columns are free
+                uint32_t sv[BKV];
+#pragma unroll
+                for (int c0 = 0; c0 < BKV; c0 += 32) tc::tmem_ld_x32(lane_addr + s_col(t) + c0, sv + c0);
+                tc::tmem_ld_wait();
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&s_free[t]);
+                if (kb + BKV - 1 > qpos || kb < qlo) {
+#pragma unroll
+                    for (int i = 0; i < BKV; ++i)
+                        if (kb + i > qpos || kb + i < qlo) sv[i] = 0xff800000u;      // -inf: replaced, whatever was there
                 }
-                continue;
-            }
-            const int first_entry = kb / p.P;
-            if (first_entry / 32 != window_at) {
-                window_at = first_entry / 32;
-                held = ahead;
-                ahead = table_window(window_at + 1);
-            }
-            // lanes 0 .. pages-1 fetch the key boxes of the block's pages, the next `pages` lanes the value boxes
-            const int slot = lane < pages_per_block ? lane : lane - pages_per_block;
-            const bool values = lane >= pages_per_block;
-            const int page = __shfl_sync(0xffffffffu, held, (first_entry + slot) & 31);
-            bool valid = false;
-            if (lane < 2 * pages_per_block) {
-                const int key0 = kb + slot * p.P;
-                valid = key0 <= pos_last && key0 + p.P > kv_lo;
-                if (valid && (page < 0 || page >= p.n_pages)) {
-                    atomicOr(p.error_flag, 4);
-                    valid = false;
-                }
-            }
-            const int n_valid = __popc(__ballot_sync(0xffffffffu, valid));          // boxes, keys and values counted apart
-            if (lane < 2 * pages_per_block) {
-                if (valid) {
-                    const int row = ((page * 2 + (values ? 1 : 0)) * p.KH + kh) * p.P;
-                    tc::tma_load_2d((values ? v_dst : k_dst) + slot * page_bytes, &map_kv, 0, row, &kv_full[s]);
-                } else if (values) {
-                    // no live key in this page: its scores are all masked; its value rows must be zeros
-                    uint4* z = reinterpret_cast<uint4*>(v_dst + slot * page_bytes);
-                    for (uint32_t i = 0; i < page_bytes / 16; ++i) z[i] = make_uint4(0, 0, 0, 0);
-                    tc::fence_proxy_async();
-                }
-            }
-            __syncwarp();
-            if (lane == 0) tc::mbar_expect_tx(&kv_full[s], (uint32_t)n_valid * page_bytes);
-        }
-        if (p.store_new && h % (p.H / p.KH) == 0) {
-            // The pair's own keys and values are its last key blocks (one per tile), and they lie in shared memory in
-            // the layout of the cache's tensor map: TMA writes them into their pages, one box per page, while the block
-            // works on them. No block of this launch reads these cache rows: with every entry starting on a key-block
-            // boundary, the key blocks that hold this step's tokens are read from k_new/v_new. A page that the entry
-            // fills only in part receives whatever follows the entry's last token in its other slots; slots past a
-            // request's length are never read by anyone.
-            if (pos0 % BKV != 0) {
-                if (lane == 0) atomicOr(p.error_flag, 2);        // the caller broke the rule: nothing is written
-            } else {
-                for (int j = n_blocks - n_tiles; j < n_blocks; ++j) {
-                    const int s = j % STAGES, kb = kb_first + j * BKV;
-                    if (!tc::mbar_wait(&kv_full[s], (j / STAGES) & 1, abort_flag)) break;
-                    if (lane < 2 * pages_per_block) {
-                        const int slot = lane < pages_per_block ? lane : lane - pages_per_block;
-                        const bool values = lane >= pages_per_block;
-                        const int key0 = kb + slot * p.P;
-                        if (key0 <= pos_last) {
-                            const int page = bt[key0 / p.P];
-                            if (page < 0 || page >= p.n_pages) atomicOr(p.error_flag, 2);
-                            else
-                                tc::tma_store_2d(&map_kv, 0, ((page * 2 + (values ? 1 : 0)) * p.KH + kh) * p.P,
-                                                 sKV + s * STAGE_BYTES + (values ? TILE_BYTES : 0) + slot * page_bytes);
+                float mx4[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+#pragma unroll
+                for (int i = 0; i < BKV; i += 2)
+                    mx4[(i >> 1) & 3] = max_of_three(mx4[(i >> 1) & 3], __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]));
+                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+                const float m_true = fmaxf(m, mx * p.scale_log2e);     // the scale is positive
+                const bool move = m_true > m + 8.f || (m == -CUDART_INF_F && m_true != -CUDART_INF_F);
+                const float alpha = move ? exp2_approx(m - m_true) : 1.f;      // 0 from -inf
+                if (move) m = m_true;
+                const float msub = m == -CUDART_INF_F ? 0.f : m;
+                if (c > 0) {
+                    // P of the block before has been read and its product added to the output: P may be overwritten, the
+                    // output rescaled
+                    alive = __all_sync(0xffffffffu, tc::mbar_wait(&o_full[t], (c - 1) & 1, abort_flag));
+                    if (!alive) break;
+                    tc::fence_after_sync();
+                    if (__any_sync(0xffffffffu, move)) {
+#pragma unroll
+                        for (int d0 = 0; d0 < D; d0 += 16) {          // in small pieces: the scores fill the registers
+                            uint32_t v[16];
+                            tc::tmem_ld_x16(lane_addr + o_col(t) + d0, v);
+                            tc::tmem_ld_wait();
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+                            tc::tmem_st_x16(lane_addr + o_col(t) + d0, v);
                         }
                     }
                 }
-                tc::bulk_commit();
-                tc::bulk_wait_all();         // shared memory has been read and the cache written before the block leaves
-            }
-        }
-    } else if (warp == 1) {
-        // ---- MMA ----
-        if (tc::elect_one()) {
-            constexpr uint32_t idesc_s = tc::idesc_bf16_f32(BQ, BKV);
-            constexpr uint32_t idesc_o = tc::idesc_bf16_f32_b_mn(BQ, D);
-            const uint32_t q_addr = tc::smem_u32(sQ);
-            int first[TILES], last[TILES], scored[TILES], added[TILES];
+                // exponentials (a masked score gives exactly 0), their sum, and P as bfloat16 into tensor memory: two
+                // consecutive keys per column
+                const unsigned long long scale2 = pair_of(__float_as_uint(p.scale_log2e), __float_as_uint(p.scale_log2e));
+                const unsigned long long shift2 = pair_of(__float_as_uint(-msub), __float_as_uint(-msub));
+                unsigned long long sums[4] = {0ull, 0ull, 0ull, 0ull};           // pairs of float32 zeros
 #pragma unroll
-            for (int t = 0; t < TILES; ++t) {
-                first[t] = block_first(t);
-                last[t] = t < n_tiles ? block_last(t) : -1;
-                scored[t] = added[t] = 0;
-            }
-            bool ok = tc::mbar_wait(q_full, 0, abort_flag);
-            tc::fence_after_sync();
-            // S_t = Q_t K_j^T for the tiles that take part in key block j, as soon as a tile's softmax warps have taken
-            // its previous scores into registers
-            auto issue_scores = [&](int j) {
-                const int s = j % STAGES;
-                if (!tc::mbar_wait(&kv_full[s], (j / STAGES) & 1, abort_flag)) { ok = false; return; }
-                const uint32_t k_addr = tc::smem_u32(sKV + s * STAGE_BYTES);
+                for (int c0 = 0; c0 < BKV; c0 += 32) {
+                    uint32_t packed[16];
 #pragma unroll
-                for (int t = 0; t < TILES; ++t) {
-                    if (j < first[t] || j > last[t]) continue;
-                    if (scored[t] > 0 && !tc::mbar_wait(&s_free[t], (scored[t] - 1) & 1, abort_flag)) { ok = false; return; }
-                    tc::fence_after_sync();
-#pragma unroll
-                    for (int k = 0; k < D / 16; ++k)
-                        tc::mma_bf16(tmem_base + s_col(t), tc::smem_desc_sw128(q_addr + t * TILE_BYTES + k * 32),
-                                     tc::smem_desc_sw128(k_addr + k * 32), idesc_s, k > 0 ? 1u : 0u);
-                    tc::mma_commit(&s_full[t]);
-                    ++scored[t];
-                }
-            };
-            if (ok) issue_scores(0);
-            for (int j = 0; j < n_blocks && ok; ++j) {
-                if (j + 1 < n_blocks) issue_scores(j + 1);
-                if (!ok) break;
-                // O_t += P_t V_j, for each tile as soon as its P is there, whichever comes first
-                const int s = j % STAGES;
-                const uint32_t v_addr = tc::smem_u32(sKV + s * STAGE_BYTES + TILE_BYTES);
-                uint32_t pending = 0;
-#pragma unroll
-                for (int t = 0; t < TILES; ++t)
-                    if (j >= first[t] && j <= last[t]) pending |= 1u << t;
-                const unsigned long long start = tc::global_ns();
-                uint32_t spins = 0;
-                while (pending && ok) {
-#pragma unroll
-                    for (int t = 0; t < TILES; ++t) {
-                        if (!(pending & (1u << t)) || !tc::mbar_try_wait(&p_ready[t], added[t] & 1)) continue;
-                        tc::fence_after_sync();
-#pragma unroll
-                        for (int k = 0; k < BKV / 16; ++k)
-                            tc::mma_bf16_a_tmem(tmem_base + o_col(t), tmem_base + p_col(t) + k * 8,
-                                                tc::smem_desc_sw128_mn(v_addr + k * 16 * D * 2, 1024), idesc_o,
-                                                (added[t] > 0 || k > 0) ? 1u : 0u);
-                        tc::mma_commit(&o_full[t]);
-                        ++added[t];
-                        pending &= ~(1u << t);
+                    for (int i = 0; i < 16; ++i) {
+                        float x0, x1;
+                        halves_of(fma_pair(pair_of(sv[c0 + 2 * i], sv[c0 + 2 * i + 1]), scale2, shift2), x0, x1);
+                        const float p0 = exp2_approx(x0), p1 = exp2_approx(x1);
+                        sums[i & 3] = add_pair(sums[i & 3], pair_of(__float_as_uint(p0), __float_as_uint(p1)));
+                        packed[i] = pack_bf16(p0, p1);
                     }
-                    if (pending && (++spins & 0x3ff) == 0 && (*abort_flag || tc::global_ns() - start > tc::WAIT_LIMIT_NS)) {
-                        *abort_flag = 1;
-                        ok = false;
+                    tc::tmem_st_x16(lane_addr + p_col(t) + c0 / 2, packed);
+                }
+                float sum4[4];
+                {
+                    float lo, hi;
+                    halves_of(add_pair(add_pair(sums[0], sums[1]), add_pair(sums[2], sums[3])), lo, hi);
+                    sum4[0] = lo; sum4[1] = hi; sum4[2] = 0.f; sum4[3] = 0.f;
+                }
+                l = l * alpha + (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+                if (kb + BKV - 1 > pos_last) {
+                    // value rows of keys past the pair's last query: unwritten cache slots, to be zeros under P = 0 (where
+                    // both tiles take part in such a block both write these zeros)
+                    const int s = j % STAGES;
+                    alive = __all_sync(0xffffffffu, tc::mbar_wait(&kv_full[s], (j / STAGES) & 1, abort_flag));
+                    if (!alive) break;
+                    if (kb + r > pos_last) {
+                        uint4* z = reinterpret_cast<uint4*>(sKV + s * STAGE_BYTES + TILE_BYTES + r * 128);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) z[i] = make_uint4(0, 0, 0, 0);
                     }
                 }
-                if (ok) tc::mma_commit(&kv_empty[s]);            // keys and values of this block have been read
+                tc::tmem_st_wait();               // P is in tensor memory
+                tc::fence_proxy_async();          // the zeroed value rows to the proxy the MMA reads through
+                tc::fence_before_sync();          // this thread's TMEM reads and writes are done
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&p_ready[t]);
             }
-        }
-    } else if (((warp - 2) >> 2) < n_tiles) {
-        // ---- softmax and output: four warps per tile, a thread owns one query row (its TMEM lane) ----
-        const int t = (warp - 2) >> 2, quarter = warp & 3;
-        const int r = quarter * 32 + lane;
-        const int t_first = tile_first(t), rows = tile_last(t) - t_first + 1;
-        const int qpos = t_first + r;
-        const int qlo = first_seen(qpos);
-        const int j_first = block_first(t), j_last = block_last(t);
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
-        // m: the maximum the row's exponentials, sum and output are relative to. It follows the true running maximum only
-        // when that has moved ahead by more than 8 (a factor of 256, harmless in float32 and bfloat16): only then is the
-        // output row in TMEM rescaled, which is rare after the first blocks. l: the row's sum.
-        float m = -CUDART_INF_F, l = 0.f;
-        bool alive = true;
-        for (int j = j_first, c = 0; j <= j_last && alive; ++j, ++c) {
-            const int kb = kb_first + j * BKV;
-            alive = __all_sync(0xffffffffu, tc::mbar_wait(&s_full[t], c & 1, abort_flag));
-            if (!alive) break;
-            tc::fence_after_sync();
-            // the row's 128 scores of the block into registers: four loads in flight, one wait; then the columns are free
-            uint32_t sv[BKV];
-#pragma unroll
-            for (int c0 = 0; c0 < BKV; c0 += 32) tc::tmem_ld_x32(lane_addr + s_col(t) + c0, sv + c0);
-            tc::tmem_ld_wait();
-            tc::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&s_free[t]);
-            if (kb + BKV - 1 > qpos || kb < qlo) {
-#pragma unroll
-                for (int i = 0; i < BKV; ++i)
-                    if (kb + i > qpos || kb + i < qlo) sv[i] = 0xff800000u;      // -inf: replaced, whatever was there
-            }
-            float mx4[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-#pragma unroll
-            for (int i = 0; i < BKV; i += 2)
-                mx4[(i >> 1) & 3] = max_of_three(mx4[(i >> 1) & 3], __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]));
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            const float m_true = fmaxf(m, mx * p.scale_log2e);     // the scale is positive
-            const bool move = m_true > m + 8.f || (m == -CUDART_INF_F && m_true != -CUDART_INF_F);
-            const float alpha = move ? exp2_approx(m - m_true) : 1.f;      // 0 from -inf
-            if (move) m = m_true;
-            const float msub = m == -CUDART_INF_F ? 0.f : m;
-            if (c > 0) {
-                // P of the block before has been read and its product added to the output: P may be overwritten, the
-                // output rescaled
-                alive = __all_sync(0xffffffffu, tc::mbar_wait(&o_full[t], (c - 1) & 1, abort_flag));
-                if (!alive) break;
+            // the output row after the last block's P.V
+            if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(&o_full[t], (j_last - j_first) & 1, abort_flag));
+            if (alive) {
                 tc::fence_after_sync();
-                if (__any_sync(0xffffffffu, move)) {
+                // (the running maximum m is in units of log2; a query always sees its own key, so m is finite here)
+                if (p.sink) l += exp2f(p.sink[h] * 1.4426950408889634f - m);
+                float inv = l > 0.f ? 1.f / l : 0.f;
+                if (p.gate && r < rows)
+                    inv *= 1.0f / (1.0f + __expf(-__bfloat162float(p.gate[(size_t)(row0 + t * BQ + r) * p.gate_stride + h])));
+                __nv_bfloat16* dst = p.out + (size_t)(row0 + t * BQ + r) * p.out_stride + (size_t)h * D;
 #pragma unroll
-                    for (int d0 = 0; d0 < D; d0 += 16) {          // in small pieces: the scores fill the registers
-                        uint32_t v[16];
-                        tc::tmem_ld_x16(lane_addr + o_col(t) + d0, v);
-                        tc::tmem_ld_wait();
+                for (int d0 = 0; d0 < D; d0 += 32) {
+                    uint32_t v[32];
+                    tc::tmem_ld_x32(lane_addr + o_col(t) + d0, v);
+                    tc::tmem_ld_wait();
+                    if (r < rows) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-                        tc::tmem_st_x16(lane_addr + o_col(t) + d0, v);
-                    }
-                }
-            }
-            // exponentials (a masked score gives exactly 0), their sum, and P as bfloat16 into tensor memory: two
-            // consecutive keys per column
-            const unsigned long long scale2 = pair_of(__float_as_uint(p.scale_log2e), __float_as_uint(p.scale_log2e));
-            const unsigned long long shift2 = pair_of(__float_as_uint(-msub), __float_as_uint(-msub));
-            unsigned long long sums[4] = {0ull, 0ull, 0ull, 0ull};           // pairs of float32 zeros
+                        for (int c = 0; c < 32; c += 8) {
+                            float f[8];
 #pragma unroll
-            for (int c0 = 0; c0 < BKV; c0 += 32) {
-                uint32_t packed[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    float x0, x1;
-                    halves_of(fma_pair(pair_of(sv[c0 + 2 * i], sv[c0 + 2 * i + 1]), scale2, shift2), x0, x1);
-                    const float p0 = exp2_approx(x0), p1 = exp2_approx(x1);
-                    sums[i & 3] = add_pair(sums[i & 3], pair_of(__float_as_uint(p0), __float_as_uint(p1)));
-                    packed[i] = pack_bf16(p0, p1);
-                }
-                tc::tmem_st_x16(lane_addr + p_col(t) + c0 / 2, packed);
-            }
-            float sum4[4];
-            {
-                float lo, hi;
-                halves_of(add_pair(add_pair(sums[0], sums[1]), add_pair(sums[2], sums[3])), lo, hi);
-                sum4[0] = lo; sum4[1] = hi; sum4[2] = 0.f; sum4[3] = 0.f;
-            }
-            l = l * alpha + (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-            if (kb + BKV - 1 > pos_last) {
-                // value rows of keys past the pair's last query: unwritten cache slots, to be zeros under P = 0 (where
-                // both tiles take part in such a block both write these zeros)
-                const int s = j % STAGES;
-                alive = __all_sync(0xffffffffu, tc::mbar_wait(&kv_full[s], (j / STAGES) & 1, abort_flag));
-                if (!alive) break;
-                if (kb + r > pos_last) {
-                    uint4* z = reinterpret_cast<uint4*>(sKV + s * STAGE_BYTES + TILE_BYTES + r * 128);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) z[i] = make_uint4(0, 0, 0, 0);
-                }
-            }
-            tc::tmem_st_wait();               // P is in tensor memory
-            tc::fence_proxy_async();          // the zeroed value rows to the proxy the MMA reads through
-            tc::fence_before_sync();          // this thread's TMEM reads and writes are done
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&p_ready[t]);
-        }
-        // the output row after the last block's P.V
-        if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(&o_full[t], (j_last - j_first) & 1, abort_flag));
-        if (alive) {
-            tc::fence_after_sync();
-            // (the running maximum m is in units of log2; a query always sees its own key, so m is finite here)
-            if (p.sink) l += exp2f(p.sink[h] * 1.4426950408889634f - m);
-            float inv = l > 0.f ? 1.f / l : 0.f;
-            if (p.gate && r < rows)
-                inv *= 1.0f / (1.0f + __expf(-__bfloat162float(p.gate[(size_t)(row0 + t * BQ + r) * p.gate_stride + h])));
-            __nv_bfloat16* dst = p.out + (size_t)(row0 + t * BQ + r) * p.out_stride + (size_t)h * D;
-#pragma unroll
-            for (int d0 = 0; d0 < D; d0 += 32) {
-                uint32_t v[32];
-                tc::tmem_ld_x32(lane_addr + o_col(t) + d0, v);
-                tc::tmem_ld_wait();
-                if (r < rows) {
-#pragma unroll
-                    for (int c = 0; c < 32; c += 8) {
-                        float f[8];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[c + i]) * inv;
-                        *reinterpret_cast<uint4*>(dst + d0 + c) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]),
-                                                                               pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+                            for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[c + i]) * inv;
+                            *reinterpret_cast<uint4*>(dst + d0 + c) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]),
+                                                                                   pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+                        }
                     }
                 }
             }
