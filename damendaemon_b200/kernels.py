@@ -64,6 +64,7 @@ _SIGNATURES = {
         "dd_retention_finish": [_c_void, _c_void, _c_int, _c_void, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_void, _c_void],
         "dd_gemm_simt": [_c_void, _c_int, _c_void, _c_int, _c_void, _c_void, _c_int, _c_void, _c_int] + [_c_int] * 6 + [_c_void],
         "dd_gemm_split_plan": [_c_int] * 4 + [_c_void],
+        "dd_gemm_stream": [_c_void, _c_int, _c_void, _c_int, _c_void, _c_void, _c_int, _c_void, _c_int] + [_c_int] * 5 + [_c_void] * 2,
         "dd_gemm_split": [_c_void, _c_int, _c_void, _c_int, _c_void, _c_void, _c_int, _c_void, _c_int] + [_c_int] * 7 + [_c_void] * 3,
         "dd_kv_store": [_c_void, _c_void, _c_int, _c_void, _c_void, _c_void, _c_int, _c_void] + [_c_int] * 7 + [_c_void, _c_void],
         "dd_attention_rows": [_c_void, _c_int, _c_void, _c_void, _c_void, _c_void, _c_int, _c_void, _c_int, _c_void, _c_void]
@@ -1199,6 +1200,30 @@ def gemm_split(a, w, bias=None, residual=None, activation=None, out=None, token_
           _ptr(out, "out", torch.float32), out.stride(0), M, N, K, ACTIVATIONS[activation],
           token_tile, plan[0] if splits is None else splits, sms, _ptr(planes), _ptr(error_flag(a.device)), _stream(),
           n_kernels=1 if planes is None else 2)
+    return out
+
+
+GEMM_STREAM_ROWS = 8            # most rows of gemm_stream
+GEMM_STREAM_REDUCTION = 8 * 7 * 256       # its longest reduction: eight blocks of a cluster, seven boxes of 256 each
+
+
+def gemm_stream(a, w, bias=None, residual=None, activation=None, out=None):
+    """act(a @ w.T + bias) (+ residual), all float32, for up to eight rows: the weights streamed once through the CUDA cores,
+    the lanes' sums added in float64 (csrc/gemm_stream_f32.cu). a [M,K], w [N,K] as gemm_split takes them, K up to
+    GEMM_STREAM_REDUCTION."""
+    _rows(a, "a"), _rows(w, "w")
+    M, K = a.shape
+    N = w.shape[0]
+    if a.dtype != torch.float32 or w.dtype != torch.float32 or w.shape[1] != K:
+        raise KernelError(f"gemm_stream: needs float32 a [M,K] and w [N,K]; got {tuple(a.shape)} {a.dtype}, {tuple(w.shape)} {w.dtype}")
+    if out is None:
+        out = torch.empty((M, N), dtype=torch.float32, device=a.device)
+    _rows(out, "out")
+    if residual is not None:
+        _rows(residual, "residual")
+    _call(library("core"), "dd_gemm_stream", _ptr(a, "a"), a.stride(0), _ptr(w, "w"), w.stride(0), _ptr(bias, "bias", torch.float32),
+          _ptr(residual, "residual", torch.float32), 0 if residual is None else residual.stride(0), _ptr(out, "out", torch.float32),
+          out.stride(0), M, N, K, ACTIVATIONS[activation], sm_count(a.device), _ptr(error_flag(a.device)), _stream())
     return out
 
 

@@ -18,6 +18,16 @@ def splits_float32(out, reduction):
     return out * reduction >= 1 << 20
 
 
+def streams_float32(rows, out, reduction):
+    """Whether a float32 product that splits_float32 takes streams its matrix through the CUDA cores (kernels.gemm_stream)
+    instead: up to eight rows, and a matrix of 12 to 200 MB (split / stream, us at 8 rows: 3072 x 1024 13.7 / 5.8, 4096 x 1024
+    9.0 / 6.8, 1024 x 4096 11.0 / 8.4, 4800 x 1600 11.9 / 9.3, 6400 x 1600 14.2 / 11.0, 1600 x 6400 14.8 / 14.2, 25600 x 1600
+    41.7 / 34.6; 50257 x 1600 60.6 / 68.3: the stream's warps reach 4.7 TB/s, what their reads of X from shared memory leave
+    them, the split product 5.3). Smaller matrices stay with the split product, which gives a row the same bits among 1 to
+    128. A row of such a product has other bits beside more than seven others than beside fewer, within the error of either."""
+    return rows <= kernels.GEMM_STREAM_ROWS and 3 << 20 <= out * reduction <= 3 << 24 and reduction <= kernels.GEMM_STREAM_REDUCTION
+
+
 def linear(runtime, a, w, bias=None, residual=None, activation=None, out_dtype=None, out=None):
     """act(a @ w.T + bias) (+ residual). float32 engine: the split product on the tensor cores or, for small matrices and
     rows that are not 16-byte aligned, or if the runtime asks for 'simt', the CUDA-core float32 kernel.
@@ -25,6 +35,8 @@ def linear(runtime, a, w, bias=None, residual=None, activation=None, out_dtype=N
     reduction width is no multiple of 8 (then the CUDA-core kernel with bfloat16 operands)."""
     if a.dtype == torch.float32 and runtime.gemm != "simt" and out_dtype in (None, torch.float32) and \
             splits_float32(w.shape[0], a.shape[1]) and kernels.gemm_split_fits(a, w):
+        if streams_float32(a.shape[0], w.shape[0], a.shape[1]):
+            return kernels.gemm_stream(a, w, bias, residual, activation, out)
         return kernels.gemm_split(a, w, bias, residual, activation, out)
     if a.dtype == torch.float32 or runtime.gemm == "simt":
         return kernels.gemm_simt(a, w, bias, residual, activation, out_dtype, out)

@@ -115,6 +115,68 @@ def test_which_float32_products_are_split(K):
     assert torch.equal(linear(auto, one, w), K.gemm_split(a[:1], w))
 
 
+@pytest.mark.parametrize("M,N,Kd", [(1, 1, 4), (8, 7, 132), (3, 1000, 1600), (8, 9000, 256), (5, 6400, 1792), (8, 1600, 1796), (2, 1600, 6400),
+                                    (8, 3001, 14336)])
+def test_streamed_product(K, M, N, Kd):
+    """Up to eight rows through the CUDA cores: the last group of rows smaller, several groups a warp, K that ends inside a box,
+    one to eight blocks on a sum. Within the bound of chains of K / 64 float32 multiply-adds and, over all outputs, no further
+    from 64 bits than the split product, which serves more rows."""
+    for mean in (0.0, 1.0):
+        a, w = operands(M, N, Kd, mean=mean)
+        want, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+        got = K.gemm_stream(a, w)
+        # a lane's pair of sums takes at most two products a sub-box of 128 k; the rest is float64 and one last rounding
+        assert ((got.double() - want).abs() <= size * (2 * (Kd / 128 + 1) + 1) * 2.0 ** -24).all()
+        if M * N >= 1024 and mean == 0.0:
+            assert (got.double() - want).norm() <= (K.gemm_split(a, w).double() - want).norm()
+        assert torch.equal(got, K.gemm_stream(a, w)), "two runs are bit-equal"
+        assert torch.equal(got[:1], K.gemm_stream(a[:1], w)), "a row does not depend on the others"
+    bias, stream = torch.randn(N, device=DEV), torch.randn(M, N, device=DEV)
+    u, allowed = want + bias.double(), size * (2 * (Kd / 128 + 1) + 1) * 2.0 ** -24
+    wide = torch.full((M, N + 8), 7.0, device=DEV)
+    full = K.gemm_stream(a, w, bias, residual=stream, activation="gelu", out=wide[:, 4:4 + N])
+    exact = 0.5 * u * (1 + torch.erf(u / 2 ** 0.5)) + stream.double()
+    assert ((full.double() - exact).abs() <= 2 * allowed + 1e-6 * (1 + u.abs())).all()
+    assert bool((wide[:, :4] == 7).all()) and bool((wide[:, 4 + N:] == 7).all())
+    in_place = stream.clone()
+    assert K.gemm_stream(a, w, bias, residual=in_place, out=in_place).data_ptr() == in_place.data_ptr()
+    assert ((in_place.double() - u - stream.double()).abs() <= allowed + 1e-6 * (1 + u.abs())).all()
+    # operands inside wider rows, whose neighbours are no numbers
+    big_a, big_w = torch.full((M, Kd + 8), float("nan"), device=DEV), torch.full((N, Kd + 8), float("nan"), device=DEV)
+    big_a[:, 4:4 + Kd], big_w[:, 4:4 + Kd] = a, w
+    assert torch.equal(K.gemm_stream(big_a[:, 4:4 + Kd], big_w[:, 4:4 + Kd]), got)
+    assert K.read_error_flag(DEV) == 0
+
+
+def test_streamed_product_of_values_that_are_not_finite(K):
+    a, w = operands(5, 200, 160, seed=5)
+    a[1, 7], a[2, 9], a[3, 30], a[4, 31] = float("inf"), float("nan"), 3.4e38, -float("inf")
+    w[5, 11], w[6, 12], w[130, 40] = float("inf"), -3.395e38, float("nan")
+    got, plain = K.gemm_stream(a, w), K.gemm_simt(a, w)
+    finite = torch.isfinite(plain)
+    assert torch.equal(torch.isnan(plain), torch.isnan(got)) and torch.equal(finite, torch.isfinite(got))
+    assert ((got - plain)[finite].abs() <= 1e-4 * (1 + plain[finite].abs())).all()
+
+
+def test_which_float32_products_are_streamed(K):
+    from types import SimpleNamespace
+    from damendaemon_b200.parts.linear import linear, streams_float32
+    assert streams_float32(8, 3072, 1024) and not streams_float32(9, 3072, 1024) and \
+        not streams_float32(1, 1600, 1600) and not streams_float32(8, 50257, 1600)
+    auto, plain = SimpleNamespace(gemm="auto"), SimpleNamespace(gemm="simt")
+    a, w = operands(9, 3072, 1024)
+    assert torch.equal(linear(auto, a[:8], w), K.gemm_stream(a[:8], w)) and torch.equal(linear(auto, a, w), K.gemm_split(a, w))
+    assert torch.equal(linear(plain, a[:8], w), K.gemm_simt(a[:8], w))
+    one = a.as_strided((1, 1024), (0, 1))
+    assert torch.equal(linear(auto, one, w), K.gemm_stream(a[:1], w))
+    for rows in (a[:1].expand(8, 1024), torch.randn(8, 1025, device=DEV)[:, 1:]):
+        assert torch.equal(linear(auto, rows, w), K.gemm_simt(rows.contiguous() if rows.stride(0) == 0 else rows, w))
+    with pytest.raises(K.KernelError, match="takes up to 8 rows"):
+        K.gemm_stream(a, w)
+    with pytest.raises(K.KernelError, match="over one another"):
+        K.gemm_stream(a[:1].expand(8, 1024), w)
+
+
 def run_of_entries(dtype, entries, keys, heads, kv_heads, d, page=16, seed=11):
     """Queries of `entries` requests with `keys` tokens each, their caches and block tables: q [entries * keys, ...] is what a
     prompt of whole requests brings, its last row of every entry what a decode step brings."""
