@@ -35,13 +35,20 @@ template <int BN> struct SplitConfig {
     static constexpr bool X_SPLIT = BN >= 64;                            // the tokens' planes come from global memory
     static constexpr int EPI_WARPS = BN >= 128 ? 8 : 4;                  // two per lane quarter for the widest tile
     static constexpr int EPI_COLS = BN * 4 / EPI_WARPS;                  // columns an epilogue thread owns
-    static constexpr int CONV_GROUPS = BN >= 128 ? 1 : 2;                // of four warps, k blocks taken in turn
+    static constexpr int CONV_GROUPS = 2;                                // of four warps, k blocks taken in turn
     static constexpr int X_WARPS = X_SPLIT ? 1 : 4;                      // one thread that fetches planes, or warps that split, k blocks taken in turn
-    static constexpr int FIRST_CONV = 2 + EPI_WARPS, FIRST_X = FIRST_CONV + 4 * CONV_GROUPS;
-    static constexpr int THREADS = 32 * (FIRST_X + X_WARPS);             // 16 warps: 128 registers a thread, 18: 96
+    // The widest tile has five whole warpgroups (the fetching warps and one that idles, two of epilogue, two that split), which
+    // share the registers by their needs: 128 x 40 + 256 x 144 + 256 x 72 of the launch's 640 x 96. With 128 for everybody and
+    // the sums live through the other warps' code, the epilogue's loads went one by one: with a residual 1,000 rows of 1,280 x
+    // 5,120 took 127 us, now 107, and 5,120 x 1,280 142, now 107; plain products 103 / 101 and 92 / 93. What bounds those is what an
+    // SM fetches, 40 KB a k block of 0.79 us (51 KB/us, 7.5 TB/s in all): half the MMAs take 2 % off.
+    static constexpr bool GROUPED = BN >= 128;
+    static constexpr int FIRST_EPI = GROUPED ? 4 : 2, FIRST_CONV = FIRST_EPI + EPI_WARPS, LAST_CONV = FIRST_CONV + 4 * CONV_GROUPS;
+    static constexpr int FIRST_X = GROUPED ? 2 : LAST_CONV;
+    static constexpr int THREADS = 32 * (GROUPED ? LAST_CONV : FIRST_X + X_WARPS);        // 18 warps: 96 registers a thread
     static constexpr int STAGING_BYTES = (BM + (X_SPLIT ? 0 : BN)) * BK * 4;
     static constexpr int OPERAND_BYTES = BN * PLANE_ROW * 3;
-    static constexpr int STAGINGS = BN >= 128 ? 5 : (BN >= 64 ? 6 : 8);
+    static constexpr int STAGINGS = BN >= 64 ? 6 : 8;
     static constexpr int OPERANDS = 4;
     static constexpr int ACCS = BN >= 128 ? 2 : 4;
     static constexpr int TMEM_COLS = ACCS * BN + OPERANDS * W_COLS <= 256 ? 256 : 512;
@@ -193,59 +200,90 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_w = tmem_base + C::ACCS * BN;     // the features' planes, behind the accumulators
 
-    float sum[C::EPI_COLS];                               // epilogue warps: this feature's sums
-    if (warp == 0) {
-        if (tc::elect_one()) {
-            tc::prefetch_tensormap(&map_w);
-            if (!C::X_SPLIT) tc::prefetch_tensormap(&map_x);
-            // weights do not depend on the kernel before this one
-            const int ahead = first_tile < n_tiles ? min(n_kblocks, C::STAGINGS) : 0;
-            for (int i = 0; i < ahead; ++i) {
-                tc::mbar_expect_tx(&staged[i], C::STAGING_BYTES);
-                tc::tma_load_2d(staging + i * C::STAGING_BYTES, &map_w, (kb_begin + i) * BK, (first_tile % tiles_n) * BM, &staged[i]);
-            }
-            if (!C::X_SPLIT) dd_grid_wait();
-            int it = 0;
-            bool ok = true;
-            for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
-                const int n0 = (tile % tiles_n) * BM, m0 = (tile / tiles_n) * BN;
-                for (int i = 0; i < n_kblocks; ++i, ++it) {
-                    const int s = it % C::STAGINGS;
-                    uint8_t* to = staging + s * C::STAGING_BYTES;
-                    if (it >= ahead) {
-                        if (!tc::mbar_wait(&staging_free[s], ((it / C::STAGINGS) & 1) ^ 1, abort_flag)) { ok = false; break; }
-                        tc::mbar_expect_tx(&staged[s], C::STAGING_BYTES);
-                        tc::tma_load_2d(to, &map_w, (kb_begin + i) * BK, n0, &staged[s]);
+    // the two barriers at which the blocks of a cluster exchange their sums, for the warps that have none
+    auto stand_by = [&] {
+        if (S == 1) return;
+        __syncwarp();
+        tc::fence_before_sync();
+        tc::cluster_arrive();
+        tc::cluster_wait();
+        tc::cluster_arrive();
+        tc::cluster_wait();
+    };
+    if (warp < C::FIRST_EPI) {
+        if constexpr (C::GROUPED) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (warp == 0) {
+            if (tc::elect_one()) {
+                tc::prefetch_tensormap(&map_w);
+                if (!C::X_SPLIT) tc::prefetch_tensormap(&map_x);
+                // weights do not depend on the kernel before this one
+                const int ahead = first_tile < n_tiles ? min(n_kblocks, C::STAGINGS) : 0;
+                for (int i = 0; i < ahead; ++i) {
+                    tc::mbar_expect_tx(&staged[i], C::STAGING_BYTES);
+                    tc::tma_load_2d(staging + i * C::STAGING_BYTES, &map_w, (kb_begin + i) * BK, (first_tile % tiles_n) * BM, &staged[i]);
+                }
+                if (!C::X_SPLIT) dd_grid_wait();
+                int it = 0;
+                bool ok = true;
+                for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
+                    const int n0 = (tile % tiles_n) * BM, m0 = (tile / tiles_n) * BN;
+                    for (int i = 0; i < n_kblocks; ++i, ++it) {
+                        const int s = it % C::STAGINGS;
+                        uint8_t* to = staging + s * C::STAGING_BYTES;
+                        if (it >= ahead) {
+                            if (!tc::mbar_wait(&staging_free[s], ((it / C::STAGINGS) & 1) ^ 1, abort_flag)) { ok = false; break; }
+                            tc::mbar_expect_tx(&staged[s], C::STAGING_BYTES);
+                            tc::tma_load_2d(to, &map_w, (kb_begin + i) * BK, n0, &staged[s]);
+                        }
+                        if (!C::X_SPLIT) tc::tma_load_2d(to + BM * BK * 4, &map_x, (kb_begin + i) * BK, m0, &staged[s]);
                     }
-                    if (!C::X_SPLIT) tc::tma_load_2d(to + BM * BK * 4, &map_x, (kb_begin + i) * BK, m0, &staged[s]);
+                }
+            }
+        } else if (warp == 1) {
+            if (tc::elect_one()) {
+                constexpr uint32_t idesc = tc::idesc_bf16_f32(BM, BN);
+                // plane of W, plane of X: the products in ascending order of size
+                constexpr int pw[6] = {2, 0, 1, 1, 0, 0}, px[6] = {0, 2, 1, 0, 1, 0};
+                for (int it = 0; it < n_its; ++it) {
+                    const int acc = it % C::ACCS, s = it % C::OPERANDS;
+                    if (!tc::mbar_wait(&acc_free[acc], ((it / C::ACCS) & 1) ^ 1, abort_flag) ||
+                        !tc::mbar_wait(&split_done[s], (it / C::OPERANDS) & 1, abort_flag)) break;
+                    tc::fence_after_sync();
+                    const uint32_t w_cols = tmem_w + s * W_COLS;
+                    const uint32_t x_addr = tc::smem_u32(operands + s * C::OPERAND_BYTES);
+#pragma unroll
+                    for (int j = 0; j < 6; ++j)
+#pragma unroll
+                        for (int k = 0; k < BK / 16; ++k)
+                            tc::mma_bf16_a_tmem(tmem_base + acc * BN, w_cols + pw[j] * (BK / 2) + k * 8,
+                                                smem_desc_sw64(x_addr + px[j] * BN * PLANE_ROW + k * 32), idesc, (j > 0 || k > 0) ? 1u : 0u);
+                    tc::mma_commit(&mma_done[s]);
+                }
+            }
+        } else if (C::GROUPED && warp == C::FIRST_X) {
+            if (tc::elect_one()) {
+                // a k block's three planes of BN tokens lie in memory as they lie in shared memory, one piece
+                dd_grid_wait();
+                int it = 0;
+                bool ok = true;
+                for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
+                    const uint8_t* from = p.planes + ((size_t)(tile / tiles_n) * total_kblocks + kb_begin) * C::OPERAND_BYTES;
+                    for (int i = 0; i < n_kblocks; ++i, ++it, from += C::OPERAND_BYTES) {
+                        const int s = it % C::OPERANDS;
+                        if (!tc::mbar_wait(&mma_done[s], ((it / C::OPERANDS) & 1) ^ 1, abort_flag)) { ok = false; break; }
+                        tc::mbar_expect_tx(&split_done[s], C::OPERAND_BYTES);
+                        bulk_load(operands + s * C::OPERAND_BYTES, from, C::OPERAND_BYTES, &split_done[s]);
+                    }
                 }
             }
         }
-    } else if (warp == 1) {
-        if (tc::elect_one()) {
-            constexpr uint32_t idesc = tc::idesc_bf16_f32(BM, BN);
-            // plane of W, plane of X: the products in ascending order of size
-            constexpr int pw[6] = {2, 0, 1, 1, 0, 0}, px[6] = {0, 2, 1, 0, 1, 0};
-            for (int it = 0; it < n_its; ++it) {
-                const int acc = it % C::ACCS, s = it % C::OPERANDS;
-                if (!tc::mbar_wait(&acc_free[acc], ((it / C::ACCS) & 1) ^ 1, abort_flag) ||
-                    !tc::mbar_wait(&split_done[s], (it / C::OPERANDS) & 1, abort_flag)) break;
-                tc::fence_after_sync();
-                const uint32_t w_cols = tmem_w + s * W_COLS;
-                const uint32_t x_addr = tc::smem_u32(operands + s * C::OPERAND_BYTES);
-#pragma unroll
-                for (int j = 0; j < 6; ++j)
-#pragma unroll
-                    for (int k = 0; k < BK / 16; ++k)
-                        tc::mma_bf16_a_tmem(tmem_base + acc * BN, w_cols + pw[j] * (BK / 2) + k * 8,
-                                            smem_desc_sw64(x_addr + px[j] * BN * PLANE_ROW + k * 32), idesc, (j > 0 || k > 0) ? 1u : 0u);
-                tc::mma_commit(&mma_done[s]);
-            }
-        }
+        stand_by();
     } else if (warp < C::FIRST_CONV) {
+        if constexpr (C::GROUPED) asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+        float sum[C::EPI_COLS];                           // this feature's sums
         dd_grid_wait();                                   // the residual is an earlier kernel's data
         const int quarter = warp & 3;
-        const int c_begin = warp >= 6 ? C::EPI_COLS : 0;
+        const int c_begin = warp >= C::FIRST_EPI + 4 ? C::EPI_COLS : 0;
         const uint32_t lane_addr = tmem_base + c_begin + ((uint32_t)(quarter * 32) << 16);
         int it = 0;
         bool ok = true;
@@ -284,7 +322,52 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
             __syncwarp();
         }
-    } else if (warp < C::FIRST_X) {
+        if (S > 1) {
+            // The blocks of the cluster add their partial tiles: block r owns every S-th slice of the 128 features and gets
+            // the others' rows of BN tokens into its shared memory. The rings are free once every block is through its k blocks.
+            const int slice = (BM + S - 1) / S;
+            float* reduce_buf = reinterpret_cast<float*>(staging);
+            __syncwarp();
+            tc::fence_before_sync();
+            tc::cluster_arrive();
+            tc::cluster_wait();
+            const int tile = first_tile, n0 = (tile % tiles_n) * BM, m0 = (tile / tiles_n) * BN;
+            const int epi = (int)threadIdx.x - 32 * C::FIRST_EPI;                // 0 .. 32 * EPI_WARPS - 1
+            {
+                const int f = quarter * 32 + lane;
+                const int owner = f / slice, lf = f - owner * slice;
+                const uint32_t remote = tc::map_to_rank(reduce_buf + ((size_t)rank * slice + lf) * BN, (uint32_t)owner);
+                const int sw = split_swizzle<BN>(lf);
+#pragma unroll
+                for (int q = 0; q < C::EPI_COLS / 4; ++q)
+                    if (m0 + c_begin + 4 * q < p.M)
+                        tc::st_cluster_f32x4(remote + (uint32_t)(((c_begin / 4 + q) ^ sw) * 16), __float_as_uint(sum[4 * q]),
+                                             __float_as_uint(sum[4 * q + 1]), __float_as_uint(sum[4 * q + 2]), __float_as_uint(sum[4 * q + 3]));
+            }
+            tc::cluster_arrive();
+            tc::cluster_wait();
+            {
+                const int first_feature = rank * slice;
+                const int my_features = max(0, min(slice, BM - first_feature));
+                const int items = my_features * min(BN / 4, (p.M - m0 + 3) / 4);
+                for (int item = epi; item < items; item += 32 * C::EPI_WARPS) {
+                    const int lf = item % my_features, c = item / my_features;
+                    const int n = n0 + first_feature + lf, m = m0 + 4 * c;
+                    const float bias = (p.bias && n < p.N) ? __ldg(p.bias + n) : 0.f;
+                    const float* mine = reduce_buf + (size_t)lf * BN + 4 * (c ^ split_swizzle<BN>(lf));
+                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int r = 0; r < S; ++r) {
+                        const float4 a = *reinterpret_cast<const float4*>(mine + (size_t)r * slice * BN);
+                        v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
+                    }
+                    if (n >= p.N) continue;
+                    const float u[4] = {v.x, v.y, v.z, v.w};
+                    finish<4>(p, m, n, u, bias);
+                }
+            }
+        }
+    } else if (warp < C::LAST_CONV) {
+        if constexpr (C::GROUPED) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
         // A thread splits the 32 k of one feature; the swizzle puts the pieces that neighbouring lanes read side by side
         // into different banks.
         const int quarter = warp & 3, row = quarter * 32 + lane, group = (warp - C::FIRST_CONV) >> 2;
@@ -315,6 +398,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&split_done[os]);
         }
+        stand_by();
     } else if (C::X_SPLIT) {
         if (tc::elect_one()) {
             // a k block's three planes of BN tokens lie in memory as they lie in shared memory, one piece
@@ -331,6 +415,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 }
             }
         }
+        stand_by();
     } else {
         // Eight values of a token's row at a time: 32 bytes of staging, 16 bytes of each plane.
         for (int it = warp - C::FIRST_X; it < n_its; it += C::X_WARPS) {
@@ -362,51 +447,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 tc::mbar_arrive(&staging_free[ss]);
             }
         }
-    }
-
-    if (S > 1) {
-        // The blocks of the cluster add their partial tiles: block r owns every S-th slice of the 128 features and gets
-        // the others' rows of BN tokens into its shared memory. The rings are free once every block is through its k blocks.
-        const int slice = (BM + S - 1) / S;
-        float* reduce_buf = reinterpret_cast<float*>(staging);
-        __syncwarp();
-        tc::fence_before_sync();
-        tc::cluster_arrive();
-        tc::cluster_wait();
-        const int tile = first_tile, n0 = (tile % tiles_n) * BM, m0 = (tile / tiles_n) * BN;
-        const int epi = (int)threadIdx.x - 64;            // 0 .. 32 * EPI_WARPS - 1 in the epilogue warps
-        if (epi >= 0 && epi < 32 * C::EPI_WARPS) {
-            const int f = (warp & 3) * 32 + lane, c_begin = warp >= 6 ? C::EPI_COLS : 0;
-            const int owner = f / slice, lf = f - owner * slice;
-            const uint32_t remote = tc::map_to_rank(reduce_buf + ((size_t)rank * slice + lf) * BN, (uint32_t)owner);
-            const int sw = split_swizzle<BN>(lf);
-#pragma unroll
-            for (int q = 0; q < C::EPI_COLS / 4; ++q)
-                if (m0 + c_begin + 4 * q < p.M)
-                    tc::st_cluster_f32x4(remote + (uint32_t)(((c_begin / 4 + q) ^ sw) * 16), __float_as_uint(sum[4 * q]),
-                                         __float_as_uint(sum[4 * q + 1]), __float_as_uint(sum[4 * q + 2]), __float_as_uint(sum[4 * q + 3]));
-        }
-        tc::cluster_arrive();
-        tc::cluster_wait();
-        if (epi >= 0 && epi < 32 * C::EPI_WARPS) {
-            const int first_feature = rank * slice;
-            const int my_features = max(0, min(slice, BM - first_feature));
-            const int items = my_features * min(BN / 4, (p.M - m0 + 3) / 4);
-            for (int item = epi; item < items; item += 32 * C::EPI_WARPS) {
-                const int lf = item % my_features, c = item / my_features;
-                const int n = n0 + first_feature + lf, m = m0 + 4 * c;
-                const float bias = (p.bias && n < p.N) ? __ldg(p.bias + n) : 0.f;
-                const float* mine = reduce_buf + (size_t)lf * BN + 4 * (c ^ split_swizzle<BN>(lf));
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int r = 0; r < S; ++r) {
-                    const float4 a = *reinterpret_cast<const float4*>(mine + (size_t)r * slice * BN);
-                    v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
-                }
-                if (n >= p.N) continue;
-                const float u[4] = {v.x, v.y, v.z, v.w};
-                finish<4>(p, m, n, u, bias);
-            }
-        }
+        stand_by();
     }
     __syncwarp();
     tc::fence_before_sync();
