@@ -16,6 +16,9 @@
 // from there instead of the cache and written to the cache page by the one warp that meets them:
 // the separate cache-write kernel is not needed on a decode step.
 //
+// Head size 64 with pages of 16 tokens and more, and none of the options, goes on to attention_decode_pages.cu (see
+// dd_attention_decode).
+//
 // The general kernel (attention_rows.cu) remains the reference for every size this one does not
 // take (grouped heads, head sizes other than 64 and 128, float32 caches).
 #include "common.cuh"
