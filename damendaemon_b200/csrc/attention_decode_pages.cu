@@ -15,6 +15,8 @@
 // With k_new/v_new the step's own key and value replace the cache row of the token's position in shared memory
 // and are written to the cache by the warp that owns the head. Rows of the last page beyond the position are
 // zeroed in shared memory (values) or masked by index (scores), so stale cache contents never reach the result.
+// A token whose position is negative sees no key and gets zeros; one beyond the block table sees the keys that have
+// pages, and the missing ones are reported (error bits 2 and 4) as a missing page is.
 // n_splits is the most splits a token's pages may be cut into (the grid's third dimension); when the grid then holds
 // more blocks than can be resident at once, the kernel gives each token its share of them, by its number of pages
 // among all tokens' pages (see the kernel), and the blocks beyond a token's count leave at once.
@@ -140,7 +142,11 @@ attention_decode_pages_kernel(const __grid_constant__ CUtensorMap map_kv, const 
     // divisions here, a hundred cycles each, stood between the positions and the first page request)
     const int span = p.max_blocks << p.log2_P;              // positions the block table can describe
     auto pages_of = [&](int position, int* first) {
-        position = min(max(position, 0), span - 1);
+        if (position < 0) {                                 // no key is visible from before the first one
+            if (first) *first = 0;
+            return 0;
+        }
+        position = min(position, span - 1);
         int from = p.window > 0 ? max(0, position - p.window + 1) : 0;
         if (p.chunk > 0) from = max(from, position - position % p.chunk);
         if (first) *first = from >> p.log2_P;
@@ -159,6 +165,10 @@ attention_decode_pages_kernel(const __grid_constant__ CUtensorMap map_kv, const 
     int first_page = 0;
     const int my_pages = pages_of(pos, &first_page);
     const int last_page = first_page + my_pages - 1;
+    // A position beyond the table: its own key has no page (to be written to, where it comes with the step), nor have the
+    // other visible keys from the table's end on. The keys that have pages are attended to.
+    if (warp == p.G && split == 0 && lane == 0 && pos >= span)
+        atomicOr(p.error_flag, (p.k_new != nullptr ? 2 : 4) | (pos > max(lo, span) ? 4 : 0));
     // pages a block should take: all pages x groups over the blocks that can be resident (every block of a token does
     // the same arithmetic on the same numbers, so they agree whatever the rounding)
     int n_splits = gridDim.z;               // few tokens: every token may have all the splits, the blocks fit anyway
@@ -190,7 +200,9 @@ attention_decode_pages_kernel(const __grid_constant__ CUtensorMap map_kv, const 
                 page = blk < 32 ? low : (blk < p.max_blocks ? high : -1);
             } else if (i0 + lane < n_mine && blk < p.max_blocks) page = bt[blk];
             if (i0 + lane < n_mine && (page < 0 || page >= p.n_pages)) {
-                atomicOr(p.error_flag, p.k_new != nullptr && blk == last_page ? 6 : 4);     // the token's own row finds no place either
+                // (the step's own key finds no place to be written to, and the page's other keys cannot be read)
+                const bool own = p.k_new != nullptr && blk == pos >> p.log2_P;
+                atomicOr(p.error_flag, own ? 2 | (pos > max(lo, blk << p.log2_P) ? 4 : 0) : 4);
                 page = -1;
             }
 #pragma unroll 1

@@ -261,6 +261,54 @@ def test_attention_decode_of_few_tokens(K, heads, page, lengths, n_splits):
             assert K.read_error_flag(DEV) == bits
 
 
+@pytest.mark.parametrize("kernel", ["rows", "pages"])
+@pytest.mark.parametrize("heads,page,n_splits", [(5, 16, 1), (25, 16, 3), (3, 128, 2)])
+def test_attention_decode_of_positions_outside_the_table(K, kernel, heads, page, n_splits):
+    """A position beyond the block table: the keys without a page are reported, the step's own as a write, and nothing is
+    written; the page kernel attends to the others (the row kernel counts a missing key as one of zeros)."""
+    hd, columns = heads * 64, 3
+    span = columns * page
+    c = paged_case(K, torch.bfloat16, heads, heads, 64, page, lengths=[span, 5], new=[1, 1], window=None, n_splits=n_splits)
+    table = c["table"][:, :columns].contiguous()
+    q, k, v = c["packed"].split(hd, dim=1)
+    at = lambda p: torch.tensor([p, 4], dtype=torch.int32, device=DEV)
+    run = lambda p, window=None, cache=c["cache"], **kw: K.attention_decode(q, cache, None, at(p), table, heads, c["scale"], window,
+                                                                            n_splits=n_splits, kernel=kernel, **kw)
+    whole = run(span - 1)
+    assert K.read_error_flag(DEV) == 0 and (whole.double().cpu() - c["ref"]).abs().max() < tol(torch.bfloat16)
+    as_whole = lambda got: bool(torch.isfinite(got).all()) and (kernel == "rows" or torch.equal(got, whole))
+    new = dict(k_new=k, v_new=v)
+    for past, own in ((0, 2), (1, 6), (page + 3, 6)):
+        got = run(span + past)
+        assert K.read_error_flag(DEV) == 4 and as_whole(got)
+        cache = c["cache"].clone()
+        got = run(span + past, cache=cache, **new)
+        assert K.read_error_flag(DEV) == own and as_whole(got)
+        assert torch.equal(cache.view(torch.int16), c["cache"].view(torch.int16)), "a key was written that has no place"
+    got = run(span + 20, window=8)
+    assert K.read_error_flag(DEV) == 4 and bool((got[0] == 0).all()) and torch.equal(got[1], run(span - 1, window=8)[1])
+    assert K.read_error_flag(DEV) == 0
+    table[0, 2] = -1                             # the page of its own position is missing: the key's place, and those before it
+    for p, own in ((2 * page, 2), (2 * page + 1, 6)):
+        run(p, cache=c["cache"].clone(), **new)
+        assert K.read_error_flag(DEV) == own
+
+
+@pytest.mark.parametrize("kernel", ["rows", "pages"])
+@pytest.mark.parametrize("heads,page,n_splits", [(5, 16, 1), (25, 16, 3), (3, 128, 2)])
+def test_attention_decode_before_the_first_position(K, kernel, heads, page, n_splits):
+    hd = heads * 64
+    c = paged_case(K, torch.bfloat16, heads, heads, 64, page, lengths=[40, 5], new=[1, 1], window=None, n_splits=n_splits)
+    q, k, v = c["packed"].split(hd, dim=1)
+    for new in ({}, dict(k_new=k, v_new=v)):
+        cache = c["cache"].clone()
+        got = K.attention_decode(q, cache, None, torch.tensor([-1, 4], dtype=torch.int32, device=DEV), c["table"], heads, c["scale"],
+                                 n_splits=n_splits, kernel=kernel, **new)
+        assert K.read_error_flag(DEV) == 0 and bool((got[0] == 0).all())
+        assert (got[1].double().cpu() - c["ref"][1]).abs().max() < tol(torch.bfloat16)
+        assert torch.equal(cache.view(torch.int16), c["cache"].view(torch.int16))
+
+
 @pytest.mark.parametrize("heads,page", [(25, 16), (8, 64), (20, 32)])
 @pytest.mark.parametrize("n_splits", [3, 8])
 @pytest.mark.parametrize("window", [None, 100])
