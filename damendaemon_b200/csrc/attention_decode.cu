@@ -314,7 +314,8 @@ attention_decode_kernel(const __nv_bfloat16* q, int q_stride, const __nv_bfloat1
         if (t4 == 0) { sh_ml[warp][0] = m; sh_ml[warp][1] = l; }
     }
     __syncthreads();
-    // combine the warps: thread d owns output dimension d
+    // combine the warps: thread d owns output dimension d (a warp or a split without a live key has the sum 0; a NaN sum, from a
+    // score that is not a number, goes on to the result)
     if (gate) gated = 1.0f / (1.0f + __expf(-__bfloat162float(gate[(size_t)t * gate_stride + h])));
     const size_t item = ((size_t)t * H + h) * n_splits + split;
     float M = -CUDART_INF_F;
@@ -322,7 +323,7 @@ attention_decode_kernel(const __nv_bfloat16* q, int q_stride, const __nv_bfloat1
     for (int w = 0; w < WARPS; ++w) M = fmaxf(M, sh_ml[w][0]);
     float L = 0.f;
 #pragma unroll
-    for (int w = 0; w < WARPS; ++w) L += sh_ml[w][1] > 0.f ? sh_ml[w][1] * exp2f(sh_ml[w][0] - M) : 0.f;
+    for (int w = 0; w < WARPS; ++w) L += sh_ml[w][1] != 0.f ? sh_ml[w][1] * exp2f(sh_ml[w][0] - M) : 0.f;
     // a sink joins the sum as one more term, exp2(sink - maximum) with the maximum taken over it too, where a token's
     // last sum is made (here without a key split, else where the splits are merged)
     const float sink2 = sink ? sink[h] * 1.4426950408889634f : -CUDART_INF_F;
@@ -335,9 +336,9 @@ attention_decode_kernel(const __nv_bfloat16* q, int q_stride, const __nv_bfloat1
     for (int d = threadIdx.x; d < D; d += WARPS * 32) {
         float acc = 0.f;
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w) acc += sh_ml[w][1] > 0.f ? sh_o[w][d] * exp2f(sh_ml[w][0] - M) : 0.f;
+        for (int w = 0; w < WARPS; ++w) acc += sh_ml[w][1] != 0.f ? sh_o[w][d] * exp2f(sh_ml[w][0] - M) : 0.f;
         if (n_splits == 1)
-            out[(size_t)t * out_stride + (size_t)h * D + d] = __float2bfloat16_rn(L_all > 0.f ? acc * with_sink / L_all * gated : 0.f);
+            out[(size_t)t * out_stride + (size_t)h * D + d] = __float2bfloat16_rn(L_all != 0.f ? acc * with_sink / L_all * gated : 0.f);
         else part_o[item * D + d] = acc;
     }
     STAMP(12);
@@ -368,17 +369,21 @@ attention_decode_kernel(const __nv_bfloat16* q, int q_stride, const __nv_bfloat1
                 oo[u] = live ? __ldcg(part_o + it * D + d) : 0.f;
             }
             float cm = Mx;
+            bool any = false;
 #pragma unroll
             for (int u = 0; u < 8; ++u)
-                if (ll[u] > 0.f) cm = fmaxf(cm, mm[u]);
-            if (cm == -CUDART_INF_F) continue;            // nothing live so far
+                if (ll[u] != 0.f) {
+                    cm = fmaxf(cm, mm[u]);
+                    any = true;
+                }
+            if (!any) continue;
             const float keep = Mx == -CUDART_INF_F ? 0.f : exp2f(Mx - cm);
             acc *= keep;
             Lx *= keep;
             Mx = cm;
 #pragma unroll
             for (int u = 0; u < 8; ++u)
-                if (ll[u] > 0.f) {
+                if (ll[u] != 0.f) {
                     const float w = exp2f(mm[u] - Mx);
                     Lx += ll[u] * w;
                     acc += oo[u] * w;
@@ -390,7 +395,7 @@ attention_decode_kernel(const __nv_bfloat16* q, int q_stride, const __nv_bfloat1
             acc *= keep;
             Lx = Lx * keep + exp2f(sink2 - M2);
         }
-        out[(size_t)t * out_stride + (size_t)h * D + d] = __float2bfloat16_rn(Lx > 0.f ? acc / Lx * gated : 0.f);
+        out[(size_t)t * out_stride + (size_t)h * D + d] = __float2bfloat16_rn(Lx != 0.f ? acc / Lx * gated : 0.f);
     }
     if (threadIdx.x == 0) counters[t * H + h] = 0;
     STAMP(13);

@@ -329,7 +329,7 @@ attention_decode_pages_kernel(const __grid_constant__ CUtensorMap map_kv, const 
     const float o0 = t4 == 0 ? o[0][0] : (t4 == 1 ? o[1][0] : (t4 == 2 ? o[2][0] : o[3][0]));
     const float o1 = t4 == 0 ? o[0][1] : (t4 == 1 ? o[1][1] : (t4 == 2 ? o[2][1] : o[3][1]));
     if (n_splits == 1) {
-        float inv = l > 0.f ? 1.f / l : 0.f;
+        float inv = l != 0.f ? 1.f / l : 0.f;
         if (p.gate) inv *= 1.0f / (1.0f + __expf(-__bfloat162float(p.gate[(size_t)t * p.gate_stride + h])));
         __nv_bfloat16* dst = p.out + (size_t)t * p.out_stride + (size_t)h * D + d;
         dst[0] = __float2bfloat16_rn(o0 * inv);
@@ -359,15 +359,17 @@ attention_decode_pages_kernel(const __grid_constant__ CUtensorMap map_kv, const 
 #pragma unroll
         for (int u = 0; u < 8; ++u)
             oo[u] = sp0 + u < n_splits ? __ldcg(reinterpret_cast<const float2*>(p.part_o + (first + sp0 + u) * D) + lane) : make_float2(0.f, 0.f);
-        float cm = ml.y > 0.f ? ml.x : -CUDART_INF_F;
+        // a split without a live key has the sum 0 and adds nothing, whatever its scratch holds; a NaN sum goes on to the result
+        const bool live = ml.y != 0.f;
+        float cm = live ? ml.x : -CUDART_INF_F;
 #pragma unroll
         for (int x = 4; x > 0; x >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, x));
         cm = fmaxf(cm, Mx);
-        if (cm == -CUDART_INF_F) continue;                  // nothing live so far
+        if (!__any_sync(0xffffffffu, live)) continue;
         const float keep = Mx == -CUDART_INF_F ? 0.f : exp2f(Mx - cm);
         Mx = cm;
-        const float w = ml.y > 0.f ? exp2f(ml.x - Mx) : 0.f;
-        float sum = ml.y > 0.f ? ml.y * w : 0.f;
+        const float w = live ? exp2f(ml.x - Mx) : 0.f;
+        float sum = live ? ml.y * w : 0.f;
 #pragma unroll
         for (int x = 4; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
         Lx = Lx * keep + sum;
@@ -376,14 +378,14 @@ attention_decode_pages_kernel(const __grid_constant__ CUtensorMap map_kv, const 
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const float wu = __shfl_sync(0xffffffffu, w, u);
-            if (wu > 0.f) {                                 // a split without a live key adds nothing, whatever its scratch holds
+            if (wu != 0.f) {
                 a0 += oo[u].x * wu;
                 a1 += oo[u].y * wu;
             }
         }
     }
     const float gated = p.gate ? 1.0f / (1.0f + __expf(-__bfloat162float(p.gate[(size_t)t * p.gate_stride + h]))) : 1.0f;
-    const float inv = Lx > 0.f ? gated / Lx : 0.f;
+    const float inv = Lx != 0.f ? gated / Lx : 0.f;
     *reinterpret_cast<uint32_t*>(p.out + (size_t)t * p.out_stride + (size_t)h * D + 2 * lane) = pack_bf16(a0 * inv, a1 * inv);
     if (lane == 0) p.counters[t * p.H + h] = 0;
 }

@@ -309,6 +309,30 @@ def test_attention_decode_before_the_first_position(K, kernel, heads, page, n_sp
         assert torch.equal(cache.view(torch.int16), c["cache"].view(torch.int16))
 
 
+@pytest.mark.parametrize("kernel", ["rows", "pages"])
+@pytest.mark.parametrize("n_splits", [1, 3, 8])
+def test_attention_decode_of_scores_that_are_not_numbers(K, kernel, n_splits):
+    """One NaN key, wherever it lies, leaves its head of that token without a result, however the keys are split; a NaN query
+    its head too. The others have the bits of the run without it."""
+    heads, hd = 5, 320
+    lengths = [300, 300, 300, 300, 300, 40, 300]
+    c = paged_case(K, torch.bfloat16, heads, heads, 64, 16, lengths=lengths, new=[1] * 7, window=None, n_splits=n_splits)
+    run = lambda q, cache: K.attention_decode(q, cache, None, c["pos"], c["table"], heads, c["scale"], n_splits=n_splits,
+                                              kernel=kernel).view(7, heads, 64)
+    clean = run(c["q"], c["cache"])
+    assert bool(torch.isfinite(clean).all())
+    cache, q = c["cache"].clone(), c["q"].clone()
+    odd = torch.zeros(7, heads, dtype=torch.bool, device=DEV)
+    for e, (key, head) in enumerate(((0, 0), (17, 1), (150, 2), (298, 4), (299, 3), (39, 0))):
+        cache[c["table"][e, key // 16], 0, head, key % 16] = float("nan")
+        odd[e, head] = True
+    q[6, 64:128] = float("nan")
+    odd[6, 1] = True
+    got = run(q, cache)
+    assert bool(torch.isnan(got[odd]).all()) and torch.equal(got[~odd], clean[~odd])
+    assert torch.equal(run(c["q"], c["cache"]), clean) and K.read_error_flag(DEV) == 0
+
+
 @pytest.mark.parametrize("heads,page", [(25, 16), (8, 64), (20, 32)])
 @pytest.mark.parametrize("n_splits", [3, 8])
 @pytest.mark.parametrize("window", [None, 100])
