@@ -16,8 +16,8 @@
 // from there instead of the cache and written to the cache page by the one warp that meets them:
 // the separate cache-write kernel is not needed on a decode step.
 //
-// Head size 64 with pages of 16 tokens and more, and none of the options, goes on to attention_decode_pages.cu (see
-// dd_attention_decode).
+// Of head size 64 with pages of 16 tokens and more, whole pages stream through attention_decode_pages.cu instead where
+// that is ahead (parts/paged_attention.py decides).
 //
 // The general kernel (attention_rows.cu) remains the reference for every size this one does not
 // take (grouped heads, head sizes other than 64 and 128, float32 caches).
@@ -402,15 +402,6 @@ attention_decode_kernel(const __nv_bfloat16* q, int q_stride, const __nv_bfloat1
 }
 }  // namespace
 
-// attention_decode_pages.cu
-DD_API int dd_attention_decode_pages_supported(int n_heads, int n_kv_heads, int head_dim, int page_size, int dtype);
-DD_API int dd_attention_decode_pages(const void* q, int q_stride, const void* k_new, const void* v_new, void* cache,
-                                     const int* tok_entry, const int* tok_pos, const int* block_table, int max_blocks,
-                                     void* out, int out_stride, float* part_o, float* part_ml, int* counters, int n_tokens,
-                                     int n_heads, int n_kv_heads, int head_dim, int page_size, int n_pages, int window,
-                                     float scale, int n_splits, int* error_flag, void* stream, int chunk, const void* gate,
-                                     int gate_stride);
-
 // A device buffer of 16 stamps per block of the following launches; null switches the stamps off.
 DD_API void dd_attention_decode_stamps(unsigned long long* buffer) { cudaMemcpyToSymbol(g_stamps, &buffer, sizeof(buffer)); }
 
@@ -483,14 +474,6 @@ DD_API int dd_attention_decode(const void* q, int q_stride, const void* k_new, c
                                float* part_ml, int* counters, int n_tokens, int n_heads, int n_kv_heads, int head_dim,
                                int page_size, int n_pages, int window, float scale, int n_splits, int* error_flag,
                                void* stream, int chunk, const void* gate, int gate_stride) {
-    // Sizes that the page-streaming kernel takes go to it: since it has no barriers of the block and merges a head at a time
-    // it is ahead at a few (token, head) pairs too (a whole decode step of 25 heads in 24 layers, rows / pages: 1 token at 64
-    // keys 0.817 / 0.752 ms, at 512 keys 0.858 / 0.833, at 900 0.897 / 0.898; 4 tokens at 512 keys 1.08 / 1.00).
-    if (dd_attention_decode_pages_supported(n_heads, n_kv_heads, head_dim, page_size, DD_BF16) && n_splits >= 1 &&
-        dd_ceil_div(max_blocks, n_splits) <= 128)
-        return dd_attention_decode_pages(q, q_stride, k_new, v_new, cache, tok_entry, tok_pos, block_table, max_blocks, out, out_stride,
-                                         part_o, part_ml, counters, n_tokens, n_heads, n_kv_heads, head_dim, page_size, n_pages, window,
-                                         scale, n_splits, error_flag, stream, chunk, gate, gate_stride);
     return dd_attention_decode_sinks(q, q_stride, k_new, v_new, cache, tok_entry, tok_pos, block_table, max_blocks, out,
                                      out_stride, part_o, part_ml, counters, n_tokens, n_heads, n_kv_heads, head_dim, page_size,
                                      n_pages, window, scale, n_splits, error_flag, stream, chunk, gate, gate_stride, 0, 0.f, nullptr, 0);

@@ -1632,9 +1632,8 @@ def attention_decode(q, cache, token_entry, positions, block_table, n_heads, sca
                      k_new=None, v_new=None, kernel="rows", chunk=None, gate=None, keep_first=0, softcap=None, sink=None,
                      exact_weights=False):
     """Decode attention (one query per token) over a bfloat16 cache. kernel 'pages': whole pages of a group of heads by TMA
-    (see attention_decode_pages_supported); 'rows': for few (token, head) pairs and for what 'pages' does not take, a warp
-    copies key rows 16 bytes at a time (see attention_decode_supported); of it the launcher gives sizes that 'pages' takes to that
-    kernel too, cut into the splits asked for here. With k_new/v_new (row views of the buffer q lives in) the step's own keys and
+    (see attention_decode_pages_supported); 'rows': a warp copies key rows 16 bytes at a time (see
+    attention_decode_supported). With k_new/v_new (row views of the buffer q lives in) the step's own keys and
     values are used from there and written into the cache by this kernel; otherwise they must be in the cache already.
     token_entry None: token t belongs to entry t (a step of single tokens in entry order). n_splits: into how many
     pieces a token's keys are cut; for 'pages' the most a token may get (the kernel deals them out by context length).

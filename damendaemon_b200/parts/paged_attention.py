@@ -16,12 +16,14 @@ import torch
 
 from .. import kernels
 
+PAGES_HEAD_DIM = 64                       # the only head size of the page-streaming decode kernel
+
 
 @dataclass(frozen=True)
 class AttentionTuning:
     """Thresholds of the kernel choice, measured on a B200 with 25 heads of 64: from pages_from_pairs on the key splits are those
     of the page-streaming decode kernel, which deals them out by the contexts; below, a token's keys are cut by
-    row_keys_per_block (the launcher of the row kernel gives sizes that page streaming takes to that kernel all the same)."""
+    row_keys_per_block, for page streaming as for the row kernel."""
     pages_from_pairs: int = 150           # decode steps with at least this many (token, head) pairs deal the splits out,
     pages_from_pair_keys: int = 200_000   # ... or with this many pairs x keys of context (one request of 16,384 keys)
     pages_per_block: int = 128            # a block of the page-streaming kernel holds the ids of this many pages
@@ -85,22 +87,28 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
     tensor = fast and runtime.attention != "mma" and not special
     # a sink alone (no kept first keys, no cap, no weights in two terms) the tcgen05 prompt kernel takes as well
     sink_only = sink is not None and not (keep_first or softcap or exact_weights)
-    def wants_pages(n_tokens):
+    def decode_splits(n_tokens):
+        """(kernel, pieces of a token's keys) for single tokens that a tensor-core decode kernel takes."""
         pairs = n_tokens * n_heads
-        return pairs >= tune.pages_from_pairs or pairs * ctx.split_context >= tune.pages_from_pair_keys
-    if ctx.decode_only and tensor and wants_pages(ctx.n_tokens) and \
-            kernels.attention_decode_pages_supported(n_heads, kv_heads, head_dim, page_size, q.dtype):
-        # whole pages of a group of heads by TMA; it takes the new keys and values from the projection and writes them
-        splits = kernels.attention_decode_pages_splits(ctx.n_tokens, n_heads, page_size, ctx.split_context, q.device)
-        splits = max(splits, -(-table.shape[1] // tune.pages_per_block))
-        # (decode only: token t is entry t, so the kernels are spared the look-up)
-        return kernels.attention_decode(q, kv, None, ctx.positions, table, n_heads, scale, window,
-                                        n_splits=splits, k_new=k_new, v_new=v_new, kernel="pages", **masked)
-    if ctx.decode_only and fast and kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype):
-        # the decode kernel takes the new keys and values from the projection and writes them itself
-        splits = ctx.key_splits(n_heads, keys_per_block=tune.row_keys_per_block, blocks_per_sm=tune.row_blocks_per_sm)
-        return kernels.attention_decode(q, kv, None, ctx.positions, table, n_heads, scale, window,
-                                        n_splits=splits, k_new=k_new, v_new=v_new, **masked, **exact)
+        # (the kernels are asked only about the head size that pages can have: an eager step asks for every layer)
+        if tensor and head_dim == PAGES_HEAD_DIM and kernels.attention_decode_pages_supported(n_heads, kv_heads, head_dim, page_size, q.dtype):
+            # whole pages of a group of heads by TMA
+            if pairs >= tune.pages_from_pairs or pairs * ctx.split_context >= tune.pages_from_pair_keys:
+                splits = kernels.attention_decode_pages_splits(n_tokens, n_heads, page_size, ctx.split_context, q.device)
+                return "pages", max(splits, -(-table.shape[1] // tune.pages_per_block))
+            splits = ctx.key_splits(n_heads, keys_per_block=tune.row_keys_per_block, blocks_per_sm=tune.row_blocks_per_sm, n_tokens=n_tokens)
+            if table.shape[1] <= splits * tune.pages_per_block:
+                return "pages", splits
+        elif not kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype):
+            return None, 0
+        return "rows", ctx.key_splits(n_heads, keys_per_block=tune.row_keys_per_block, blocks_per_sm=tune.row_blocks_per_sm, n_tokens=n_tokens)
+    if ctx.decode_only and fast:
+        kernel, splits = decode_splits(ctx.n_tokens)
+        if kernel:
+            # the decode kernels take the new keys and values from the projection and write them (decode only: token t is entry t,
+            # so they are spared the look-up)
+            return kernels.attention_decode(q, kv, None, ctx.positions, table, n_heads, scale, window,
+                                            n_splits=splits, k_new=k_new, v_new=v_new, kernel=kernel, **masked, **exact)
     # key/value groups and small heads (8 requests x 25 heads on 5, 400 keys: 9 us, 32 through the general kernel and the cache
     # write; 32 x 16 on 4, 600 keys: 37 / 69; 8 x 32 heads of 128 on 8: 32 / 41)
     if ctx.decode_only and tensor and cores():
@@ -114,28 +122,20 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
     # key blocks on a single token (measured with 56 decoding requests beside 8 portions of 249 tokens, 36 layers:
     # 8.3 ms a step through the prompt kernel alone, against 4.5 ms for 2,048 prompt tokens).
     n1 = ctx.n_single if tcgen05 or mma else 0
-    rows = n1 and kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype)
-    if n1 and not rows and not (tensor and cores()):
+    kernel, splits = decode_splits(n1) if n1 and kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype) else (None, 0)
+    if n1 and not kernel and not (tensor and cores()):
         n1 = 0
     out = None
     if n1:
         out = torch.empty((q.shape[0], n_heads * head_dim), dtype=q.dtype, device=q.device)
-        pages = rows and tensor and wants_pages(n1) and \
-            kernels.attention_decode_pages_supported(n_heads, kv_heads, head_dim, page_size, q.dtype)
-        if pages:
-            splits = kernels.attention_decode_pages_splits(n1, n_heads, page_size, ctx.split_context, q.device)
-            splits = max(splits, -(-table.shape[1] // tune.pages_per_block))
-        elif rows:
-            splits = ctx.key_splits(n_heads, keys_per_block=tune.row_keys_per_block, blocks_per_sm=tune.row_blocks_per_sm,
-                                    n_tokens=n1)
-        if not rows:
+        if not kernel:
             kernels.attention_tokens(q[:n1], kv, ctx.positions[:n1], table, n_heads, scale, window, n_splits=token_splits(ctx, n1, n_heads),
                                      out=out[:n1], k_new=None if k_new is None else k_new[:n1], v_new=None if v_new is None else v_new[:n1],
                                      chunk=chunk, gate=None if gate is None else gate[:n1])
         else:
             kernels.attention_decode(q[:n1], kv, None, ctx.positions[:n1], table, n_heads, scale, window, n_splits=splits,
                                      out=out[:n1], k_new=None if k_new is None else k_new[:n1],
-                                     v_new=None if v_new is None else v_new[:n1], kernel="pages" if pages else "rows",
+                                     v_new=None if v_new is None else v_new[:n1], kernel=kernel,
                                      chunk=chunk, gate=None if gate is None else gate[:n1], **exact)
         if n1 == ctx.n_entries:
             return out

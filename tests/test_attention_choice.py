@@ -64,13 +64,13 @@ class Recorder:
 
 
 def step(n_single, portions, heads=25, head_dim=64, dtype=torch.bfloat16, context=768, aligned=False, attention="auto",
-         writable=True, page=16):
+         writable=True, page=16, tuning=None):
     """A context of n_single single-token entries followed by portions (a list of lengths), and its q, k, v and cache."""
     lengths = [1] * n_single + list(portions)
     n, e = sum(lengths), len(lengths)
     start = torch.tensor([sum(lengths[:i]) for i in range(e + 1)], dtype=torch.int32)
     group = types.SimpleNamespace(name="all")
-    runtime = types.SimpleNamespace(attention=attention, attention_tuning=pa.AttentionTuning())
+    runtime = types.SimpleNamespace(attention=attention, attention_tuning=tuning or pa.AttentionTuning())
     ctx = StepContext(n_tokens=n, n_entries=e, n_wanted=1, token_ids=torch.zeros(n, dtype=torch.int32),
                       positions=torch.zeros(n, dtype=torch.int32), token_entry=torch.zeros(n, dtype=torch.int32),
                       want_rows=torch.zeros(1, dtype=torch.int32), entry_slot=torch.zeros(e, dtype=torch.int32),
@@ -99,10 +99,13 @@ def run(recorder, *args, **kwargs):
 
 def test_decode_steps_by_pairs_and_context(recorder):
     assert run(recorder, 8, [])[-1] == ("decode-pages", 8, True, True)          # 200 pairs: whole pages by TMA
-    assert run(recorder, 4, [])[-1] == ("decode-rows", 4, True, True)           # 100 pairs at 768 keys: rows
-    assert run(recorder, 1, [], context=16384)[-1][0] == "decode-pages"         # one long request: pages again
-    assert run(recorder, 1, [], context=4096)[-1][0] == "decode-rows"
+    assert run(recorder, 4, [])[-1] == ("decode-pages", 4, True, True)          # ... however few there are
+    assert run(recorder, 1, [], context=16384)[-1][0] == "decode-pages"
+    assert run(recorder, 1, [], context=4096)[-1][0] == "decode-pages"
     assert run(recorder, 2, [], context=4096)[-1][0] == "decode-pages"
+    assert run(recorder, 4, [], head_dim=128)[-1] == ("decode-rows", 4, True, True)       # pages are of heads of 64 only: rows
+    assert run(recorder, 4, [], attention="mma")[-1] == ("decode-rows", 4, True, True)    # no TMA kernels on request
+    assert run(recorder, 8, [], attention="mma")[-1] == ("decode-rows", 8, True, True)
     assert run(recorder, 8, [], writable=False)[-1] == ("decode-pages", 8, True, False)   # another layer's cache: nothing to write
     assert run(recorder, 8, [], attention="rows")[-1][0] == "rows"              # the general kernel on request
     assert run(recorder, 8, [], dtype=torch.float32)[-1][0] == "rows"           # the float32 path
@@ -113,7 +116,7 @@ def test_mixed_steps_are_split(recorder):
     assert calls == [("decode-pages", 56, True, True), ("prefill-tcgen05", 8, True, 8)]      # fused cache write for the portions
     recorder.calls.clear()
     calls = run(recorder, 3, [100, 7])
-    assert calls == [("decode-rows", 3, True, True), ("kv_store", 107), ("prefill-tcgen05", 2, False, 2)]
+    assert calls == [("decode-pages", 3, True, True), ("kv_store", 107), ("prefill-tcgen05", 2, False, 2)]
     recorder.calls.clear()
     calls = run(recorder, 0, [128, 128], aligned=True)
     assert calls == [("prefill-tcgen05", 2, True, 2)]

@@ -173,6 +173,23 @@ def test_attention_rows_split_decode(K, dtype, n_splits):
     assert (out.float() - one.float()).abs().max() < tol(dtype)
 
 
+@pytest.mark.parametrize("heads,page,tokens", [(5, 16, 1), (25, 16, 4), (3, 128, 2)])
+def test_attention_decode_runs_the_kernel_that_is_named(K, heads, page, tokens):
+    """'rows' is the row kernel for sizes that page streaming takes as well: the bits of the entry point that has no other
+    kernel, and any alignment of the result's rows that a bfloat16 may have."""
+    hd, lengths = heads * 64, [540, 3, 77, 300][:tokens]
+    c = paged_case(K, torch.bfloat16, heads, heads, 64, page, lengths=lengths, new=[1] * tokens, window=None, n_splits=2)
+    run = lambda **kw: K.attention_decode(c["q"], c["cache"], None, c["pos"], c["table"], heads, c["scale"], n_splits=2, **kw)
+    rows, pages = run(kernel="rows"), run(kernel="pages")
+    # (a sink of no weight adds zero to the sum: the options' entry point)
+    sinks = run(kernel="rows", sink=torch.full((heads,), -float("inf"), device=DEV))
+    assert torch.equal(rows, sinks) and torch.equal(rows, run()) and not torch.equal(rows, pages)
+    wide = torch.full((tokens, hd + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+    assert torch.equal(run(kernel="rows", out=wide[:, 3:3 + hd]), rows)
+    assert bool((wide[:, :3] == 7).all()) and bool((wide[:, 3 + hd:] == 7).all())
+    assert K.read_error_flag(DEV) == 0
+
+
 @pytest.mark.parametrize("d,heads,page", [(64, 5, 16), (128, 3, 8), (64, 25, 16)])
 @pytest.mark.parametrize("n_splits", [1, 3, 8])
 @pytest.mark.parametrize("window", [None, 100])
@@ -246,19 +263,21 @@ def test_attention_decode_pages(K, heads, page, n_splits, window):
                                                 (3, 128, [1000])])
 @pytest.mark.parametrize("n_splits", [1, 4, 9])
 def test_attention_decode_of_few_tokens(K, heads, page, lengths, n_splits):
-    """Few (token, head) pairs are page-streamed in groups of at most four heads (the last group smaller), whichever kernel is
-    asked for; a page that is missing is reported, as a write too where the token's own key belongs there."""
+    """Few (token, head) pairs are page-streamed in groups of at most four heads (the last group smaller); a page that is
+    missing is reported, as a write too where the token's own key belongs there. The row kernel agrees."""
     c = paged_case(K, torch.bfloat16, heads, heads, 64, page, lengths=lengths, new=[1] * len(lengths), window=None, n_splits=n_splits, spike=5)
     args = (None, c["pos"], c["table"], heads, c["scale"])
     out, pages = (K.attention_decode(c["q"], c["cache"], *args, n_splits=n_splits, kernel=k) for k in ("rows", "pages"))
-    assert K.read_error_flag(DEV) == 0 and torch.equal(out, pages)
-    assert (out.double().cpu() - c["ref"]).abs().max() < tol(torch.bfloat16)
+    assert K.read_error_flag(DEV) == 0
+    for got in (out, pages):
+        assert (got.double().cpu() - c["ref"]).abs().max() < tol(torch.bfloat16)
     for own, bits in ((False, 4), (True, 6)):
         if len(lengths) == 1 and (own or lengths[0] > page):
             args[2][0, (lengths[0] - 1) // page if own else 0] = -1
             new = {} if not own else dict(k_new=c["packed"][:, heads * 64:2 * heads * 64], v_new=c["packed"][:, 2 * heads * 64:])
-            K.attention_decode(c["q"], c["cache"], *args, n_splits=n_splits, **new)
-            assert K.read_error_flag(DEV) == bits
+            for kernel in ("rows", "pages"):
+                K.attention_decode(c["q"], c["cache"], *args, n_splits=n_splits, kernel=kernel, **new)
+                assert K.read_error_flag(DEV) == bits
 
 
 @pytest.mark.parametrize("kernel", ["rows", "pages"])
