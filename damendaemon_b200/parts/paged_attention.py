@@ -21,11 +21,14 @@ PAGES_HEAD_DIM = 64                       # the only head size of the page-strea
 
 @dataclass(frozen=True)
 class AttentionTuning:
-    """Thresholds of the kernel choice, measured on a B200 with 25 heads of 64: from pages_from_pairs on the key splits are those
-    of the page-streaming decode kernel, which deals them out by the contexts; below, a token's keys are cut by
-    row_keys_per_block, for page streaming as for the row kernel."""
-    pages_from_pairs: int = 150           # decode steps with at least this many (token, head) pairs deal the splits out,
-    pages_from_pair_keys: int = 200_000   # ... or with this many pairs x keys of context (one request of 16,384 keys)
+    """Thresholds of the kernel choice. Whole pages by TMA are ahead of rows at any number of single tokens (us a layer of a
+    whole decode step on a B200, rows / pages: 25 heads, one request at 64, 300, 600, 900 keys 31.3 / 28.5, 31.3 / 29.7,
+    31.2 / 30.4, 31.6 / 31.6; two at 900 34.9 / 32.9, four at 540 37.2 / 33.6, eight at 540 39.3 / 35.4; 16 heads, eight at 900
+    37.9 / 33.0; one request of 4,000 keys in a table of 4,096 42.3 / 38.7), so by default every step takes them. The
+    splits are dealt out by the contexts (attention_decode_pages_splits): cut by row_keys_per_block instead, four requests at
+    900 keys x 25 heads took 42.0 us and eight at 900 x 16 heads 40.7 (now 35.5 and 33.0)."""
+    pages_from_pairs: int = 1             # steps with at least this many (token, head) pairs stream whole pages,
+    pages_from_pair_keys: int = 200_000   # ... or with this many pairs x keys of context; others take the row kernel
     pages_per_block: int = 128            # a block of the page-streaming kernel holds the ids of this many pages
     row_keys_per_block: int = 128         # key split of the row decode kernel: keys per block ...
     row_blocks_per_sm: int = 2            # ... and blocks wanted per SM
@@ -91,17 +94,15 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
         """(kernel, pieces of a token's keys) for single tokens that a tensor-core decode kernel takes."""
         pairs = n_tokens * n_heads
         # (the kernels are asked only about the head size that pages can have: an eager step asks for every layer)
-        if tensor and head_dim == PAGES_HEAD_DIM and kernels.attention_decode_pages_supported(n_heads, kv_heads, head_dim, page_size, q.dtype):
+        many = pairs >= tune.pages_from_pairs or pairs * ctx.split_context >= tune.pages_from_pair_keys
+        if tensor and many and head_dim == PAGES_HEAD_DIM and \
+                kernels.attention_decode_pages_supported(n_heads, kv_heads, head_dim, page_size, q.dtype):
             # whole pages of a group of heads by TMA
-            if pairs >= tune.pages_from_pairs or pairs * ctx.split_context >= tune.pages_from_pair_keys:
-                splits = kernels.attention_decode_pages_splits(n_tokens, n_heads, page_size, ctx.split_context, q.device)
-                return "pages", max(splits, -(-table.shape[1] // tune.pages_per_block))
-            splits = ctx.key_splits(n_heads, keys_per_block=tune.row_keys_per_block, blocks_per_sm=tune.row_blocks_per_sm, n_tokens=n_tokens)
-            if table.shape[1] <= splits * tune.pages_per_block:
-                return "pages", splits
-        elif not kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype):
-            return None, 0
-        return "rows", ctx.key_splits(n_heads, keys_per_block=tune.row_keys_per_block, blocks_per_sm=tune.row_blocks_per_sm, n_tokens=n_tokens)
+            splits = kernels.attention_decode_pages_splits(n_tokens, n_heads, page_size, ctx.split_context, q.device)
+            return "pages", max(splits, -(-table.shape[1] // tune.pages_per_block))
+        if kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype):
+            return "rows", ctx.key_splits(n_heads, keys_per_block=tune.row_keys_per_block, blocks_per_sm=tune.row_blocks_per_sm, n_tokens=n_tokens)
+        return None, 0
     if ctx.decode_only and fast:
         kernel, splits = decode_splits(ctx.n_tokens)
         if kernel:

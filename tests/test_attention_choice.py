@@ -111,6 +111,26 @@ def test_decode_steps_by_pairs_and_context(recorder):
     assert run(recorder, 8, [], dtype=torch.float32)[-1][0] == "rows"           # the float32 path
 
 
+def test_thresholds_of_a_tuning_leave_small_steps_to_the_row_kernel(recorder):
+    tuning = pa.AttentionTuning(pages_from_pairs=150, pages_from_pair_keys=200_000)
+    assert run(recorder, 8, [], tuning=tuning)[-1] == ("decode-pages", 8, True, True)          # 200 pairs: whole pages by TMA
+    assert run(recorder, 4, [], tuning=tuning)[-1] == ("decode-rows", 4, True, True)           # 100 pairs at 768 keys: rows
+    assert run(recorder, 1, [], context=16384, tuning=tuning)[-1][0] == "decode-pages"         # one long request: pages again
+    assert run(recorder, 1, [], context=4096, tuning=tuning)[-1][0] == "decode-rows"
+    assert run(recorder, 2, [], context=4096, tuning=tuning)[-1][0] == "decode-pages"
+
+
+def test_the_splits_of_a_few_tokens_are_dealt_out(recorder, monkeypatch):
+    """... by their contexts, as those of many are: a count of its own for a few cut 8 requests x 16 heads at 900 keys in three."""
+    asked = []
+    monkeypatch.setattr(recorder, "attention_decode_pages_splits", lambda *a: asked.append(a[:4]) or 7, raising=False)
+    taken = []
+    monkeypatch.setattr(recorder, "attention_decode", lambda q, *a, n_splits=1, kernel="rows", **m: taken.append((kernel, n_splits)) or q)
+    run(recorder, 1, [])
+    run(recorder, 8, [], heads=16)
+    assert asked == [(1, 25, 16, 768), (8, 16, 16, 768)] and taken == [("pages", 7)] * 2
+
+
 def test_mixed_steps_are_split(recorder):
     calls = run(recorder, 56, [249] * 8, aligned=True)
     assert calls == [("decode-pages", 56, True, True), ("prefill-tcgen05", 8, True, 8)]      # fused cache write for the portions
