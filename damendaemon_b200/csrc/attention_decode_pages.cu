@@ -3,7 +3,7 @@
 //
 // In the cache a page holds the keys of all heads side by side and then the values ([page][K|V][head][slot][64]):
 // the keys of G neighbouring heads are one run of G x page_size rows of 128 bytes. A block owns (token, group of
-// G <= 7 heads, split of the token's pages); one warp asks TMA for one box of G x page_size rows of keys and one
+// G <= 8 heads, split of the token's pages); one warp asks TMA for one box of G x page_size rows of keys and one
 // of values per page, as many pages ahead as the ring holds, so a block moves its bytes in pieces of tens of KB with two instructions
 // each (copying the same bytes 16 at a time, one key row per 8 lanes, the memory system delivered 4.5 TB/s;
 // in boxes of this size it delivers 5.4). The 128-byte swizzle of the tensor map is the layout ldmatrix wants.
@@ -26,7 +26,7 @@
 #include <math_constants.h>
 
 namespace {
-constexpr int D = 64, TILE = 16, MAX_GROUP = 7, MAX_THREADS = (MAX_GROUP + 1) * 32;      // a warp a head, and one that requests pages
+constexpr int D = 64, TILE = 16, MAX_GROUP = 8;      // heads of a block: a warp each, and one that requests pages
 constexpr int MAX_BLOCK_PAGES = 128;          // pages a block may own; 1 << 7 below
 constexpr int MAX_STAGES = 3;                 // deeper rings are no faster and leave fewer blocks an SM (see the kernel)
 
@@ -89,7 +89,9 @@ __device__ __forceinline__ uint32_t tile_off(int r, int c) { return (uint32_t)(r
 // (xl, 64 steps) 129.7 / 117.8 ms, 64 from 256 keys on 204.1 / 195.8, 32 of 16 to 800 keys (medium) 48.9 / 44.4.
 // 80 registers and three stages leave three blocks an SM: with 104 registers and two blocks the last of these takes 45.9
 // (and the first 118.0), with two stages 44.5 (122.3), with four 46.2; a spilled register costs more than any of them.
-__global__ void __launch_bounds__(MAX_THREADS, 3)
+// Groups of eight (288 threads) take two blocks' registers, 96 a thread.
+template <int MOST>
+__global__ void __launch_bounds__((MOST + 1) * 32, MOST < 8 ? 3 : 2)
 attention_decode_pages_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_last, const Params p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -406,8 +408,10 @@ EncodeTiled encode_fn() {
     return fn;
 }
 
-// Heads per block, spread evenly over the groups: up to seven (a warp each, 256 box rows at most), since the fewer and
-// larger the boxes the better they stream (64 tokens x 25 heads: a step of 195 ms in groups of 7, 214 in groups of 5);
+// Heads per block, spread evenly over the groups: up to eight (a warp each, 256 box rows at most), since the fewer and
+// larger the boxes the better they stream (64 tokens x 25 heads: a step of 195 ms in groups of 7, 214 in groups of 5; us a
+// layer of a whole step in groups of at most seven / eight: 32 heads, 32 tokens at 540 keys 82.4 / 74.8, 64 at 900 148.1 /
+// 130.2; 16 heads, 64 at 900 73.3 / 72.0; 8 heads, 64 at 900 49.7 / 47.5);
 // up to four while a step has so few tokens that its blocks, in eight splits, stay below 1.35 an SM: then it is the
 // chain of a block's pages that counts (1 token x 16 heads: 0.5 to 2 % of a whole step, 5 tokens 2 %).
 void grouping(int n_tokens, int n_heads, int page_size, int sm_count, int* group, int* n_groups) {
@@ -493,7 +497,8 @@ DD_API int dd_attention_decode_pages(const void* q, int q_stride, const void* k_
     const int smem = p.stages * 2 * box_bytes + 1024 + MAX_STAGES * (2 * 8 + 4);
     static int configured = 0;
     if (configured < smem) {
-        cudaError_t e = cudaFuncSetAttribute(attention_decode_pages_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(attention_decode_pages_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_pages_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return dd_fail("dd_attention_decode_pages: shared memory of %d bytes refused: %s", smem, cudaGetErrorString(e));
         configured = smem;
     }
@@ -515,6 +520,9 @@ DD_API int dd_attention_decode_pages(const void* q, int q_stride, const void* k_
     p.n_pages = n_pages; p.window = window; p.chunk = chunk; p.gate = (const __nv_bfloat16*)gate; p.gate_stride = gate_stride;
     p.scale_log2e = scale * 1.4426950408889634f;
     p.n_tokens = n_tokens;
-    dd_launch(attention_decode_pages_kernel, dim3(n_tokens, n_groups, n_splits), dim3((p.G + 1) * 32), (size_t)smem, (cudaStream_t)stream, maps[0], maps[1], p);
+    const dim3 grid(n_tokens, n_groups, n_splits), block((p.G + 1) * 32);
+    cudaStream_t s = (cudaStream_t)stream;
+    if (p.G < 8) dd_launch(attention_decode_pages_kernel<7>, dim3(grid), dim3(block), (size_t)smem, s, maps[0], maps[1], p);
+    else dd_launch(attention_decode_pages_kernel<8>, dim3(grid), dim3(block), (size_t)smem, s, maps[0], maps[1], p);
     return dd_check_launch("dd_attention_decode_pages");
 }

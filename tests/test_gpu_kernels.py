@@ -383,6 +383,14 @@ def test_attention_decode_pages_deals_its_splits(K, heads, page, n_splits, windo
     assert bool(same.all()), "the fused kernel did not write the new key and value into the cache"
 
 
+@pytest.mark.parametrize("heads,page", [(8, 16), (16, 32), (31, 16), (32, 16)])
+@pytest.mark.parametrize("n_splits", [1, 6])
+def test_attention_decode_pages_in_groups_of_eight(K, heads, page, n_splits):
+    """Head counts that groups of up to eight take in fewer blocks than groups of seven; 31: the last group holds seven."""
+    test_attention_decode_pages_deals_its_splits(K, heads, page, n_splits, None)
+    assert K.attention_decode_pages_splits(32, 32, 16, 1024, DEV) == 6          # 128 blocks a split, not the 160 of groups of seven
+
+
 @pytest.mark.parametrize("d,heads,kv_heads,page", [(64, 5, 5, 16), (128, 4, 2, 8), (64, 6, 1, 32)])
 @pytest.mark.parametrize("window", [None, 70])
 def test_attention_prefill_bf16(K, d, heads, kv_heads, page, window):
