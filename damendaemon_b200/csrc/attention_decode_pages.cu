@@ -27,7 +27,6 @@
 
 namespace {
 constexpr int D = 64, TILE = 16, MAX_GROUP = 8;      // heads of a block: a warp each, and one that requests pages
-constexpr int MAX_BLOCK_PAGES = 128;          // pages a block may own; 1 << 7 below
 constexpr int MAX_STAGES = 3;                 // deeper rings are no faster and leave fewer blocks an SM (see the kernel)
 
 struct Params {
@@ -177,7 +176,6 @@ attention_decode_pages_kernel(const __grid_constant__ CUtensorMap map_kv, const 
     if (p.deal) {
         const float share = fmaxf(1.f, ceilf((float)total_pages * (float)gridDim.y * p.inv_block_budget));
         n_splits = max(1, (int)(((float)my_pages + 0.5f * share) / share));
-        n_splits = max(n_splits, (my_pages + MAX_BLOCK_PAGES - 1) >> 7);
         n_splits = min(n_splits, (int)gridDim.z);
         if (split >= n_splits) return;
     }
@@ -446,11 +444,10 @@ DD_API int dd_attention_decode_pages_splits(int n_tokens, int n_heads, int page_
     const int most = pages / 16 > 8 ? pages / 16 : 8;
     if (splits > most) splits = most;
     if (splits > pages) splits = pages;
-    if (splits < dd_ceil_div(pages, MAX_BLOCK_PAGES)) splits = dd_ceil_div(pages, MAX_BLOCK_PAGES);
     return splits < 1 ? 1 : splits;
 }
 
-// The arguments of dd_attention_decode (attention_decode.cu); max_blocks / n_splits may not exceed 128 pages.
+// The arguments of dd_attention_decode (attention_decode.cu).
 DD_API int dd_attention_decode_pages(const void* q, int q_stride, const void* k_new, const void* v_new, void* cache,
                                      const int* tok_entry, const int* tok_pos, const int* block_table, int max_blocks,
                                      void* out, int out_stride, float* part_o, float* part_ml, int* counters, int n_tokens,
@@ -463,8 +460,6 @@ DD_API int dd_attention_decode_pages(const void* q, int q_stride, const void* k_
                        "tokens (got %d, %d, %d, %d)", n_heads, n_kv_heads, head_dim, page_size);
     if (n_splits < 1 || n_splits > 65535 || (n_splits > 1 && (!part_o || !part_ml || !counters)))
         return dd_fail("dd_attention_decode_pages: n_splits=%d needs scratch and counters", n_splits);
-    if (dd_ceil_div(max_blocks, n_splits) > MAX_BLOCK_PAGES)
-        return dd_fail("dd_attention_decode_pages: %d pages in %d splits are more than %d pages per block", max_blocks, n_splits, MAX_BLOCK_PAGES);
     if (q_stride % 8 || out_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)cache & 15) || ((uintptr_t)out & 3))
         return dd_fail("dd_attention_decode_pages: rows must be 16-byte aligned");
     if (n_tokens > 65535) return dd_fail("dd_attention_decode_pages: too many tokens");

@@ -29,7 +29,6 @@ class AttentionTuning:
     900 keys x 25 heads took 42.0 us and eight at 900 x 16 heads 40.7 (now 35.5 and 33.0)."""
     pages_from_pairs: int = 1             # steps with at least this many (token, head) pairs stream whole pages,
     pages_from_pair_keys: int = 200_000   # ... or with this many pairs x keys of context; others take the row kernel
-    pages_per_block: int = 128            # a block of the page-streaming kernel holds the ids of this many pages
     row_keys_per_block: int = 128         # key split of the row decode kernel: keys per block ...
     row_blocks_per_sm: int = 2            # ... and blocks wanted per SM
 
@@ -98,8 +97,7 @@ def paged_attention(ctx, q, k, v, cache, n_heads, scale, window=None, chunk=None
         if tensor and many and head_dim == PAGES_HEAD_DIM and \
                 kernels.attention_decode_pages_supported(n_heads, kv_heads, head_dim, page_size, q.dtype):
             # whole pages of a group of heads by TMA
-            splits = kernels.attention_decode_pages_splits(n_tokens, n_heads, page_size, ctx.split_context, q.device)
-            return "pages", max(splits, -(-table.shape[1] // tune.pages_per_block))
+            return "pages", kernels.attention_decode_pages_splits(n_tokens, n_heads, page_size, ctx.split_context, q.device)
         if kernels.attention_decode_supported(n_heads, kv_heads, head_dim, q.dtype):
             return "rows", ctx.key_splits(n_heads, keys_per_block=tune.row_keys_per_block, blocks_per_sm=tune.row_blocks_per_sm, n_tokens=n_tokens)
         return None, 0

@@ -391,6 +391,28 @@ def test_attention_decode_pages_in_groups_of_eight(K, heads, page, n_splits):
     assert K.attention_decode_pages_splits(32, 32, 16, 1024, DEV) == 6          # 128 blocks a split, not the 160 of groups of seven
 
 
+@pytest.mark.parametrize("n_splits", [1, 3, 16])
+@pytest.mark.parametrize("window", [None, 2500])
+def test_attention_decode_pages_of_long_contexts(K, n_splits, window):
+    """Block tables of more than 64 entries, which are looked up 32 at a time: contexts that end on both sides of a multiple of
+    32 pages, up to 257 pages in one block, a window that starts behind entry 64, merges of 16 splits; a page that is
+    missing late in the table."""
+    heads, lengths = 3, [1025, 2049, 4100, 3]
+    c = paged_case(K, torch.bfloat16, heads, heads, 64, 16, lengths=lengths, new=[1] * 4, window=window, n_splits=n_splits, spike=None)
+    run = lambda q, cache, **kw: K.attention_decode(q, cache, None, c["pos"], c["table"], heads, c["scale"], window,
+                                                    n_splits=n_splits, kernel="pages", **kw)
+    out = run(c["q"], c["cache"])
+    assert K.read_error_flag(DEV) == 0 and (out.double().cpu() - c["ref"]).abs().max() < tol(torch.bfloat16)
+    q, k, v = c["packed"].split(heads * 64, dim=1)
+    wiped = c["cache"].clone()
+    for e, L in enumerate(lengths):
+        wiped[int(c["table"][e, (L - 1) // 16]), :, :, (L - 1) % 16] = float("nan")
+    assert torch.equal(run(q, wiped, k_new=k, v_new=v), out) and K.read_error_flag(DEV) == 0
+    c["table"][2, 200] = -1
+    got = run(c["q"], c["cache"])
+    assert K.read_error_flag(DEV) == 4 and bool(torch.isfinite(got).all()) and torch.equal(got[[0, 1, 3]], out[[0, 1, 3]])
+
+
 @pytest.mark.parametrize("d,heads,kv_heads,page", [(64, 5, 5, 16), (128, 4, 2, 8), (64, 6, 1, 32)])
 @pytest.mark.parametrize("window", [None, 70])
 def test_attention_prefill_bf16(K, d, heads, kv_heads, page, window):
