@@ -1,6 +1,8 @@
 """Matrix products of the parts: one call that picks the kernel for the engine dtype."""
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from .. import kernels
@@ -18,19 +20,54 @@ def splits_float32(out, reduction):
     return out * reduction >= 1 << 20
 
 
+RESIDENT_CLUSTERS = (148, 74, 45, 33, 26, 22, 15, 15)       # clusters of 1 to 8 blocks that a B200 holds at once, one block an SM
+STREAM_BOX_US = (0.32, 0.40, 0.46, 0.32, 0.46, 0.46, 0.37, 0.35)       # gemm_stream by blocks of a cluster: us a row and box of 256 k
+
+
+@functools.lru_cache(maxsize=4096)
+def stream_is_ahead(out, reduction):
+    """Whether gemm_stream is estimated to take less time than gemm_split for up to eight rows. Neither is ahead over a whole
+    range: both cut their work into rounds of what the GPU holds, at different sizes. The estimates, in us, were fitted to 217
+    shapes (out 300 to 100,000, reduction 128 to 14,336, 12 to 200 MB) that were timed with both. The product that they take
+    is the slower one by up to 8 % (1,024 x 11,008: 20.9 for 19.4), mostly by none; the stream alone is by up to 70 %
+    (split / stream at 8 rows: 4,096 x 4,096 18.4 / 27.6, 11,008 x 4,096 51.4 / 66.7, 65,536 x 128 14.5 / 24.7, 32,000 x 1,536
+    41.8 / 42.9; but 2,048 x 2,048 15.6 / 8.0, 9,000 x 1,280 13.3 / 11.9, 1,600 x 6,400 15.2 / 14.4)."""
+    up = lambda a, b: -(-a // b)
+    # split: a block takes its share of a tile's k blocks; tiles beyond the resident clusters wait for a second wave
+    blocks = up(reduction, 32)
+    share = up(blocks, kernels._split_plan(kernels.GEMM_STREAM_ROWS, out, reduction, RESIDENT_CLUSTERS[0])[0])
+    cluster = up(blocks, share)
+    waves = up(up(out, 128), RESIDENT_CLUSTERS[cluster - 1])
+    split = 5.4 + 0.37 * share * waves + (3.7 * (waves - 1) if cluster > 1 else 0)
+    # stream: a warp takes two to four rows of the matrix at a time, the fewest in all; the blocks that share K wait for one another
+    # in every round
+    part = up(up(reduction, up(reduction, 7 * 256)), 128) * 128
+    cluster, boxes = up(reduction, part), up(part, 256)
+    warps = 16 * RESIDENT_CLUSTERS[cluster - 1]
+    at_once = min((4, 3, 2), key=lambda r: up(up(out, r), warps) * r)
+    rounds = up(up(out, at_once), warps)
+    start, row = (1.9, 0.66) if cluster == 1 else (1.0 + 2.2 * rounds, 0.55)
+    stream = start + (row + STREAM_BOX_US[cluster - 1] * boxes) * rounds * at_once
+    return max(stream, out * reduction * 4 / 4.7e6) < split
+
+
 def streams_float32(rows, out, reduction):
     """Whether a float32 product that splits_float32 takes streams its matrix through the CUDA cores (kernels.gemm_stream)
-    instead: up to eight rows, and a matrix of 12 to 200 MB (split / stream, us at 8 rows: 3072 x 1024 13.7 / 5.8, 4096 x 1024
-    9.0 / 6.8, 1024 x 4096 11.0 / 8.4, 4800 x 1600 11.9 / 9.3, 6400 x 1600 14.2 / 11.0, 1600 x 6400 14.8 / 14.2, 25600 x 1600
-    41.7 / 34.6; 50257 x 1600 60.6 / 68.3: the stream's warps reach 4.7 TB/s, what their reads of X from shared memory leave
-    them, the split product 5.3). Smaller matrices stay with the split product, which gives a row the same bits among 1 to
-    128. A row of such a product has other bits beside more than seven others than beside fewer, within the error of either."""
-    return rows <= kernels.GEMM_STREAM_ROWS and 3 << 20 <= out * reduction <= 3 << 24 and reduction <= kernels.GEMM_STREAM_REDUCTION
+    instead: up to eight rows and a matrix of 12 to 200 MB, where that is ahead (split / stream, us at 8 rows: 3072 x 1024
+    13.7 / 5.8, 4096 x 1024 9.0 / 6.8, 1024 x 4096 11.0 / 8.4, 4800 x 1600 11.9 / 9.3, 6400 x 1600 14.2 / 11.0, 1600 x 6400
+    14.8 / 14.2, 25600 x 1600 41.7 / 34.6; 50257 x 1600 60.6 / 68.3: the stream's warps reach 4.7 TB/s, what their reads of X from
+    shared memory leave them, the split product 5.3). Smaller matrices stay with the split product. A row of a streamed
+    product has other bits beside more than seven others, where the split product takes over, than beside fewer, within
+    the error of either (gemm='simt' keeps them)."""
+    return rows <= kernels.GEMM_STREAM_ROWS and 3 << 20 <= out * reduction <= 3 << 24 and reduction <= kernels.GEMM_STREAM_REDUCTION \
+        and stream_is_ahead(out, reduction)
 
 
 def linear(runtime, a, w, bias=None, residual=None, activation=None, out_dtype=None, out=None):
-    """act(a @ w.T + bias) (+ residual). float32 engine: the split product on the tensor cores or, for small matrices and
-    rows that are not 16-byte aligned, or if the runtime asks for 'simt', the CUDA-core float32 kernel.
+    """act(a @ w.T + bias) (+ residual). float32 engine: the split product on the tensor cores, or for up to eight rows the
+    product that streams the matrix (a row's last bits may change between eight rows and nine, see streams_float32, and
+    beyond 128, see splits_float32); for small matrices and rows that are not 16-byte aligned, or if the runtime asks for 'simt',
+    the CUDA-core float32 kernel, whose rows do not depend on what is beside them.
     bfloat16 engine: the tcgen05 tensor-core kernel, unless the runtime asks for 'simt' or the
     reduction width is no multiple of 8 (then the CUDA-core kernel with bfloat16 operands)."""
     if a.dtype == torch.float32 and runtime.gemm != "simt" and out_dtype in (None, torch.float32) and \

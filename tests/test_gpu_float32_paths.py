@@ -177,6 +177,21 @@ def test_which_float32_products_are_streamed(K):
         K.gemm_stream(a[:1].expand(8, 1024), w)
 
 
+@pytest.mark.parametrize("N,Kd,streamed", [
+    # measured at 1 and 8 rows, split product / stream (us)
+    (4096, 4096, False),        # 18.0 / 26.6: more rows than the clusters that are resident take in one round
+    (65536, 128, False),        # 14.3 / 24.4: little to sum for every row
+    (11008, 4096, False), (4096, 11008, False), (5632, 2048, False), (50000, 1000, False), (32000, 1536, False), (3200, 6400, False),
+    (2048, 2048, True),         # 15.2 / 8.1: more clusters of the split product than are resident
+    (1600, 6400, True), (1280, 5120, True), (1024, 4096, True), (25600, 1600, True), (512, 8192, True), (4800, 1600, True)])
+def test_a_matrix_is_streamed_where_that_is_ahead(K, N, Kd, streamed):
+    from types import SimpleNamespace
+    from damendaemon_b200.parts.linear import linear, streams_float32
+    assert streams_float32(1, N, Kd) == streamed and streams_float32(8, N, Kd) == streamed and not streams_float32(9, N, Kd)
+    a, w = operands(3, N, Kd)
+    assert torch.equal(linear(SimpleNamespace(gemm="auto"), a, w), (K.gemm_stream if streamed else K.gemm_split)(a, w))
+
+
 def run_of_entries(dtype, entries, keys, heads, kv_heads, d, page=16, seed=11):
     """Queries of `entries` requests with `keys` tokens each, their caches and block tables: q [entries * keys, ...] is what a
     prompt of whole requests brings, its last row of every entry what a decode step brings."""
