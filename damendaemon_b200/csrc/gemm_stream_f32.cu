@@ -16,6 +16,7 @@
 // each 9.5, 11.2, 6.1 (50,257 x 1,600: 75.7 us, now 68.3); two blocks of 8 warps an SM 10.5, 11.0, 5.7.
 #include "common.cuh"
 #include "tcgen05.cuh"
+#include <atomic>
 
 namespace {
 
@@ -262,33 +263,48 @@ template <int R> int smem_bytes(int splits) {
     return StreamConfig<R>::SMEM_BYTES + (splits > 1 ? splits * WARPS * StreamConfig<R>::OUTS * 8 : 0);
 }
 
+constexpr int MAX_DEVICES = 16;             // whose answers are kept; of others they are asked for anew
+
+int device() {
+    int d = -1;
+    return cudaGetDevice(&d) == cudaSuccess ? d : -1;
+}
+
+// The kernel's shared memory, once a device (two threads that both ask set the same).
 template <int R> cudaError_t configure() {
-    static const cudaError_t configured = cudaFuncSetAttribute(gemm_stream_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, StreamConfig<R>::MOST_BYTES);
-    return configured;
+    static std::atomic<bool> configured[MAX_DEVICES];
+    const int d = device();
+    const bool kept = d >= 0 && d < MAX_DEVICES;
+    if (kept && configured[d].load(std::memory_order_acquire)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(gemm_stream_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, StreamConfig<R>::MOST_BYTES);
+    if (kept && e == cudaSuccess) configured[d].store(true, std::memory_order_release);
+    return e;
 }
 
 // Clusters that are resident at once: of four blocks fewer than a quarter of the SMs' number, and a second wave of them
-// doubles the time.
+// doubles the time. Of every R the same: each takes more than half of an SM's shared memory, so one block fits.
 int resident_clusters(int splits, int sm_count) {
-    static int resident[MAX_SPLITS + 1];
-    if (!resident[splits]) {
-        int n = 0;
+    static std::atomic<int> resident[MAX_DEVICES][MAX_SPLITS + 1];
+    static_assert(StreamConfig<2>::SMEM_BYTES > 114 * 1024 && StreamConfig<3>::SMEM_BYTES > 114 * 1024 && StreamConfig<4>::SMEM_BYTES > 114 * 1024, "one block an SM");
+    const int d = device();
+    const bool kept = d >= 0 && d < MAX_DEVICES;
+    int n = kept ? resident[d][splits].load(std::memory_order_relaxed) : 0;
+    if (!n) {
         cudaLaunchAttribute attrs[2];
         cudaLaunchConfig_t config = launch_config(smem_bytes<4>(splits), splits, nullptr, attrs);
-        config.gridDim = dim3(sm_count / splits * splits);
+        config.gridDim = dim3(splits);
         config.numAttrs = 1;
         if (configure<4>() != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_stream_kernel<4>, &config) != cudaSuccess || n < 1) {
             cudaGetLastError();
             n = sm_count / splits;
-        }
-        resident[splits] = n < sm_count / splits ? n : sm_count / splits;
+        } else if (kept) resident[d][splits].store(n, std::memory_order_relaxed);
     }
-    return resident[splits];
+    return n < sm_count / splits ? n : sm_count / splits;
 }
 
 template <int R>
 int launch(const CUtensorMap& map_x, const StreamParams& p, int splits, int clusters, cudaStream_t s) {
-    if (configure<R>() != cudaSuccess) return dd_fail("dd_gemm_stream: shared memory refused: %s", cudaGetErrorString(configure<R>()));
+    if (cudaError_t e = configure<R>()) return dd_fail("dd_gemm_stream: shared memory refused: %s", cudaGetErrorString(e));
     cudaLaunchAttribute attrs[2];
     cudaLaunchConfig_t config = launch_config(smem_bytes<R>(splits), splits, s, attrs);
     const int groups = dd_ceil_div(p.N, R);
@@ -299,6 +315,11 @@ int launch(const CUtensorMap& map_x, const StreamParams& p, int splits, int clus
 }
 
 }  // namespace
+
+// How many clusters of so many blocks dd_gemm_stream takes to be resident at once on the current device's first sm_count SMs.
+DD_API int dd_gemm_stream_clusters(int splits, int sm_count) {
+    return splits < 1 || splits > MAX_SPLITS || sm_count < splits ? 0 : resident_clusters(splits, sm_count);
+}
 
 // X [M,K] (M up to 8) and W [N,K] float32, 16-byte aligned, row strides and K multiples of 4, rows that do not lie over one
 // another; bias [N] or null; residual [M,N] (row stride ldr, may be out itself) or null; out [M,N] float32.

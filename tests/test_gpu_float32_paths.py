@@ -192,6 +192,16 @@ def test_a_matrix_is_streamed_where_that_is_ahead(K, N, Kd, streamed):
     assert torch.equal(linear(SimpleNamespace(gemm="auto"), a, w), (K.gemm_stream if streamed else K.gemm_split)(a, w))
 
 
+def test_resident_clusters_of_the_streamed_product(K):
+    """Asked first for a part of the GPU and by several threads: the answer for all of it is not that of the part."""
+    from concurrent.futures import ThreadPoolExecutor
+    ask = K.library("core").dd_gemm_stream_clusters
+    assert ask(2, 16) <= 8 and ask(0, 148) == 0 and ask(9, 148) == 0 and ask(8, 7) == 0
+    with ThreadPoolExecutor(8) as pool:
+        for n, got in enumerate(pool.map(lambda n: [ask(n, 148) for _ in range(50)], range(1, 9)), start=1):
+            assert len(set(got)) == 1 and 148 // n // 2 < got[0] <= 148 // n
+
+
 def run_of_entries(dtype, entries, keys, heads, kv_heads, d, page=16, seed=11):
     """Queries of `entries` requests with `keys` tokens each, their caches and block tables: q [entries * keys, ...] is what a
     prompt of whole requests brings, its last row of every entry what a decode step brings."""
