@@ -760,7 +760,7 @@ def _float32_attention_case(batch, length, dev, decode):
 
 
 def build(name, device="cuda:0"):
-    """name: gemm_<qkv|proj|fc|fc2|head>_m<tokens> | gemm32_<...>_m<tokens> (float32, CUDA cores) | gemmsplit_<...>_m<tokens> (float32 in three bfloat16 parts) |
+    """name: gemm_<qkv|proj|fc|fc2|head>_m<tokens> | gemm32_<...>_m<tokens> (float32, CUDA cores) | gemmsplit_<...>_m<tokens> (float32 in three bfloat16 parts) | gemmstream_<...>_m<tokens> (float32 streamed, up to 8) |
     attn32_decode_b<batch>_c<context> | attn32_prefill_p<prompts>_t<tokens> (the float32 kernels) | attn_decode_b<batch>[_c<context>] (page streaming) | attn_decode_rows_b<batch>[_c<context>] | attn_prefill_p<prompts>_t<tokens> | attn_prefill | attn_prefill_store (the kernel writes the cache too) | attn_prefill_mma |
     attn_prefill_long (one prompt of 4,096 tokens) | layernorm_m<rows> | rmsnorm_m<rows> | rotary_m<rows> |
     grouped_<up|upsilu|down|route|score>_m<tokens> (sixteen experts, two per token; upsilu: the silu form of the unit;
@@ -867,6 +867,8 @@ def build(name, device="cuda:0"):
         return _gemm32_case(parts[1], int(parts[2][1:]), device)
     if parts[0] == "gemmsplit" and len(parts) == 3 and parts[1] in SHAPES and parts[2][0] == "m":
         return _gemm32_case(parts[1], int(parts[2][1:]), device, K.gemm_split)
+    if parts[0] == "gemmstream" and len(parts) == 3 and parts[1] in SHAPES and parts[2][0] == "m":
+        return _gemm32_case(parts[1], int(parts[2][1:]), device, K.gemm_stream)
     if name.startswith("attn32_decode_b"):
         batch, context = name[len("attn32_decode_b"):].split("_c")
         return _float32_attention_case(int(batch), int(context), device, decode=True)

@@ -86,8 +86,9 @@ __device__ __forceinline__ uint32_t tile_off(int r, int c) { return (uint32_t)(r
 // the warp that finishes last, through a counter per head: before, the blocks' barriers, fences and the last block's
 // walk over all its heads were 4.4 us behind the last key. Whole passes, before and now: 8 requests from 512 keys on
 // (xl, 64 steps) 129.7 / 117.8 ms, 64 from 256 keys on 204.1 / 195.8, 32 of 16 to 800 keys (medium) 48.9 / 44.4.
-// 80 registers and three stages leave three blocks an SM: with 104 registers and two blocks the last of these takes 45.9
-// (and the first 118.0), with two stages 44.5 (122.3), with four 46.2; a spilled register costs more than any of them.
+// With pages of 16 tokens, three stages of groups of up to six heads (75 KB) and 80 registers leave three blocks an SM; groups of
+// seven and eight (87 and 99 KB) leave two. Measured with 16 heads in groups of six (medium) and 25 in groups of seven (xl):
+// 104 registers and two blocks 45.9 ms (118.0), two stages 44.5 (122.3), four 46.2; a spilled register costs more than any.
 // Groups of eight (288 threads) take two blocks' registers, 96 a thread.
 template <int MOST>
 __global__ void __launch_bounds__((MOST + 1) * 32, MOST < 8 ? 3 : 2)
@@ -478,7 +479,9 @@ DD_API int dd_attention_decode_pages(const void* q, int q_stride, const void* k_
     int n_groups = 0;
     grouping(n_tokens, n_heads, page_size, sm_count, &p.G, &n_groups);
     const int box_bytes = p.G * page_size * 128;
-    p.stages = (106 * 1024) / (2 * box_bytes);            // two blocks per SM
+    // Stages for two blocks an SM, and the splits are dealt out for two, also where the groups are so small that three of
+    // MAX_STAGES fit (up to six heads of 16 tokens): a budget of three has not been measured.
+    p.stages = (106 * 1024) / (2 * box_bytes);
     int blocks_per_sm = 2;
     if (p.stages < 2) {                                               // large pages: one block per SM
         p.stages = (210 * 1024) / (2 * box_bytes);

@@ -210,6 +210,22 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         tc::cluster_arrive();
         tc::cluster_wait();
     };
+    // one thread: the tokens' planes that a kernel before this one wrote (X_SPLIT). A k block's three planes of BN tokens lie in
+    // memory as they lie in shared memory, one piece
+    auto fetch_planes = [&] {
+        dd_grid_wait();
+        int it = 0;
+        bool ok = true;
+        for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
+            const uint8_t* from = p.planes + ((size_t)(tile / tiles_n) * total_kblocks + kb_begin) * C::OPERAND_BYTES;
+            for (int i = 0; i < n_kblocks; ++i, ++it, from += C::OPERAND_BYTES) {
+                const int s = it % C::OPERANDS;
+                if (!tc::mbar_wait(&mma_done[s], ((it / C::OPERANDS) & 1) ^ 1, abort_flag)) { ok = false; break; }
+                tc::mbar_expect_tx(&split_done[s], C::OPERAND_BYTES);
+                bulk_load(operands + s * C::OPERAND_BYTES, from, C::OPERAND_BYTES, &split_done[s]);
+            }
+        }
+    };
     if (warp < C::FIRST_EPI) {
         if constexpr (C::GROUPED) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
         if (warp == 0) {
@@ -261,21 +277,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 }
             }
         } else if (C::GROUPED && warp == C::FIRST_X) {
-            if (tc::elect_one()) {
-                // a k block's three planes of BN tokens lie in memory as they lie in shared memory, one piece
-                dd_grid_wait();
-                int it = 0;
-                bool ok = true;
-                for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
-                    const uint8_t* from = p.planes + ((size_t)(tile / tiles_n) * total_kblocks + kb_begin) * C::OPERAND_BYTES;
-                    for (int i = 0; i < n_kblocks; ++i, ++it, from += C::OPERAND_BYTES) {
-                        const int s = it % C::OPERANDS;
-                        if (!tc::mbar_wait(&mma_done[s], ((it / C::OPERANDS) & 1) ^ 1, abort_flag)) { ok = false; break; }
-                        tc::mbar_expect_tx(&split_done[s], C::OPERAND_BYTES);
-                        bulk_load(operands + s * C::OPERAND_BYTES, from, C::OPERAND_BYTES, &split_done[s]);
-                    }
-                }
-            }
+            if (tc::elect_one()) fetch_planes();
         }
         stand_by();
     } else if (warp < C::FIRST_CONV) {
@@ -400,21 +402,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         }
         stand_by();
     } else if (C::X_SPLIT) {
-        if (tc::elect_one()) {
-            // a k block's three planes of BN tokens lie in memory as they lie in shared memory, one piece
-            dd_grid_wait();
-            int it = 0;
-            bool ok = true;
-            for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
-                const uint8_t* from = p.planes + ((size_t)(tile / tiles_n) * total_kblocks + kb_begin) * C::OPERAND_BYTES;
-                for (int i = 0; i < n_kblocks; ++i, ++it, from += C::OPERAND_BYTES) {
-                    const int s = it % C::OPERANDS;
-                    if (!tc::mbar_wait(&mma_done[s], ((it / C::OPERANDS) & 1) ^ 1, abort_flag)) { ok = false; break; }
-                    tc::mbar_expect_tx(&split_done[s], C::OPERAND_BYTES);
-                    bulk_load(operands + s * C::OPERAND_BYTES, from, C::OPERAND_BYTES, &split_done[s]);
-                }
-            }
-        }
+        if (tc::elect_one()) fetch_planes();
         stand_by();
     } else {
         // Eight values of a token's row at a time: 32 bytes of staging, 16 bytes of each plane.
