@@ -407,14 +407,19 @@ EncodeTiled encode_fn() {
     return fn;
 }
 
-// Heads per block, spread evenly over the groups: up to eight (a warp each, 256 box rows at most), since the fewer and
-// larger the boxes the better they stream (64 tokens x 25 heads: a step of 195 ms in groups of 7, 214 in groups of 5; us a
-// layer of a whole step in groups of at most seven / eight: 32 heads, 32 tokens at 540 keys 82.4 / 74.8, 64 at 900 148.1 /
-// 130.2; 16 heads, 64 at 900 73.3 / 72.0; 8 heads, 64 at 900 49.7 / 47.5);
+// Heads per block, spread evenly over the groups: up to seven (a warp each, 256 box rows at most), since the fewer and
+// larger the boxes the better they stream (64 tokens x 25 heads: a step of 195 ms in groups of 7, 214 in groups of 5); up to
+// eight for 31 and 32 heads, four groups of them instead of five full ones of seven (us a layer of a whole step, seven / eight:
+// 32 tokens at 540 keys 82.4 / 74.8, 64 at 900 146.6 / 129.5, 64 at 16 to 768 keys 94.4 / 96.0). Where groups of seven leave
+// places free, they stay: three groups of six and not two of eight for 16 heads, since three smaller blocks share an SM (64
+// at 16 to 768 keys 54.6 / 58.4, at 900 73.6 / 72.1; 24 heads 67.9 / 71.3, at 900 92.9 / 100.9); and one of six or more groups
+// saved brings nothing (40 heads, 32 tokens at 900 keys 131.0 / 134.4);
 // up to four while a step has so few tokens that its blocks, in eight splits, stay below 1.35 an SM: then it is the
 // chain of a block's pages that counts (1 token x 16 heads: 0.5 to 2 % of a whole step, 5 tokens 2 %).
 void grouping(int n_tokens, int n_heads, int page_size, int sm_count, int* group, int* n_groups) {
     int most = MAX_GROUP < 256 / page_size ? MAX_GROUP : 256 / page_size;
+    const int sevens = dd_ceil_div(n_heads, 7);
+    if (most > 7 && (sevens > 5 || dd_ceil_div(n_heads, sevens) < 7)) most = 7;
     if (most > 4 && (long long)n_tokens * dd_ceil_div(n_heads, 4) * 8 * 20 <= 27ll * sm_count) most = 4;
     *n_groups = dd_ceil_div(n_heads, most);
     *group = dd_ceil_div(n_heads, *n_groups);

@@ -23,7 +23,7 @@ PAGES_HEAD_DIM = 64                       # the only head size of the page-strea
 class AttentionTuning:
     """Thresholds of the kernel choice. Whole pages by TMA are ahead of rows at any number of single tokens (us a layer of a
     whole decode step on a B200, rows / pages: 25 heads, one request at 64, 300, 600, 900 keys 31.3 / 28.5, 31.3 / 29.7,
-    31.2 / 30.4, 31.6 / 31.6; two at 900 34.9 / 32.9, four at 540 37.2 / 33.6, eight at 540 39.3 / 35.4; 16 heads, eight at 900
+    31.2 / 30.4, 31.6 / 31.6; two at 900 34.9 / 32.9, four at 540 37.2 / 33.6; 16 heads, eight at 900
     37.9 / 33.0; one request of 4,000 keys in a table of 4,096 42.3 / 38.7), so by default every step takes them. The
     splits are dealt out by the contexts (attention_decode_pages_splits): cut by row_keys_per_block instead, four requests at
     900 keys x 25 heads took 42.0 us and eight at 900 x 16 heads 40.7 (now 35.5 and 33.0)."""

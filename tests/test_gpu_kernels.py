@@ -222,6 +222,13 @@ def test_attention_decode_bf16(K, d, heads, page, n_splits, window):
     assert bool(same.all()), "the fused kernel did not write the new key and value into the cache"
 
 
+@pytest.mark.parametrize("n_splits", [1, 3])
+def test_attention_decode_bf16_of_small_pages(K, n_splits):
+    """Pages that page streaming does not take: the row kernel's tables of more than 64 entries."""
+    assert not K.attention_decode_pages_supported(3, 3, 64, 8, torch.bfloat16)
+    test_attention_decode_bf16(K, 64, 3, 8, n_splits, None)
+
+
 @pytest.mark.parametrize("heads,page", [(5, 16), (25, 16), (17, 32), (3, 64), (2, 128), (33, 16)])
 @pytest.mark.parametrize("n_splits", [1, 2, 3, 8, 11])
 @pytest.mark.parametrize("window", [None, 100])
@@ -383,12 +390,14 @@ def test_attention_decode_pages_deals_its_splits(K, heads, page, n_splits, windo
     assert bool(same.all()), "the fused kernel did not write the new key and value into the cache"
 
 
-@pytest.mark.parametrize("heads,page", [(8, 16), (16, 32), (31, 16), (32, 16)])
+@pytest.mark.parametrize("heads,page", [(31, 16), (32, 16), (32, 32), (16, 16), (24, 32), (40, 16)])
 @pytest.mark.parametrize("n_splits", [1, 6])
-def test_attention_decode_pages_in_groups_of_eight(K, heads, page, n_splits):
-    """Head counts that groups of up to eight take in fewer blocks than groups of seven; 31: the last group holds seven."""
+def test_attention_decode_pages_in_groups_of_seven_and_eight(K, heads, page, n_splits):
+    """31 and 32 heads in four groups of up to eight (31: the last holds seven), 16 and 24 in groups of six, 40 in six groups."""
     test_attention_decode_pages_deals_its_splits(K, heads, page, n_splits, None)
-    assert K.attention_decode_pages_splits(32, 32, 16, 1024, DEV) == 6          # 128 blocks a split, not the 160 of groups of seven
+    # the most splits follow from the groups: 2.5 x 296 blocks over 32 tokens and so many groups, rounded up
+    groups = {31: 4, 32: 4, 16: 3, 24: 4, 40: 6}[heads]
+    assert K.attention_decode_pages_splits(32, heads, 16, 1024, DEV) == -(-5 * 2 * 148 // (2 * 32 * groups))
 
 
 @pytest.mark.parametrize("n_splits", [1, 3, 16])
